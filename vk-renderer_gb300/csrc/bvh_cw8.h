@@ -28,7 +28,10 @@ namespace vkt {
 //            lo x (w8, w9), lo y (w10, w11), lo z (w12, w13),
 //            hi x (w14, w15), hi y (w16, w17), hi z (w18, w19);
 //            box = [p + lo * 2^(e - 127), p + hi * 2^(e - 127)] per axis,
-//            which contains the binary child's (padded) box exactly
+//            which contains the binary child's (padded) box with a margin of
+//            1/64 grid step on each side (the kernel's slab distances, with
+//            2^15 steps added and taken off, round by up to 3/512 step);
+//            p - 2^15 * 2^(e - 127) is a float too
 //   w20, w21 hit-mask bits of slot k: a leaf of c primitives (1..6) ->
 //            (1 << c) - 1; an interior child -> 1; an empty slot -> 0
 //   w22, w23 bit position of slot k: a leaf -> o, its first primitive being
@@ -48,16 +51,49 @@ constexpr uint32_t kCw8MaxLeafPrims = 6;
 constexpr uint32_t kCw8MaxNodePrims = 24;
 
 // Collapses a binary BVH (tracer_bvh_node, root 0, children side by side,
-// leaves = ranges of the leaf-ordered primitive array) into 8-wide nodes.
-// Each node takes a binary interior node's two children and repeatedly
-// replaces the interior child of largest surface area by its two children
-// while it has fewer than eight and its leaf children hold at most 24
-// primitives.  order_out[k] = leaf-ordered slot of the 8-wide order's
+// leaves = ranges of the leaf-ordered primitive array) into 8-wide nodes:
+// the cut of the binary tree with the least expected cost (the dynamic
+// programme of Ylitie et al., section 3.1: surface area x 1 for a node
+// visit, x kPrimCost for a primitive of a leaf child), where a subtree of at
+// most kMergePrims primitives may become one leaf child and a node's leaf
+// children hold at most 24 primitives.  order_out[k] = leaf-ordered slot of the 8-wide order's
 // primitive k.  *depth_out = levels of 8-wide nodes (the traversal stack
 // holds at most one entry per level).  Returns false (no 8-wide BVH) when a
 // leaf holds more than 6 primitives or a coordinate's magnitude exceeds 1e6
 // (the quantised slab test's range).
 bool build_cw8(const tracer_bvh_node* nodes, uint32_t num_nodes, std::vector<Cw8Node>& out,
                std::vector<uint32_t>& order_out, uint32_t* depth_out);
+
+// The node the kernels read, 96 bytes (three 256-bit loads), as 24
+// little-endian words: a Cw8Node's boxes with the grid written out as floats
+// and its masks gathered.
+//   w0..w2   p - 2^15 * step per axis (float, exact): the kernel makes a byte
+//            q the float 2^15 + q with one byte permute, so that a plane is
+//            w0 + (2^15 + q) * step
+//   w3..w5   the grid steps (float x, y, z)
+//   w6       child_base, w7 prim_base: as Cw8Node's; slot k's primitives start
+//            at prim_base + popc(leaf mask below k) + popc(two mask below k)
+//   w8       imask | leaf mask << 8 | two mask << 16: bit k of each = slot k
+//            holds an interior child / a leaf child / a leaf child of two
+//            primitives (leaf children hold one or two); w9 0
+//   w10..w21 quantised box bytes, slot k in byte k % 4 of the word pair:
+//            lo x, hi x, lo y, hi y, lo z, hi z; w22, w23 0
+struct alignas(32) W8Node {
+    uint32_t w[24];
+};
+static_assert(sizeof(W8Node) == 96, "device node is 96 bytes");
+
+// One W8Node per node of an 8-wide BVH whose leaf children hold at most two
+// primitives each; false otherwise.
+bool pack_w8(const std::vector<Cw8Node>& in, std::vector<W8Node>& out);
+
+// Splits every leaf of a binary BVH over triangles down to single triangles
+// (kCw8MaxLeafPrims at most per leaf), keeping the nodes above.  tri[k]: low
+// and high corner of the box of leaf-ordered triangle k.  out: the deeper
+// tree, its leaves ranges of a new order whose entry j is leaf-ordered slot
+// slot_out[j].  A part's box is that of its triangles, padded as the binary
+// builder's, and inside the leaf's.
+void split_leaves(const tracer_bvh_node* nodes, uint32_t num_nodes, const double (*tri)[6],
+                  std::vector<tracer_bvh_node>& out, std::vector<uint32_t>& slot_out);
 
 }  // namespace vkt

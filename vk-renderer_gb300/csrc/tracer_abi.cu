@@ -57,6 +57,7 @@ struct SceneBuffers {
     uint32_t wide_depth = 0;  // deepest 4-wide BVH
     bool wide = false;        // 4-wide nodes present
     uint32_t cw8_depth = 0;   // levels of the 8-wide BVH
+    uint32_t n_cw8_nodes = 0;
     bool cw8 = false;         // 8-wide BVH present (triangle-only scenes)
     bool bvh = false;
     bool loaded = false;
@@ -420,11 +421,9 @@ int pick_width_for(tracer_ctx* c, const tracer_trace_params* p, bool have_wide, 
         return fail(c, TRACER_ERR_INVALID_ARG, "bvh_width %u must be 0, 2, 4 or 8", p->bvh_width);
     if (p->bvh_width == 8 || (p->bvh_width == 0 && have_cw8)) {
         if (!have_cw8) return fail(c, TRACER_ERR_INVALID_ARG, "the scene has no 8-wide BVH (triangle-only scenes)");
-        if (stack < cw8_depth) {
-            if (p->stack_depth)
-                return fail(c, TRACER_ERR_STACK_OVERFLOW, "8-wide traversal needs a stack of %u entries", cw8_depth);
-            stack = cw8_depth;
-        }
+        // its own need, whatever the caller's stack_depth (which bounds the
+        // binary traversal's): split leaves can make it the deeper tree
+        if (stack < cw8_depth) stack = cw8_depth;
         wide = WF_WIDTH_8;
         return TRACER_OK;
     }
@@ -444,9 +443,11 @@ int pick_width_for(tracer_ctx* c, const tracer_trace_params* p, bool have_wide, 
     return TRACER_OK;
 }
 
-// Traversal steps a ray may take over a BVH of `nodes` nodes: each node is
-// entered at most once per pass, so twice the node count (plus slack) is
-// never reached by a valid BVH; tracer_set_traversal_limit overrides it.
+// Traversal steps a ray may take over a BVH of `nodes` nodes (the larger of
+// the binary and the 8-wide one, which may hold more than a binary BVH with
+// large leaves): each node is entered at most once per pass, so twice the
+// node count (plus slack) is never reached by a valid BVH;
+// tracer_set_traversal_limit overrides it.
 uint32_t trav_limit(const tracer_ctx* c, uint32_t nodes)
 {
     return c->trav_cap ? c->trav_cap : 2 * nodes + 16;
@@ -481,12 +482,31 @@ int pick_width(tracer_ctx* c, const tracer_trace_params* p, uint32_t& stack, int
 // The 8-wide BVH of a triangle BVH and the triangles in its order: 64-byte
 // records (v0, original id) (v1 - v0, leaf-ordered slot) (v2 - v0, 0) (0),
 // from the leaf-ordered triangle records `tri` (3 float4 each, as uploaded).
-// Returns false when the scene gets none (bvh_cw8.h).
-bool make_cw8(const std::vector<tracer_bvh_node>& tnodes, const std::vector<float4>& tri, std::vector<Cw8Node>& nodes,
+// The binary leaves are split to single triangles first.  Returns false when
+// the scene gets none (bvh_cw8.h).
+bool make_cw8(const std::vector<tracer_bvh_node>& tnodes, const std::vector<float4>& tri, std::vector<W8Node>& nodes,
               std::vector<float4>& prims, uint32_t& depth)
 {
-    std::vector<uint32_t> order;
-    if (tnodes.empty() || !build_cw8(tnodes.data(), (uint32_t)tnodes.size(), nodes, order, &depth)) return false;
+    if (tnodes.empty()) return false;
+    for (const tracer_bvh_node& n : tnodes)
+        if ((uint32_t)n.count > kCw8MaxLeafPrims) return false;
+    const size_t nt = tri.size() / 3;
+    std::vector<double> box(6 * nt);  // of (v0, v0 + e1, v0 + e2), the triangle the kernels test
+    for (size_t k = 0; k < nt; ++k) {
+        const float4 a = tri[3 * k], b = tri[3 * k + 1], e = tri[3 * k + 2];
+        const double v[3] = {a.x, a.y, a.z}, e1[3] = {b.x, b.y, b.z}, e2[3] = {e.x, e.y, e.z};
+        for (int q = 0; q < 3; ++q) {
+            box[6 * k + q] = v[q] + std::min(0.0, std::min(e1[q], e2[q]));
+            box[6 * k + 3 + q] = v[q] + std::max(0.0, std::max(e1[q], e2[q]));
+        }
+    }
+    std::vector<tracer_bvh_node> split;
+    std::vector<uint32_t> order, slot_of;
+    split_leaves(tnodes.data(), (uint32_t)tnodes.size(), reinterpret_cast<const double(*)[6]>(box.data()), split,
+                 slot_of);
+    std::vector<Cw8Node> coded;
+    if (!build_cw8(split.data(), (uint32_t)split.size(), coded, order, &depth) || !pack_w8(coded, nodes)) return false;
+    for (uint32_t& s : order) s = slot_of[s];
     prims.assign(4 * order.size(), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
     for (size_t k = 0; k < order.size(); ++k) {
         const uint32_t slot = order[k];
@@ -736,7 +756,7 @@ int tracer_upload_scene(tracer_ctx* c, const tracer_scene_desc* d)
     if (!encode_refs(tnodes.data(), (uint32_t)tnodes.size(), tenc) ||
         !encode_refs(snodes.data(), (uint32_t)snodes.size(), senc))
         return fail(c, TRACER_ERR_BAD_BVH, "a BVH leaf holds more than 64 primitives or starts beyond 2^25");
-    std::vector<Cw8Node> cw8;
+    std::vector<W8Node> cw8;
     std::vector<float4> cw8_prims;
     uint32_t cw8_depth = 0;
     const bool cw8_ok = s.bvh && s.nt > 0 && s.ns == 0 && make_cw8(tnodes, tri, cw8, cw8_prims, cw8_depth);
@@ -767,6 +787,7 @@ int tracer_upload_scene(tracer_ctx* c, const tracer_scene_desc* d)
     s.wide = wide_ok;
     s.cw8 = cw8_ok;
     s.cw8_depth = cw8_depth;
+    s.n_cw8_nodes = cw8_ok ? (uint32_t)cw8.size() : 0u;
     s.loaded = true;
     ++c->scene_version;
     return TRACER_OK;
@@ -868,7 +889,7 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
     a.sky = V3{p->sky[0], p->sky[1], p->sky[2]};
     a.sky_on = !(p->sky[0] == 0.0f && p->sky[1] == 0.0f && p->sky[2] == 0.0f);
     a.stack_depth = stack;
-    const uint32_t nn = s.n_tri_nodes > s.n_sph_nodes ? s.n_tri_nodes : s.n_sph_nodes;
+    const uint32_t nn = std::max(std::max(s.n_tri_nodes, s.n_sph_nodes), s.n_cw8_nodes);
     a.trav_limit = trav_limit(c, nn);
     a.rgba8 = (mask & (1u << TRACER_AOV_RGBA8)) ? c->rgba8.p : nullptr;
     a.rgba32f = (mask & (1u << TRACER_AOV_RGBA32F)) ? c->rgba32f.p : nullptr;
@@ -1175,7 +1196,7 @@ extern "C" int tracer_trace_noalloc(tracer_ctx* c, const tracer_frame* f, const 
     a.sky = V3{p->sky[0], p->sky[1], p->sky[2]};
     a.sky_on = !(p->sky[0] == 0.0f && p->sky[1] == 0.0f && p->sky[2] == 0.0f);
     a.stack_depth = stack;
-    const uint32_t nn = s.n_tri_nodes > s.n_sph_nodes ? s.n_tri_nodes : s.n_sph_nodes;
+    const uint32_t nn = std::max(std::max(s.n_tri_nodes, s.n_sph_nodes), s.n_cw8_nodes);
     a.trav_limit = trav_limit(c, nn);
     a.rgba8 = static_cast<uchar4*>(rgba8_out);
     a.rgba32f = static_cast<float4*>(rgba32f_out);
@@ -1243,7 +1264,7 @@ struct PackedScene {
     std::vector<uint32_t> sid, emit;
     std::vector<tracer_bvh_node> tnodes, snodes, tenc, senc;
     std::vector<WideNode> twide, swide;
-    std::vector<Cw8Node> cw8;
+    std::vector<W8Node> cw8;
     std::vector<float4> cw8_prims;
     uint32_t depth = 0, wide_depth = 0, cw8_depth = 0;
     bool wide = false, cw8_ok = false;
@@ -1461,7 +1482,7 @@ extern "C" int tracer_upload_scenes(tracer_ctx* c, const tracer_scene_desc* desc
         b.wide_depth = std::max(b.wide_depth, p.wide_depth);
         b.cw8_depth = std::max(b.cw8_depth, p.cw8_depth);
         c->batch_depth[k] = p.depth;
-        c->batch_nodes[k] = (uint32_t)std::max(p.tnodes.size(), p.snodes.size());
+        c->batch_nodes[k] = (uint32_t)std::max(std::max(p.tnodes.size(), p.snodes.size()), p.cw8.size());
         c->batch_emitters = c->batch_emitters || !p.emit.empty();
     }
     b.nt = (uint32_t)(tri.size() / 3);
@@ -1831,7 +1852,7 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
     a.sky = V3{p->sky[0], p->sky[1], p->sky[2]};
     a.sky_on = !(p->sky[0] == 0.0f && p->sky[1] == 0.0f && p->sky[2] == 0.0f);
     a.stack_depth = stack;
-    const uint32_t nn = s.n_tri_nodes > s.n_sph_nodes ? s.n_tri_nodes : s.n_sph_nodes;
+    const uint32_t nn = std::max(std::max(s.n_tri_nodes, s.n_sph_nodes), s.n_cw8_nodes);
     a.trav_limit = trav_limit(c, nn);
     a.stats = c->stats.p;
     a.status = c->status.p;

@@ -1,153 +1,140 @@
-// Device side of the compressed 8-wide BVH (layout: bvh_cw8.h): one node's
-// eight quantised slab tests and the node groups a traversal keeps.
+// Device side of the 8-wide BVH (node layout: W8Node in bvh_cw8.h): one
+// node's eight slab tests and the groups a traversal keeps.
 //
-// A node group is (child_base, remaining hit interior children << 24 | imask):
-// bit 24 + (k ^ s ^ 7) stands for slot k (s = the ray's direction octant), so
-// the highest set bit is the next child to visit and slot k's node index is
-// child_base + popc(imask & ((1 << k) - 1)).  A primitive group is
-// (prim_base, bit i = primitive prim_base + i still to test).
+// A node group is (child_base, interior children hit and not yet visited |
+// imask << 8), bit k = slot k: slot k's node index is
+// child_base + popc(imask & ((1 << k) - 1)).  A leaf group is (prim_base,
+// leaf children hit and not yet tested | leaf mask << 8 | two mask << 16).
 #pragma once
 
 #include "tracer_traverse.cuh"
 
 namespace vkt {
 
-// The ray's quantities for the 8-wide slab test: the direction octant and,
-// per axis, the slab planes' order (near plane = low bound for a
-// non-negative inverse direction).
-struct Cw8Ray {
+// The ray's quantities for the 8-wide slab test.  Octant s of the direction:
+// bit a set for a negative inverse direction on axis a.  pref4, pref2, pref1:
+// the slots whose bit 2, 1, 0 equals s's, i.e. the half to visit first.
+struct W8Ray {
     BoxRay br;
-    uint32_t oct7;  // (octant s) ^ 7
+    uint32_t pref4, pref2, pref1;
 };
 
-__device__ __forceinline__ Cw8Ray make_cw8ray(const Ray& r)
+__device__ __forceinline__ W8Ray make_w8ray(const Ray& r)
 {
-    Cw8Ray c;
+    W8Ray c;
     c.br = make_boxray(r);
-    const uint32_t s = (c.br.ix < 0.0f ? 1u : 0u) | (c.br.iy < 0.0f ? 2u : 0u) | (c.br.iz < 0.0f ? 4u : 0u);
-    c.oct7 = s ^ 7u;
+    const bool fx = c.br.ix < 0.0f, fy = c.br.iy < 0.0f, fz = c.br.iz < 0.0f;
+    c.pref1 = fx ? 0xAAu : 0x55u;
+    c.pref2 = fy ? 0xCCu : 0x33u;
+    c.pref4 = fz ? 0xF0u : 0x0Fu;
     return c;
 }
 
-// Byte k of w as a float (exact).  An integer-to-float conversion: the
-// kernel's busiest pipe is the integer ALU (58 % in ncu), and the
-// conversion's pipe is another one; a byte permute into 2^23 + b minus 2^23
-// (ALU + FMA) measured slower on c1 (71.8 against 69.1 ms per frame), and so
-// did a conversion of the low byte of the shifted word (cvt.rn.f32.u8: 61.8
-// against 60.4).
-__device__ __forceinline__ float ubyte_f(uint32_t w, int k)
+// Byte k of w as the float 2^15 + byte: one byte permute into the bits of
+// 2^15 (an integer-to-float conversion takes as many instructions, or a
+// slower pipe).
+__device__ __forceinline__ float byte_f(uint32_t w, int k)
 {
-    return __uint2float_rn((w >> (8 * k)) & 0xFFu);
+    return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7404u | (uint32_t)k << 4));
 }
+
+// The group of the root alone: the one interior child (slot 0) of a group of
+// its own.
+__device__ __forceinline__ uint2 w8_root() { return make_uint2(0u, 1u | 1u << 8); }
+__device__ __forceinline__ bool w8_any(uint2 G) { return (G.y & 0xFFu) != 0u; }
 
 // Visits node `idx`: tests its children's boxes against the ray with the
 // current best distance tbest and returns the node group of the interior
-// children hit (G) and the primitive group of the leaf children hit (P).
-// Each box is [p + q_lo * step, p + q_hi * step] per axis, which contains
-// the binary child's padded box; the slab distances are
-// fma(q, step * ix, fma(p, ix, -o * ix)), and a child is hit iff
-// max(near distances, 0) <= min(far distances, tbest) * (1 + 2^-20): the
-// binary test's acceptance, on a box that contains the binary box, so every
-// box the binary traversal enters is entered here too.
-__device__ __forceinline__ void cw8_visit(const float4* nodes, uint32_t idx, const Cw8Ray& r, float tbest, uint2& G,
-                                          uint2& P)
+// children hit (G) and the leaf group of the leaf children hit (P).  The slab
+// distances are fma(2^15 + q, step * ix, fma(p - 2^15 * step, ix, -o * ix)); a
+// child is hit iff max(near distances, 0) <= min(far distances, tbest), the
+// right side times (1 + 2^-20): the binary test's acceptance, on a box that
+// contains the binary box with a margin above these distances' rounding, so
+// every box the binary traversal enters is entered here too.
+__device__ __forceinline__ void w8_visit(const float4* nodes, uint32_t idx, const W8Ray& r, float tbest, uint2& G,
+                                         uint2& P)
 {
-    uint32_t a[8], b[8], c[8];
+    uint32_t u[8], v[8], w[8];
     const float4* n = nodes + 6 * (size_t)idx;
-    ldg256u(n, a);
-    ldg256u(n + 2, b);
-    ldg256u(n + 4, c);
-    const float px = __uint_as_float(a[0]), py = __uint_as_float(a[1]), pz = __uint_as_float(a[2]);
-    const float sx = __uint_as_float((a[3] & 0xFFu) << 23);
-    const float sy = __uint_as_float(((a[3] >> 8) & 0xFFu) << 23);
-    const float sz = __uint_as_float(((a[3] >> 16) & 0xFFu) << 23);
-    const float ax = sx * r.br.ix, ay = sy * r.br.iy, az = sz * r.br.iz;
-    const float bx = __fmaf_rn(px, r.br.ix, r.br.nx);
-    const float by = __fmaf_rn(py, r.br.iy, r.br.ny);
-    const float bz = __fmaf_rn(pz, r.br.iz, r.br.nz);
-    // near / far plane words per axis (two words = eight slots)
+    ldg256u(n, u);
+    ldg256u(n + 2, v);
+    ldg256u(n + 4, w);
+    const float ax = __uint_as_float(u[3]) * r.br.ix, bx = __fmaf_rn(__uint_as_float(u[0]), r.br.ix, r.br.nx);
+    const float ay = __uint_as_float(u[4]) * r.br.iy, by = __fmaf_rn(__uint_as_float(u[1]), r.br.iy, r.br.ny);
+    const float az = __uint_as_float(u[5]) * r.br.iz, bz = __fmaf_rn(__uint_as_float(u[2]), r.br.iz, r.br.nz);
+    const float tb = tbest * BOX_SLACK;
+    const float2 ax2 = make_float2(ax, ax), ay2 = make_float2(ay, ay), az2 = make_float2(az, az);
+    const float2 bx2 = make_float2(bx, bx), by2 = make_float2(by, by), bz2 = make_float2(bz, bz);
     const bool fx = r.br.ix < 0.0f, fy = r.br.iy < 0.0f, fz = r.br.iz < 0.0f;
-    // b = w8..w15: lo x (b0, b1), lo y (b2, b3), lo z (b4, b5), hi x (b6, b7)
-    // c = w16..w23: hi y (c0, c1), hi z (c2, c3), bits (c4, c5), positions (c6, c7)
-    const uint32_t lox[2] = {b[0], b[1]}, loy[2] = {b[2], b[3]}, loz[2] = {b[4], b[5]};
-    const uint32_t hix[2] = {b[6], b[7]}, hiy[2] = {c[0], c[1]}, hiz[2] = {c[2], c[3]};
-    const uint32_t oct4 = r.oct7 * 0x01010101u;
-    uint32_t mask = 0;
+    uint32_t miss = 0;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t qnx = fx ? hix[h] : lox[h], qfx = fx ? lox[h] : hix[h];
-        const uint32_t qny = fy ? hiy[h] : loy[h], qfy = fy ? loy[h] : hiy[h];
-        const uint32_t qnz = fz ? hiz[h] : loz[h], qfz = fz ? loz[h] : hiz[h];
-        const uint32_t bits4 = c[4 + h];
-        const uint32_t pos4 = c[6 + h] ^ (oct4 & a[6 + h]);  // interior children: slot ^ s ^ 7
+    for (int h = 1; h >= 0; --h) {
+        // near / far plane words per axis, four slots each
+        const uint32_t nx = fx ? v[4 + h] : v[2 + h], qx = fx ? v[2 + h] : v[4 + h];
+        const uint32_t ny = fy ? w[h] : v[6 + h], qy = fy ? v[6 + h] : w[h];
+        const uint32_t nz = fz ? w[4 + h] : w[2 + h], qz = fz ? w[2 + h] : w[4 + h];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float tnx = __fmaf_rn(ubyte_f(qnx, k), ax, bx);
-            const float tny = __fmaf_rn(ubyte_f(qny, k), ay, by);
-            const float tnz = __fmaf_rn(ubyte_f(qnz, k), az, bz);
-            const float tfx = __fmaf_rn(ubyte_f(qfx, k), ax, bx);
-            const float tfy = __fmaf_rn(ubyte_f(qfy, k), ay, by);
-            const float tfz = __fmaf_rn(ubyte_f(qfz, k), az, bz);
-            const float tmin = fmaxf(fmax3(tnx, tny, tnz), 0.0f);
-            const float tmax = fminf(fmin3(tfx, tfy, tfz), tbest);
-            if (tmin <= tmax * BOX_SLACK)
-                mask |= __byte_perm(bits4, 0u, 0x4440u | (uint32_t)k) << __byte_perm(pos4, 0u, 0x4440u | (uint32_t)k);
+        for (int k = 2; k >= 0; k -= 2) {
+            auto two = [&](uint32_t q, float2 a, float2 c) {
+                return __ffma2_rn(make_float2(byte_f(q, k), byte_f(q, k + 1)), a, c);
+            };
+            const float2 x0 = two(nx, ax2, bx2), y0 = two(ny, ay2, by2), z0 = two(nz, az2, bz2);
+            const float2 x1 = two(qx, ax2, bx2), y1 = two(qy, ay2, by2), z1 = two(qz, az2, bz2);
+            const float2 tn = make_float2(fmax3(x0.x, y0.x, z0.x), fmax3(x0.y, y0.y, z0.y));
+            const float2 tf = make_float2(fmin3(x1.x, y1.x, z1.x), fmin3(x1.y, y1.y, z1.y));
+            const float2 mn = make_float2(-tn.x, -tn.y);
+            const float2 d1 = __ffma2_rn(tf, make_float2(BOX_SLACK, BOX_SLACK), mn);
+            const float2 d3 = __fadd2_rn(make_float2(tb, tb), mn);
+            miss = __funnelshift_l(__float_as_uint(fmin3(d1.y, tf.y, d3.y)), miss, 1);
+            miss = __funnelshift_l(__float_as_uint(fmin3(d1.x, tf.x, d3.x)), miss, 1);
         }
     }
-    G = make_uint2(a[4], (mask & 0xFF000000u) | (a[3] >> 24));
-    P = make_uint2(a[5], mask & 0x00FFFFFFu);
+    const uint32_t hit = ~miss;
+    const uint32_t imask = v[0] & 0xFFu;
+    G = make_uint2(u[6], (hit & imask) | imask << 8);
+    P = make_uint2(u[7], (v[0] >> 8 & hit & 0xFFu) | (v[0] & 0x00FFFF00u));
 }
 
-// Takes the next child of a node group (which has one): its node index; the
-// group keeps the others.
-__device__ __forceinline__ uint32_t cw8_next(uint2& G, uint32_t oct7)
+// Takes the next child of a node group (which has one), the one the ray's
+// octant meets first: its node index; the group keeps the others.
+__device__ __forceinline__ uint32_t w8_next(uint2& G, const W8Ray& r)
 {
-    const int bit = 31 - __clz(G.y);
-    const uint32_t slot = (uint32_t)(bit - 24) ^ oct7;
-    G.y &= ~(1u << bit);
-    return G.x + __popc(G.y & ((1u << slot) - 1u) & 0xFFu);
+    uint32_t x = G.y & 0xFFu, p;
+    p = x & r.pref4;
+    x = p ? p : x;
+    p = x & r.pref2;
+    x = p ? p : x;
+    p = x & r.pref1;
+    x = p ? p : x;  // one bit
+    G.y ^= x;
+    return G.x + __popc((G.y >> 8) & (x - 1u));
 }
 
-// Tests primitive k of the 8-wide order: a 64-byte record
-// (v0, original id) (v1 - v0, leaf-ordered slot) (v2 - v0, 0) (0), read as a
-// 256-bit and a 128-bit load (the last 16 bytes are padding); on acceptance
-// the hit records the leaf-ordered slot (the storage slot every other kernel
-// indexes).
-__device__ __forceinline__ float cw8_tri(const float4* tris, uint32_t k, const Ray& ray, uint32_t& id, uint32_t& slot)
+// Takes the next leaf child of a leaf group (which has one): its first
+// primitive, and whether it has a second.
+__device__ __forceinline__ uint32_t w8_next_leaf(uint2& P, bool& two)
 {
-    float4 ta, tb;
-    ldg256(tris + 4 * (size_t)k, ta, tb);
-    const float4 tc = __ldg(tris + 4 * (size_t)k + 2);
-    id = __float_as_uint(ta.w);
-    slot = __float_as_uint(tb.w);
-    return tri_intersect(ray, v3(ta), v3(tb), v3(tc));
+    const uint32_t x = P.y & (0u - P.y) & 0xFFu;  // lowest of the bits below 8
+    P.y ^= x;
+    const uint32_t below = (x - 1u) * 0x0101u;  // x - 1 in both bytes
+    two = ((P.y >> 16) & x) != 0u;
+    return P.x + __popc((P.y >> 8) & below);
 }
 
+// Tests primitive k0 of the 8-wide order and, if two, the next.  A record is
+// 64 bytes (v0, original id) (v1 - v0, leaf-ordered slot) (v2 - v0, 0) (0),
+// read as a 256-bit and a 128-bit load; both records are fetched before
+// either test, so the two L2 round trips overlap.  On acceptance the hit
+// records the leaf-ordered slot (the storage slot every other kernel indexes).
 template <bool STATS>
-__device__ __forceinline__ void cw8_test_tri(const float4* tris, uint32_t k, const Ray& ray, Hit& h, Counters& cnt)
-{
-    if (STATS) cnt.c[C_TRIS]++;
-    uint32_t id, slot;
-    const float tt = cw8_tri(tris, k, ray, id, slot);
-    if (accept_strict(tt, id, h)) {
-        h.t = tt;
-        h.prim = id;
-        h.kind = 1;
-        h.slot = slot;
-    }
-}
-
-// Tests primitives k0 and, if two, k1: both records are fetched before
-// either test, so the two L2 round trips overlap.
-template <bool STATS>
-__device__ __forceinline__ void cw8_test_tri2(const float4* tris, uint32_t k0, uint32_t k1, bool two, const Ray& ray,
-                                              Hit& h, Counters& cnt)
+__device__ __forceinline__ void cw8_test_tri2(const float4* tris, uint32_t k0, bool two, const Ray& ray, Hit& h,
+                                              Counters& cnt)
 {
     if (STATS) cnt.c[C_TRIS] += two ? 2 : 1;
     float4 a0, b0, a1, b1;
     ldg256(tris + 4 * (size_t)k0, a0, b0);
     const float4 c0 = __ldg(tris + 4 * (size_t)k0 + 2);
-    const uint32_t k = two ? k1 : k0;
+    const uint32_t k = two ? k0 + 1u : k0;
     ldg256(tris + 4 * (size_t)k, a1, b1);
     const float4 c1 = __ldg(tris + 4 * (size_t)k + 2);
     const float t0 = tri_intersect(ray, v3(a0), v3(b0), v3(c0));
@@ -166,150 +153,14 @@ __device__ __forceinline__ void cw8_test_tri2(const float4* tris, uint32_t k0, u
     }
 }
 
-// Position of the n-th (from 0) set bit of m, which has more than n.
-__device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n)
-{
-    for (; n != 0u; --n) m &= m - 1u;
-    return (uint32_t)(__ffs(m) - 1);
-}
-
-// Per-lane record of the shared primitive phase, in shared memory: what the
-// other lanes of the warp need to test this lane's primitives for it.
-struct alignas(16) Cw8Share {
-    float4 o, d;               // the ray
-    unsigned long long best;   // (distance bits << 32) | id of the best hit so far
-    const float4* tris;        // the lane's scene's primitives (8-wide order)
-    uint32_t excl, first;      // the lane's first item in the warp's order, its first group entry
-    uint32_t slot, pad;        // storage slot of the hit that set `best`
+// Per-lane record of the extend kernel in shared memory: what a lane does not
+// need while it visits nodes (its registers then hold a node).
+struct alignas(16) W8Lane {
+    float4 o, d;         // the ray; .w: scene, path slot
+    const float4* tris;  // the lane's scene's primitives (8-wide order)
+    uint32_t prim, slot; // best hit so far: id, storage slot (NO_PRIM: none)
 };
-static_assert(sizeof(Cw8Share) == 64, "shared record is 64 bytes");
-
-// (distance, id) as one integer that orders like the strict (t, id) order
-// for non-negative distances (their bit patterns order like their values).
-__device__ __forceinline__ unsigned long long hit_key(float t, uint32_t id)
-{
-    return ((unsigned long long)__float_as_uint(t) << 32) | id;
-}
-
-// Position of the n-th (from 0) set bit of m, which has more than n: popc
-// bisection, a fixed number of steps.
-__device__ __forceinline__ uint32_t nth_bit32(uint32_t m, uint32_t n)
-{
-    uint32_t pos = 0;
-#pragma unroll
-    for (int w = 16; w >= 2; w >>= 1) {
-        const uint32_t c = (uint32_t)__popc(m & ((1u << w) - 1u));
-        if (n >= c) {
-            n -= c;
-            pos += (uint32_t)w;
-            m >>= w;
-        }
-    }
-    return pos + ((n >= (m & 1u)) ? 1u : 0u);
-}
-
-// The warp's remaining held primitives, shared out over all 32 lanes: item i
-// of the warp (lanes' items in lane order, each lane's in group and bit
-// order) is tested by lane i % 32 in step i / 32.  Each lane with items
-// publishes its ray, primitive array, best hit and item offset in its
-// Cw8Share record; a step's lanes find their owners from a ballot of the
-// owners with items in the step and the step's segment starts, fetch the
-// owner's ray from its record, and lower the owner's best (distance, id) key
-// with a shared-memory atomic minimum (a candidate counts when distance >
-// EPSILON; min over the keys is the strict-ties order, so the owner ends with
-// the hit it would get testing every item itself, in any order); the lane
-// whose candidate is the minimum after the step records its slot.  Every
-// lane of the warp calls this (warp-synchronous).
-//   held: the calling lane's group entries (entry g at held[g * stride]),
-//   readable by the other lanes of the warp; sh: the calling lane's record
-//   (the warp's lanes' records adjacent); rest: the lane has items left:
-//   `cur` (its group in progress, taken from entry j - 1) and entries
-//   j .. nh - 1.
-template <bool STATS>
-__device__ __forceinline__ void cw8_warp_prims(const float4* tris, uint2* held, Cw8Share* sh, int stride, int lane,
-                                               bool rest, uint2 cur, int j, int nh, const Ray& ray, Hit& h,
-                                               Counters& cnt)
-{
-    const unsigned full = 0xFFFFFFFFu;
-    int first = j;
-    uint32_t r = 0;
-    if (rest) {
-        if (cur.y != 0u) {
-            --first;  // j >= 1: cur came from entry j - 1
-            held[first * stride] = cur;
-        }
-        for (int g = first; g < nh; ++g) r += (uint32_t)__popc(held[g * stride].y);
-    }
-    uint32_t incl = r;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(full, incl, o);
-        if (lane >= o) incl += v;
-    }
-    const uint32_t excl = incl - r;
-    const uint32_t total = __shfl_sync(full, incl, 31);
-    const unsigned long long key0 = hit_key(h.t, h.prim);
-    if (rest) {
-        sh->o = make_float4(ray.o.x, ray.o.y, ray.o.z, 0.0f);
-        sh->d = make_float4(ray.d.x, ray.d.y, ray.d.z, 0.0f);
-        sh->best = key0;
-        sh->tris = tris;
-        sh->excl = excl;
-        sh->first = (uint32_t)first;
-    }
-    __syncwarp();
-    Cw8Share* const wsh = sh - lane;
-    for (uint32_t base = 0; base < total; base += 32u) {
-        const uint32_t idx = base + (uint32_t)lane;
-        // owners with items in this step, in lane order = the step's segments
-        const unsigned in = __ballot_sync(full, r != 0u && excl < base + 32u && incl > base);
-        const unsigned starts =
-            __reduce_or_sync(full, (r != 0u && excl >= base && excl < base + 32u) ? 1u << (excl - base) : 0u);
-        unsigned long long key = ~0ull;
-        Cw8Share* osh = wsh;
-        uint32_t slot = 0;
-        if (idx < total) {
-            // segment of this lane: starts at or before it, plus one if the
-            // step opens inside an earlier owner's items
-            const unsigned upto = lane == 31 ? starts : (starts & ((2u << lane) - 1u));
-            const uint32_t n = (uint32_t)__popc(upto) - 1u + ((starts & 1u) ? 0u : 1u);
-            const int o = (int)nth_bit32(in, n);
-            osh = wsh + o;
-            uint32_t rank = idx - osh->excl;
-            const uint2* hg = held + (o - lane);
-            int g = (int)osh->first;
-            uint2 grp = hg[g * stride];
-            uint32_t c = (uint32_t)__popc(grp.y);
-            while (rank >= c) {
-                rank -= c;
-                ++g;
-                grp = hg[g * stride];
-                c = (uint32_t)__popc(grp.y);
-            }
-            if (STATS) cnt.c[C_TRIS]++;
-            const Ray ro{v3(osh->o), v3(osh->d)};
-            uint32_t tid;
-            const float tt = cw8_tri(osh->tris, grp.x + nth_set_bit(grp.y, rank), ro, tid, slot);
-            if (tt > EPSILON) {
-                key = hit_key(tt, tid);
-                atomicMin(&osh->best, key);
-            }
-        }
-        __syncwarp();
-        if (key != ~0ull && key == *reinterpret_cast<volatile unsigned long long*>(&osh->best)) osh->slot = slot;
-        __syncwarp();
-    }
-    if (rest) {
-        const unsigned long long k = *reinterpret_cast<volatile unsigned long long*>(&sh->best);
-        if (k != key0) {
-            h.t = __uint_as_float((uint32_t)(k >> 32));
-            h.prim = (uint32_t)k;
-            h.kind = 1;
-            h.slot = *reinterpret_cast<volatile uint32_t*>(&sh->slot);
-        }
-    }
-    __syncwarp();
-}
+static_assert(sizeof(W8Lane) == 48, "lane record is 48 bytes");
 
 // Closest hit of one ray by one thread over the 8-wide BVH of a
 // triangle-only scene, for the finishing kernel: the extend kernel's node
@@ -329,12 +180,13 @@ __device__ __forceinline__ bool closest_cw8(const DevScene& sc, const Ray& ray, 
     b.slot = 0;
     if (!isnan3(ray.d)) {
         if (sc.n_tri_nodes > 0 && sc.nt > 0) {
-            const Cw8Ray cr = make_cw8ray(ray);
-            uint2 G = make_uint2(0u, (1u << (24 + (0u ^ cr.oct7))) | 1u);
+            const W8Ray cr = make_w8ray(ray);
+            const float4* nodes = sc.tri_cw8;
+            uint2 G = w8_root();
             int sp = 0;
             uint32_t steps = 0;
             for (;;) {
-                if ((G.y & 0xFF000000u) == 0u) {
+                if (!w8_any(G)) {
                     if (sp == 0) break;
                     --sp;
                     const int2 e = stk.e[sp * stk.stride];
@@ -344,8 +196,8 @@ __device__ __forceinline__ bool closest_cw8(const DevScene& sc, const Ray& ray, 
                     atomicCAS(status, ST_OK, ST_TRAVERSAL_LIMIT);
                     break;
                 }
-                const uint32_t idx = cw8_next(G, cr.oct7);
-                if (G.y & 0xFF000000u) {
+                const uint32_t idx = w8_next(G, cr);
+                if (w8_any(G)) {
                     if (sp >= stk.cap) {
                         atomicCAS(status, ST_OK, ST_STACK_OVERFLOW);
                     } else {
@@ -354,10 +206,13 @@ __device__ __forceinline__ bool closest_cw8(const DevScene& sc, const Ray& ray, 
                     }
                 }
                 uint2 P;
-                cw8_visit(sc.tri_cw8, idx, cr, b.t, G, P);
-                if (STATS) cnt.c[C_NODES] += 3;
-                for (uint32_t m = P.y; m != 0u; m &= m - 1u)
-                    cw8_test_tri<STATS>(sc.tri_cw8_prims, P.x + (uint32_t)(__ffs(m) - 1), ray, b, cnt);
+                w8_visit(nodes, idx, cr, b.t, G, P);
+                if (STATS) cnt.c[C_NODES] += 4;
+                while (w8_any(P)) {
+                    bool two;
+                    const uint32_t k = w8_next_leaf(P, two);
+                    cw8_test_tri2<STATS>(sc.tri_cw8_prims, k, two, ray, b, cnt);
+                }
             }
         }
         planes_pass<STATS>(sc, ray, b, cnt);

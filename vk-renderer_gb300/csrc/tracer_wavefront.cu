@@ -351,55 +351,52 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
     if (STATS) flush_counters(a, cnt);
 }
 
-// Primitive groups a lane of the 8-wide traversal may hold back while the
-// warp's slowest lane is still looking for its first (c1 frame, ms: 1 ->
-// 100.8, 2 -> 69.1, 4 -> 61.1, 6 -> 60.9, 8 -> 61.1, 12 -> 63.1; with the
-// shared primitive phase below: 4 -> 61.4, 5 -> 60.6, 6 -> 60.4).  Capping
-// the primitives held instead (12, 16, 20) measured 61.3-63.1.
+// Leaf groups a lane of the 8-wide traversal may hold back while the warp's
+// slowest lane is still looking for its first (c1 frame, ms: 4 -> 43.9, 6 ->
+// 42.4, 8 -> 42.4, 12 -> 42.3; each takes 8 bytes of shared memory a thread).
 constexpr int kCw8Postpone = 6;
 
-// Held primitives are tested two per lane and step while at least this many
-// lanes of the warp have some left; the rest are shared out over all 32
-// lanes (cw8_warp_prims).  1 = never shared, 33 = always.  c1 frame, ms:
-// 1 -> 60.4, 8 -> 58.1, 12 -> 58.0, 16 -> 58.4, 24 -> 61.3, 33 -> 67.8: a
-// shared step (owner look-up, the owner's ray from shared memory, an atomic
-// minimum) takes longer than a sequential one, so only the tail is shared.
-// (One primitive per sequential step and the owner found by shuffles
-// instead: 61.4 unshared, 60.1-60.4 at 8.)
-constexpr int kCw8SharedBelow = 12;
-// (Lanes whose ray is done and who hold no primitives taking their next ray
-// inside the node phase, rather than idling until the primitive phase ends:
-// 62.6 against 57.9 ms -- the fetch in every node step costs more than the
-// idle lanes.)
-
-// The extend kernel over the compressed 8-wide BVH (triangle scenes; strict
-// ties).  Same phases as wf_extend_bvh: idle lanes fetch rays; all lanes visit
-// 8-wide nodes (one per lane and step: eight quantised slab tests, the hit
-// interior children become a node group on the stack, the hit leaves a
-// primitive group held back) until every lane still tracing holds some
-// primitives, lanes that hold fewer than kCw8Postpone groups going on; then
-// all lanes test their held primitives, two per lane and step (both records
-// fetched before either test), the warp sharing out the last ones.  Node
-// groups are visited nearest-octant first; which boxes are entered depends
-// on the order, the closest hit under strict ties does not.
-// 64 registers, eight 128-thread blocks per SM; bounds for 10 or 12 blocks
-// (48 or 40 registers) spill 190 / 298 bytes and measured 65.7 / 75.0 ms on
-// the c1 frame against 60.4.
+// The extend kernel over the 8-wide BVH (triangle scenes; strict ties).
+// Phases as in wf_extend_bvh: idle lanes fetch rays; all lanes visit 8-wide
+// nodes (one per lane and step: eight quantised slab tests, the hit interior
+// children become a node group on the stack, the hit leaves a leaf group held
+// back) until every lane still tracing holds some leaves, lanes that hold
+// fewer than kCw8Postpone groups going on; then all lanes test their held
+// leaves, one leaf (at most two triangles, both records fetched before
+// either test) per lane and step.  Node groups are visited nearest-octant
+// first; which boxes are entered depends on the order, the closest hit under
+// strict ties does not.
+//
+// What bounds it (c1 scene, ncu): L1's data pipe 68 %, the integer pipe 62 %,
+// issue 60 %, all three by the node visits (36 a ray, 5-10 triangle tests).
+// So the node is three 256-bit loads, not more and narrower ones: a 128-byte
+// node with its planes as 16-bit floats saves the byte conversions but was
+// slower here, c1 frame 52.0 ms against 46.3 (seven or eight loads a visit,
+// L1 83 %), though faster in the finishing kernels.  Pairs of slots share one
+// packed multiply-add (43.1 against 46.3 ms).  c1 frame over the steps: 58.0
+// ms with binary leaves as leaf children (43 tests a ray), 54.2 with leaves
+// split and the collapse planned by cost, 42.4 with this node and kernel.
+// Sharing the last leaves of a phase out over the warp no longer pays (43.1;
+// it needs 16 more bytes and the phase is a sixth of the work now), nor does
+// ending the node phase once 4, 6, 8 or 12 lanes idle (45.1, 44.1, 43.8, 44.0).
+// 72 registers, seven 128-thread blocks per SM (64 registers and eight
+// blocks: 34 bytes spilled, 43.8 ms; 80 and six: 42.8).
 template <bool STATS, bool MULTI, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
+__global__ void __launch_bounds__(BLOCK, 896 / BLOCK)
     wf_extend_cw8(TraceArgs a, WfState s, int qsel, const TraceArgs* slots)
 {
     extern __shared__ int smem[];
     const unsigned full = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
-    // stack of node groups, then held primitive groups (entry j of a thread
-    // at j * BLOCK + threadIdx.x), then the threads' shared-phase records
+    // stack of node groups, then held leaf groups (entry j of a thread at
+    // j * BLOCK + threadIdx.x), then the threads' records.  The stack holds at
+    // most one group per level of the tree (siblings left behind on the way
+    // down), and stack_depth is at least its number of levels.
     uint2* stk = reinterpret_cast<uint2*>(smem) + threadIdx.x;
     uint2* held = reinterpret_cast<uint2*>(smem) + (size_t)a.stack_depth * BLOCK + threadIdx.x;
-    Cw8Share* shr =
-        reinterpret_cast<Cw8Share*>(reinterpret_cast<uint2*>(smem) + ((size_t)a.stack_depth + kCw8Postpone) * BLOCK) +
+    W8Lane* rec =
+        reinterpret_cast<W8Lane*>(reinterpret_cast<uint2*>(smem) + ((size_t)a.stack_depth + kCw8Postpone) * BLOCK) +
         threadIdx.x;
-    const int cap = (int)a.stack_depth;
     const uint32_t total = s.count[qsel];
     const uint32_t* queue = qsel ? s.queue[1] : s.queue[0];
     if (blockIdx.x == 0 && threadIdx.x == 0) s.count[qsel ^ 1] = 0;
@@ -407,14 +404,13 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
 #pragma unroll
     for (int k = 0; k < C_COUNT; ++k) cnt.c[k] = 0;
     bool has = false, exhausted = false;
-    uint32_t pid = 0, scene = 0, steps = 0;
-    Ray ray{};
-    Cw8Ray cr{};
-    Hit h{};
+    uint32_t steps = 0;
+    W8Ray cr{};
+    float tbest = 0.0f;
     uint2 G = make_uint2(0u, 0u);
     int sp = 0, nh = 0;
-    const float4* nodes = nullptr;
-    const float4* tris = nullptr;
+    // one scene: its nodes (a kernel argument); batched: the lane's scene's
+    const float4* my_nodes = nullptr;
     // idle lanes take the next rays of the queue (warp-aggregated: one
     // atomic per warp and call)
     auto fetch = [&]() {
@@ -430,39 +426,43 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
             exhausted = true;
             return;
         }
-        pid = queue[qi];
-        scene = MULTI ? s.scene_of[pid] : 0;
+        const uint32_t pid = queue[qi];
+        const uint32_t scene = MULTI ? s.scene_of[pid] : 0;
         const DevScene& sc = SCENE_ARGS(MULTI, a, slots, scene).sc;
         const float4 ro = s.ray_o[pid];
         const float4 rd = s.ray_d[pid];
-        ray = Ray{v3(ro), v3(rd)};
-        h.t = ro.w;
-        h.prim = 0;  // see accept_strict
-        h.kind = 0;
-        h.slot = 0;
+        const Ray ray{v3(ro), v3(rd)};
         steps = 0;
         if (STATS) cnt.c[C_CLOSEST]++;
         has = true;
         if (isnan3(ray.d) || !(sc.n_tri_nodes > 0 && sc.nt > 0)) {
             // no BVH work: NaN directions hit nothing; planes only
+            Hit h{ro.w, 0u, 0, 0u};
             if (!isnan3(ray.d)) planes_pass<STATS>(sc, ray, h, cnt);
             if (STATS && h.kind) cnt.c[C_HITS]++;
             s.hit[pid] = make_uint4(__float_as_uint(h.t), h.prim, h.slot, (uint32_t)h.kind);
             has = false;
         } else {
-            cr = make_cw8ray(ray);
-            nodes = sc.tri_cw8;
-            tris = sc.tri_cw8_prims;
-            // the root: the one interior child (slot 0) of a group of its own
-            G = make_uint2(0u, (1u << (24 + (0u ^ cr.oct7))) | 1u);
+            rec->o = make_float4(ro.x, ro.y, ro.z, __uint_as_float(scene));
+            rec->d = make_float4(rd.x, rd.y, rd.z, __uint_as_float(pid));
+            rec->tris = sc.tri_cw8_prims;
+            rec->prim = 0u;  // see accept_strict
+            rec->slot = NO_PRIM;
+            tbest = ro.w;
+            cr = make_w8ray(ray);
+            if (MULTI) my_nodes = sc.tri_cw8;
+            G = w8_root();
             sp = 0;
         }
     };
     // a ray whose traversal is over and whose primitives are all tested:
     // planes, then its result
     auto finish_ray = [&]() {
-        const DevScene& sc = SCENE_ARGS(MULTI, a, slots, scene).sc;
-        planes_pass<STATS>(sc, ray, h, cnt);
+        const float4 o = rec->o, d = rec->d;
+        const uint32_t pid = __float_as_uint(d.w), slot = rec->slot;
+        Hit h{tbest, rec->prim, slot != NO_PRIM ? 1 : 0, slot != NO_PRIM ? slot : 0u};
+        const DevScene& sc = SCENE_ARGS(MULTI, a, slots, __float_as_uint(o.w)).sc;
+        planes_pass<STATS>(sc, Ray{v3(o), v3(d)}, h, cnt);
         if (STATS && h.kind) cnt.c[C_HITS]++;
         s.hit[pid] = make_uint4(__float_as_uint(h.t), h.prim, h.slot, (uint32_t)h.kind);
         has = false;
@@ -476,69 +476,55 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
         }
         // 2) nodes, until every lane still tracing holds primitives
         for (;;) {
-            const bool search = has && nh < kCw8Postpone && ((G.y & 0xFF000000u) != 0u || sp > 0);
+            const bool search = has && nh < kCw8Postpone && (w8_any(G) || sp > 0) && steps < a.trav_limit;
             if (!__any_sync(full, search && nh == 0)) break;
             if (search) {
-                if ((G.y & 0xFF000000u) == 0u) {
+                ++steps;
+                if (!w8_any(G)) {
                     --sp;
                     G = stk[sp * BLOCK];
                 }
-                if (++steps > a.trav_limit) {
-                    atomicCAS(a.status, ST_OK, ST_TRAVERSAL_LIMIT);
-                    G = make_uint2(0u, 0u);
-                    sp = 0;
-                } else {
-                    const uint32_t idx = cw8_next(G, cr.oct7);
-                    if (G.y & 0xFF000000u) {
-                        if (sp >= cap) {
-                            atomicCAS(a.status, ST_OK, ST_STACK_OVERFLOW);
-                        } else {
-                            stk[sp * BLOCK] = G;
-                            ++sp;
-                        }
-                    }
-                    uint2 P;
-                    cw8_visit(nodes, idx, cr, h.t, G, P);
-                    if (STATS) cnt.c[C_NODES] += 3;
-                    if (P.y) {
-                        held[nh * BLOCK] = P;
-                        ++nh;
-                    }
+                const uint32_t idx = w8_next(G, cr);
+                if (w8_any(G)) {
+                    stk[sp * BLOCK] = G;
+                    ++sp;
                 }
+                uint2 P;
+                w8_visit(MULTI ? my_nodes : a.sc.tri_cw8, idx, cr, tbest, G, P);
+                if (STATS) cnt.c[C_NODES] += 4;
+                held[nh * BLOCK] = P;
+                nh += w8_any(P) ? 1 : 0;
             }
         }
-        // 3) the held primitives: two per lane and step while at least
-        // kCw8SharedBelow lanes have some left, then the rest shared out
-        // over the warp
-        {
+        if (has && steps >= a.trav_limit && (w8_any(G) || sp > 0)) {  // give up the rest of this ray's nodes
+            atomicCAS(a.status, ST_OK, ST_TRAVERSAL_LIMIT);
+            G = make_uint2(0u, 0u);
+            sp = 0;
+        }
+        // 3) the held leaves: one leaf (two primitives at most) per lane and step
+        if (nh > 0) {
             int j = 0;
             uint2 cur = make_uint2(0u, 0u);
+            const Ray ray{v3(rec->o), v3(rec->d)};
+            const float4* tris = MULTI ? rec->tris : a.sc.tri_cw8_prims;
+            Hit h{tbest, rec->prim, 1, rec->slot};
             for (;;) {
-                const bool lf = has && (cur.y != 0u || j < nh);
-                if (__popc(__ballot_sync(full, lf)) < kCw8SharedBelow) break;
-                if (lf) {
-                    if (cur.y == 0u) {
-                        cur = held[j * BLOCK];
-                        ++j;
-                    }
-                    const uint32_t k0 = cur.x + (uint32_t)(__ffs(cur.y) - 1);
-                    cur.y &= cur.y - 1u;
-                    if (cur.y == 0u && j < nh) {
-                        cur = held[j * BLOCK];
-                        ++j;
-                    }
-                    const bool two = cur.y != 0u;
-                    const uint32_t k1 = two ? cur.x + (uint32_t)(__ffs(cur.y) - 1) : k0;
-                    if (two) cur.y &= cur.y - 1u;
-                    cw8_test_tri2<STATS>(tris, k0, k1, two, ray, h, cnt);
+                if (!w8_any(cur)) {
+                    if (j == nh) break;
+                    cur = held[j * BLOCK];
+                    ++j;
                 }
+                bool two;
+                const uint32_t k = w8_next_leaf(cur, two);
+                cw8_test_tri2<STATS>(tris, k, two, ray, h, cnt);
             }
-            const bool rest = has && (cur.y != 0u || j < nh);
-            if (__any_sync(full, rest)) cw8_warp_prims<STATS>(tris, held, shr, BLOCK, lane, rest, cur, j, nh, ray, h, cnt);
+            tbest = h.t;
+            rec->prim = h.prim;
+            rec->slot = h.slot;
+            nh = 0;
         }
-        nh = 0;
         // 4) finished rays: planes and the result
-        if (has && (G.y & 0xFF000000u) == 0u && sp == 0) finish_ray();
+        if (has && !w8_any(G) && sp == 0) finish_ray();
     }
     if (STATS) flush_counters(a, cnt);
 }
@@ -754,7 +740,7 @@ static void smem_attr(K k, size_t smem)
 // reference) or held primitive groups (8-wide: 8 B per group).
 static size_t wf_extend_smem(size_t stack_depth, uint32_t block, int wide)
 {
-    return (stack_depth * 8 + (wide == WF_WIDTH_8 ? kCw8Postpone * 8 + sizeof(Cw8Share) : kPostpone * 4)) * block;
+    return (stack_depth * 8 + (wide == WF_WIDTH_8 ? kCw8Postpone * 8 + sizeof(W8Lane) : kPostpone * 4)) * block;
 }
 
 template <int TIE, bool STATS, bool MULTI, int BLOCK>
