@@ -121,7 +121,7 @@ struct tracer_ctx {
     DevBuf<uint2> hit;
     DevBuf<float4> linear;
     DevBuf<unsigned long long> stats;
-    DevBuf<int> status;
+    int* status = nullptr;  // traversal status word in pinned host memory: kernels write it only on an error
     uint32_t last_mask = 0;
     // wavefront path state (scratch, one slot per pixel)
     DevBuf<float4> wf_ray_o, wf_ray_d, wf_acc, wf_mask, wf_accum;
@@ -215,30 +215,33 @@ template <class T> cudaError_t upload(DevBuf<T>& b, const T* src, size_t n)
 }
 
 // Bounded wait on an event: polls instead of blocking so a stuck GPU turns
-// into TRACER_ERR_TIMEOUT rather than a hang.
-int wait_event(tracer_ctx* c, cudaEvent_t ev)
+// into TRACER_ERR_TIMEOUT rather than a hang.  The first spin_us microseconds
+// without sleeping: a sleep of any length returns after some 100 us here
+// (present pass of one context back to back: 125 us a call with sleeps from
+// the start, 47 with a spin), longer than many whole traces.
+constexpr int kSpinResult = 2000;  // the end of a trace
+constexpr int kSpinRound = 100;    // a queue length, three rounds behind the launches
+int wait_event(tracer_ctx* c, cudaEvent_t ev, int spin_us)
 {
     auto t0 = std::chrono::steady_clock::now();
     for (;;) {
         cudaError_t e = cudaEventQuery(ev);
         if (e == cudaSuccess) return TRACER_OK;
         if (e != cudaErrorNotReady) return cuda_fail(c, e, "waiting for the GPU");
-        auto ms = std::chrono::duration_cast<std::chrono::milliseconds>(std::chrono::steady_clock::now() - t0).count();
-        if (ms > (long long)c->timeout_ms)
+        auto us = std::chrono::duration_cast<std::chrono::microseconds>(std::chrono::steady_clock::now() - t0).count();
+        if (us > (long long)c->timeout_ms * 1000)
             return fail(c, TRACER_ERR_TIMEOUT, "GPU did not finish within %u ms", c->timeout_ms);
-        std::this_thread::sleep_for(std::chrono::microseconds(50));
+        if (us >= spin_us) std::this_thread::sleep_for(std::chrono::microseconds(50));
     }
 }
 
 int finish(tracer_ctx* c)
 {
     if (!c->pending) return TRACER_OK;
-    int r = wait_event(c, c->done);
+    int r = wait_event(c, c->done, kSpinResult);
     if (r != TRACER_OK) return r;
     c->pending = false;
-    int st = 0;
-    cudaError_t e = cudaMemcpy(&st, c->status.p, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(c, e, "reading the device status");
+    const int st = *static_cast<volatile int*>(c->status);
     if (st == ST_TRAVERSAL_LIMIT)
         return fail(c, TRACER_ERR_TRAVERSAL_LIMIT, "a ray exceeded the BVH traversal step limit");
     if (st == ST_STACK_OVERFLOW)
@@ -374,7 +377,7 @@ int run_wavefront(tracer_ctx* c, const TraceArgs& a, WfConfig& wc, size_t nslots
         if (e == cudaSuccess) e = cudaEventRecord(c->count_events[slot], st);
         if (e == cudaSuccess && r >= (uint64_t)kCountLag) {
             const int old = (int)((r - kCountLag) % kCountSlots);
-            int w = wait_event(c, c->count_events[old]);
+            int w = wait_event(c, c->count_events[old], kSpinRound);
             if (w != TRACER_OK) return w;
             const uint32_t live = c->pinned_counts[old];
             if (live == 0) break;
@@ -583,7 +586,8 @@ int tracer_create(tracer_ctx** out, int cuda_device)
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = dalloc(c->stats, C_COUNT);
-    if (e == cudaSuccess) e = dalloc(c->status, 1);
+    if (e == cudaSuccess) e = cudaMallocHost(&c->status, sizeof(int));
+    if (e == cudaSuccess) *c->status = 0;
     if (e == cudaSuccess) e = dalloc(c->wf_count, 4);
     if (e == cudaSuccess) e = cudaMallocHost(&c->pinned_counts, sizeof(uint32_t) * kCountSlots);
     if (e == cudaSuccess) {
@@ -605,7 +609,7 @@ void tracer_destroy(tracer_ctx* c)
 {
     if (!c) return;
     cudaSetDevice(c->device);
-    if (c->pending && c->done) wait_event(c, c->done);
+    if (c->pending && c->done) wait_event(c, c->done, kSpinResult);
     c->scene.release();
     c->batch.release();
     c->adj.release();
@@ -629,7 +633,7 @@ void tracer_destroy(tracer_ctx* c)
     c->hit.release();
     c->linear.release();
     c->stats.release();
-    c->status.release();
+    if (c->status) cudaFreeHost(c->status);
     release_wavefront(c);
     c->wf_count.release();
     if (c->pinned_counts) cudaFreeHost(c->pinned_counts);
@@ -896,12 +900,12 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
     a.hit = (mask & (1u << TRACER_AOV_PRIMARY_HIT)) ? c->hit.p : nullptr;
     a.linear = (mask & (1u << TRACER_AOV_LINEAR)) ? c->linear.p : nullptr;
     a.stats = c->stats.p;
-    a.status = c->status.p;
+    a.status = c->status;
     const int stats = (p->stats || (mask & (1u << TRACER_AOV_STATS))) ? 1 : 0;
     if (stats) c->last_mask |= 1u << TRACER_AOV_STATS;
     cudaStream_t st = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : c->stream;
-    e = cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * C_COUNT, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->status.p, 0, sizeof(int), st);
+    *c->status = 0;  // nothing of this context is in flight (finish above)
+    if (stats) e = cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * C_COUNT, st);
     if (e != cudaSuccess) return cuda_fail(c, e, "trace set-up");
     c->last_kernel = kernel;
     c->last_rounds = 0;
@@ -965,7 +969,7 @@ int tracer_measure_l2_read(tracer_ctx* c, size_t bytes, uint32_t passes, double*
     if (e == cudaSuccess) e = launch_l2_read(buf.p, bytes, passes, sink.p, blocks, c->stream);
     if (e == cudaSuccess) e = cudaEventRecord(ev[1], c->stream);
     if (e == cudaSuccess) {
-        r = wait_event(c, ev[1]);
+        r = wait_event(c, ev[1], kSpinResult);
         float ms = 0.0f;
         if (r == TRACER_OK) e = cudaEventElapsedTime(&ms, ev[0], ev[1]);
         if (r == TRACER_OK && e == cudaSuccess && ms > 0.0f) *gbs = (double)bytes * passes / (ms * 1e-3) / 1e9;
@@ -1596,15 +1600,15 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
         a.rgba32f = (mask & (1u << TRACER_AOV_RGBA32F)) ? c->b_rgba32f.p + base[k] : nullptr;
         a.hit = (mask & (1u << TRACER_AOV_PRIMARY_HIT)) ? c->b_hit.p + base[k] : nullptr;
         a.stats = c->stats.p;
-        a.status = c->status.p;
+        a.status = c->status;
         a.pixel_base = (uint32_t)base[k];
         a.num_slots = (uint32_t)total;
         c->batch_w[k] = p.width;
         c->batch_h[k] = p.height;
     }
     e = cudaMemcpyAsync(c->batch_slots.p, slots, sizeof(TraceArgs) * n, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * C_COUNT, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->status.p, 0, sizeof(int), st);
+    *c->status = 0;  // nothing of this context is in flight (finish above)
+    if (e == cudaSuccess && stats) e = cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * C_COUNT, st);
     if (e != cudaSuccess) return cuda_fail(c, e, "batch set-up");
     c->last_kernel = kernel;
     c->last_rounds = 0;
@@ -1830,7 +1834,7 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
     }
     if (e == cudaSuccess) e = cudaMemsetAsync(ab.grad.p, 0, ng * sizeof(double), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * C_COUNT, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->status.p, 0, sizeof(int), st);
+    *c->status = 0;  // nothing of this context is in flight (finish above)
     if (e != cudaSuccess) return cuda_fail(c, e, "adjoint set-up");
 
     TraceArgs a;
@@ -1855,7 +1859,7 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
     const uint32_t nn = std::max(std::max(s.n_tri_nodes, s.n_sph_nodes), s.n_cw8_nodes);
     a.trav_limit = trav_limit(c, nn);
     a.stats = c->stats.p;
-    a.status = c->status.p;
+    a.status = c->status;
     c->last_rounds = 0;
     c->last_prof_rounds = 0;
     c->last_round_entries = 0;
@@ -2159,11 +2163,11 @@ extern "C" int tracer_trace_whitted(tracer_ctx* c, const tracer_frame* f, const 
     a.rgba8 = (mask & (1u << TRACER_AOV_RGBA8)) ? c->rgba8.p : nullptr;
     a.rgba32f = (mask & (1u << TRACER_AOV_RGBA32F)) ? c->rgba32f.p : nullptr;
     a.stats = c->stats.p;
-    a.status = c->status.p;
+    a.status = c->status;
     const int stats = (p->stats || (mask & (1u << TRACER_AOV_STATS))) ? 1 : 0;
     cudaStream_t st = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : c->stream;
-    e = cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * C_COUNT, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->status.p, 0, sizeof(int), st);
+    *c->status = 0;  // nothing of this context is in flight (finish above)
+    if (stats) e = cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * C_COUNT, st);
     if (e != cudaSuccess) return cuda_fail(c, e, "trace set-up");
     c->width = p->width;
     c->height = p->height;
