@@ -201,9 +201,10 @@ typedef struct tracer_trace_params {
     uint32_t wavefront;     /* wavefront extend kernel: resident CTAs per SM; 0 = occupancy maximum */
     uint32_t aov_mask;      /* bit (1 << TRACER_AOV_*) per image written; 0 = RGBA8 only */
     uint32_t stats;         /* nonzero: count rays, node fetches and primitive tests */
-    uint32_t bvh_width;     /* wavefront traversal: 0 = auto (= 2), 2 = the binary BVH, 4 = 4-wide nodes
-                               collapsed from it (same boxes, same hits; measured slower on sparse
-                               triangle soups, where it tests boxes the binary traversal culls) */
+    uint32_t bvh_width;     /* wavefront traversal: 0 = auto (8-wide nodes over the triangles, in the rounds
+                               of triangle-only scenes and in every path kernel), 2 = the binary BVH,
+                               4 = 4-wide nodes collapsed from it in the rounds (measured slower on
+                               sparse triangle soups), 8 = 8-wide (triangle-only scenes); same hits */
     uint32_t tail_paths;    /* wavefront: once fewer than this many paths are live, one kernel runs each of
                                them to the end of its pixel (remaining bounces and samples) instead of
                                further rounds; a frame with fewer pixels than this runs no round at all.
@@ -377,7 +378,8 @@ int tracer_last_rounds(tracer_ctx* ctx, tracer_round_info* out, uint32_t cap, ui
  * scene once at start-up, then calls this entry point per frame.
  *
  * It runs the wavefront kernels on the scene uploaded to ctx, 128 threads per
- * block, binary traversal (bvh_width 0 or 2; other widths are refused; the
+ * block (the rounds with the binary traversal, the finishing launch with the
+ * 8-wide one unless bvh_width is 2; widths other than 0 and 2 are refused; the
  * block field is not read), with no queue length read back: when the image
  * has fewer pixels than tail_paths -- always with the automatic threshold,
  * which is the extend kernel's resident threads as in tracer_trace -- the

@@ -49,16 +49,16 @@ struct SceneBuffers {
     DevBuf<float4> tri, mats, sph_geo, sph_rec, planes, tri_nodes, sph_nodes;
     DevBuf<float4> tri_wide, sph_wide;  // the BVHs as 4-wide nodes
     DevBuf<float4> tri_enc, sph_enc;    // the binary BVHs with pre-encoded child references
-    DevBuf<float4> tri_cw8, tri_cw8_prims;  // compressed 8-wide BVH over the triangles, triangles in its order
+    DevBuf<float4> tri_cw8, tri_cw8_prims;  // 8-wide BVH over the triangles, triangles in its order
     DevBuf<uint32_t> sph_id, emit;
     uint32_t nt = 0, nm = 0, ns = 0, np = 0, ne = 0;
     uint32_t n_tri_nodes = 0, n_sph_nodes = 0;
     uint32_t depth = 0;       // deepest BVH
     uint32_t wide_depth = 0;  // deepest 4-wide BVH
     bool wide = false;        // 4-wide nodes present
-    uint32_t cw8_depth = 0;   // levels of the 8-wide BVH
+    uint32_t cw8_depth = 0;   // levels of the 8-wide BVH (0: none)
     uint32_t n_cw8_nodes = 0;
-    bool cw8 = false;         // 8-wide BVH present (triangle-only scenes)
+    bool cw8 = false;         // the extend kernel may use it (triangle-only scenes)
     bool bvh = false;
     bool loaded = false;
     void release()
@@ -426,7 +426,7 @@ int pick_width_for(tracer_ctx* c, const tracer_trace_params* p, bool have_wide, 
         if (!have_cw8) return fail(c, TRACER_ERR_INVALID_ARG, "the scene has no 8-wide BVH (triangle-only scenes)");
         // its own need, whatever the caller's stack_depth (which bounds the
         // binary traversal's): split leaves can make it the deeper tree
-        if (stack < cw8_depth) stack = cw8_depth;
+        stack = std::max(stack, cw8_depth);
         wide = WF_WIDTH_8;
         return TRACER_OK;
     }
@@ -475,6 +475,11 @@ bool camera_inverse(const tracer_camera& cam, float out[9])
         }
     return true;
 }
+
+// The caller asked for the binary (or 4-wide) traversal by name: then the
+// per-thread traversals of the shade and finishing kernels are binary too;
+// otherwise they use the triangles' 8-wide BVH wherever the scene has one.
+bool binary_asked(const tracer_trace_params* p) { return p->bvh_width == 2 || p->bvh_width == 4; }
 
 int pick_width(tracer_ctx* c, const tracer_trace_params* p, uint32_t& stack, int& wide)
 {
@@ -763,7 +768,7 @@ int tracer_upload_scene(tracer_ctx* c, const tracer_scene_desc* d)
     std::vector<W8Node> cw8;
     std::vector<float4> cw8_prims;
     uint32_t cw8_depth = 0;
-    const bool cw8_ok = s.bvh && s.nt > 0 && s.ns == 0 && make_cw8(tnodes, tri, cw8, cw8_prims, cw8_depth);
+    const bool cw8_ok = s.bvh && s.nt > 0 && make_cw8(tnodes, tri, cw8, cw8_prims, cw8_depth);
 
     cudaError_t e = upload(s.tri, tri.data(), tri.size());
     if (e == cudaSuccess) e = upload(s.mats, reinterpret_cast<const float4*>(d->materials), 3 * (size_t)s.nm);
@@ -789,8 +794,8 @@ int tracer_upload_scene(tracer_ctx* c, const tracer_scene_desc* d)
         return cuda_fail(c, e, "scene upload");
     }
     s.wide = wide_ok;
-    s.cw8 = cw8_ok;
-    s.cw8_depth = cw8_depth;
+    s.cw8 = cw8_ok && s.ns == 0;
+    s.cw8_depth = cw8_ok ? cw8_depth : 0u;
     s.n_cw8_nodes = cw8_ok ? (uint32_t)cw8.size() : 0u;
     s.loaded = true;
     ++c->scene_version;
@@ -892,7 +897,7 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
     a.rr_start = p->rr_start;
     a.sky = V3{p->sky[0], p->sky[1], p->sky[2]};
     a.sky_on = !(p->sky[0] == 0.0f && p->sky[1] == 0.0f && p->sky[2] == 0.0f);
-    a.stack_depth = stack;
+    a.stack_depth = std::max(stack, s.cw8_depth);
     const uint32_t nn = std::max(std::max(s.n_tri_nodes, s.n_sph_nodes), s.n_cw8_nodes);
     a.trav_limit = trav_limit(c, nn);
     a.rgba8 = (mask & (1u << TRACER_AOV_RGBA8)) ? c->rgba8.p : nullptr;
@@ -934,9 +939,10 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
         uint32_t wstack = stack;
         r = pick_width(c, p, wstack, wc.wide);
         if (r != TRACER_OK) return r;
-        a.stack_depth = wstack;
         if (wc.wide == WF_WIDTH_8) wc.cw8_stack = s.cw8_depth;
-        if (wc.wide != WF_WIDTH_8) a.sc.tri_cw8 = a.sc.tri_cw8_prims = nullptr;  // finishing kernel: binary too
+        if (binary_asked(p)) a.sc.tri_cw8 = a.sc.tri_cw8_prims = nullptr;
+        else wstack = std::max(wstack, s.cw8_depth);
+        a.stack_depth = wstack;
         r = run_wavefront(c, a, wc, npx, (uint64_t)p->spp * p->max_depth + 1, wstack, p->wavefront, p->tail_paths, st);
         if (r != TRACER_OK) return r;
     }
@@ -1171,11 +1177,12 @@ extern "C" int tracer_trace_noalloc(tracer_ctx* c, const tracer_frame* f, const 
                     p->bvh_width);
     const SceneBuffers& s = c->scene;
     const uint32_t need = s.bvh ? (s.depth > 1 ? s.depth : 1) : 0;
-    const uint32_t stack = p->stack_depth ? p->stack_depth : need;
+    uint32_t stack = p->stack_depth ? p->stack_depth : need;
     if (s.bvh && stack < need)
         return fail(c, TRACER_ERR_STACK_OVERFLOW, "stack depth %u below the BVH depth %u", stack, need);
     if ((size_t)stack * 256 * 8 > 200 * 1024)
         return fail(c, TRACER_ERR_INVALID_ARG, "stack depth %u exceeds shared memory", stack);
+    stack = std::max(stack, s.cw8_depth);
     if (cudaSetDevice(c->device) != cudaSuccess) return fail(c, TRACER_ERR_CUDA, "cannot select device %d", c->device);
     unsigned char* base = nullptr;
     int r = noalloc_scratch(c, &base);
@@ -1185,7 +1192,11 @@ extern "C" int tracer_trace_noalloc(tracer_ctx* c, const tracer_frame* f, const 
     std::memset(&a, 0, sizeof a);
     a.sc = DevScene{s.tri.p, s.mats.p, s.sph_geo.p, s.sph_id.p, s.sph_rec.p, s.planes.p, s.emit.p, s.tri_nodes.p,
                     s.sph_nodes.p, s.nt, s.nm, s.ns, s.np, s.ne, s.n_tri_nodes, s.n_sph_nodes,
-                    s.tri_wide.p, s.sph_wide.p, s.tri_enc.p, s.sph_enc.p, nullptr, nullptr};  // binary traversal only
+                    s.tri_wide.p, s.sph_wide.p, s.tri_enc.p, s.sph_enc.p, nullptr, nullptr};
+    if (!binary_asked(p)) {  // the finishing kernel's traversal; the rounds' is binary
+        a.sc.tri_cw8 = s.tri_cw8.p;
+        a.sc.tri_cw8_prims = s.tri_cw8_prims.p;
+    }
     a.fr.aspect = f->aspect_ratio;
     a.fr.seed = f->seed;
     a.fr.cpos = V3{f->camera.pos[0], f->camera.pos[1], f->camera.pos[2]};
@@ -1346,8 +1357,8 @@ void pack_scene(const tracer_scene_desc& d, PackedScene& out)
         const float* em = d.spheres[i].mat.emissive;
         if (!(em[0] == 0.0f && em[1] == 0.0f && em[2] == 0.0f)) out.emit.push_back(i);
     }
-    out.cw8_ok = d.num_triangles > 0 && d.num_spheres == 0 &&
-                 make_cw8(out.tnodes, out.tri, out.cw8, out.cw8_prims, out.cw8_depth);
+    out.cw8_ok = d.num_triangles > 0 && make_cw8(out.tnodes, out.tri, out.cw8, out.cw8_prims, out.cw8_depth);
+    if (!out.cw8_ok) out.cw8_depth = 0;
 }
 
 int validate_desc(tracer_ctx* c, const tracer_scene_desc& d, uint32_t k)
@@ -1403,14 +1414,14 @@ extern "C" int tracer_upload_scenes(tracer_ctx* c, const tracer_scene_desc* desc
     std::vector<Off> off(n);
     bool wide_all = true, cw8_all = true;
     for (uint32_t k = 0; k < n; ++k)
-        cw8_all = cw8_all && packed[k].cw8_ok;
+        cw8_all = cw8_all && packed[k].cw8_ok && descs[k].num_spheres == 0;
     for (uint32_t k = 0; k < n; ++k) {
         const tracer_scene_desc& d = descs[k];
         const PackedScene& p = packed[k];
         off[k] = Off{tri.size(),    mats.size(),  geo.size(),  rec.size(),  planes.size(),
                      tnodes.size(), snodes.size(), sid.size(), emit.size(), twide.size(),
                      swide.size(),  tenc.size(),  senc.size(), tcw8.size(), tcw8p.size()};
-        if (cw8_all) {  // 6 and 4 float4 per record: every scene's part stays 32-byte aligned
+        if (p.cw8_ok) {  // 6 and 4 float4 per record: every scene's part stays 32-byte aligned
             const float4* cn = reinterpret_cast<const float4*>(p.cw8.data());
             tcw8.insert(tcw8.end(), cn, cn + 6 * p.cw8.size());
             tcw8p.insert(tcw8p.end(), p.cw8_prims.begin(), p.cw8_prims.end());
@@ -1454,8 +1465,8 @@ extern "C" int tracer_upload_scenes(tracer_ctx* c, const tracer_scene_desc* desc
     if (e == cudaSuccess) e = upload(b.sph_enc, senc.data(), senc.size());
     if (e == cudaSuccess && wide_all) e = upload(b.tri_wide, twide.data(), twide.size());
     if (e == cudaSuccess && wide_all) e = upload(b.sph_wide, swide.data(), swide.size());
-    if (e == cudaSuccess && cw8_all) e = upload(b.tri_cw8, tcw8.data(), tcw8.size());
-    if (e == cudaSuccess && cw8_all) e = upload(b.tri_cw8_prims, tcw8p.data(), tcw8p.size());
+    if (e == cudaSuccess) e = upload(b.tri_cw8, tcw8.data(), tcw8.size());
+    if (e == cudaSuccess) e = upload(b.tri_cw8_prims, tcw8p.data(), tcw8p.size());
     if (e != cudaSuccess) {
         b.release();
         return cuda_fail(c, e, "batch upload");
@@ -1481,8 +1492,8 @@ extern "C" int tracer_upload_scenes(tracer_ctx* c, const tracer_scene_desc* desc
                                       wide_all ? at(b.tri_wide, off[k].twide) : nullptr,
                                       wide_all ? at(b.sph_wide, off[k].swide) : nullptr,
                                       at(b.tri_enc, off[k].tenc), at(b.sph_enc, off[k].senc),
-                                      cw8_all ? at(b.tri_cw8, off[k].tcw8) : nullptr,
-                                      cw8_all ? at(b.tri_cw8_prims, off[k].tcw8p) : nullptr};
+                                      p.cw8_ok ? at(b.tri_cw8, off[k].tcw8) : nullptr,
+                                      p.cw8_ok ? at(b.tri_cw8_prims, off[k].tcw8p) : nullptr};
         b.wide_depth = std::max(b.wide_depth, p.wide_depth);
         b.cw8_depth = std::max(b.cw8_depth, p.cw8_depth);
         c->batch_depth[k] = p.depth;
@@ -1528,6 +1539,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
                                 wide);
         if (rw != TRACER_OK) return rw;
     }
+    stack = std::max(stack, c->batch.cw8_depth);
     const uint32_t mask = p0.aov_mask ? p0.aov_mask : (1u << TRACER_AOV_RGBA8);
     const int stats = (p0.stats || (mask & (1u << TRACER_AOV_STATS))) ? 1 : 0;
     std::vector<size_t> base(n);
@@ -1580,7 +1592,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
         TraceArgs& a = slots[k];
         std::memset(&a, 0, sizeof a);
         a.sc = c->batch_scenes[k];
-        if (wide != WF_WIDTH_8) a.sc.tri_cw8 = a.sc.tri_cw8_prims = nullptr;  // finishing kernel: binary too
+        if (binary_asked(&p0)) a.sc.tri_cw8 = a.sc.tri_cw8_prims = nullptr;
         a.fr.aspect = f.aspect_ratio;
         a.fr.seed = f.seed;
         a.fr.cpos = V3{f.camera.pos[0], f.camera.pos[1], f.camera.pos[2]};
@@ -1655,7 +1667,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
             wc.shade_grid = (uint32_t)(sg < (size_t)c->sm_count * 8 ? sg : (size_t)c->sm_count * 8);
             // the graph bakes in sizes, launch shapes and buffer addresses
             std::vector<uint64_t> key = {n, total, max_rounds, block, stack, (uint64_t)stats, wc.extend_grid,
-                                         (uint64_t)wide, p0.tail_paths,
+                                         (uint64_t)wide, (uint64_t)binary_asked(&p0), p0.tail_paths,
                                          (uint64_t)(uintptr_t)c->wf_ray_o.p, (uint64_t)(uintptr_t)c->batch_slots.p,
                                          (uint64_t)(uintptr_t)c->b_rgba8.p, (uint64_t)(uintptr_t)c->b_rgba32f.p,
                                          (uint64_t)(uintptr_t)c->b_hit.p, mask};
@@ -1855,7 +1867,7 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
     a.rr_start = p->rr_start;
     a.sky = V3{p->sky[0], p->sky[1], p->sky[2]};
     a.sky_on = !(p->sky[0] == 0.0f && p->sky[1] == 0.0f && p->sky[2] == 0.0f);
-    a.stack_depth = stack;
+    a.stack_depth = std::max(stack, s.cw8_depth);
     const uint32_t nn = std::max(std::max(s.n_tri_nodes, s.n_sph_nodes), s.n_cw8_nodes);
     a.trav_limit = trav_limit(c, nn);
     a.stats = c->stats.p;
@@ -1886,9 +1898,10 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
         uint32_t wstack = stack;
         r = pick_width(c, p, wstack, wc.wide);
         if (r != TRACER_OK) return r;
-        a.stack_depth = wstack;
         if (wc.wide == WF_WIDTH_8) wc.cw8_stack = s.cw8_depth;
-        if (wc.wide != WF_WIDTH_8) a.sc.tri_cw8 = a.sc.tri_cw8_prims = nullptr;
+        if (binary_asked(p)) a.sc.tri_cw8 = a.sc.tri_cw8_prims = nullptr;
+        else wstack = std::max(wstack, s.cw8_depth);
+        a.stack_depth = wstack;
         const AdjWf aw{dldi, lin, ab.grad.p, s.nm, ab.pix.p, use_log ? ab.log.p : nullptr};
         c->last_kernel = TRACER_KERNEL_WAVEFRONT;
         c->last_launches = 1;  // + generate, rounds; the FP64-to-float conversion
@@ -1907,7 +1920,7 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
         EdgeArgs ea{dldi, ab.grad.p + 6 * (size_t)s.nm, {}, c->edge_samples, 0.01f, ab.segs.p, ab.nsegs.p, seg_cap};
         if (!camera_inverse(f->camera, ea.binv)) return fail(c, TRACER_ERR_INVALID_ARG, "degenerate camera basis");
         TraceArgs ae = a;
-        ae.stack_depth = stack;  // the binary traversal's
+        ae.stack_depth = std::max(stack, ae.sc.tri_cw8 ? s.cw8_depth : 0u);
         e = launch_edge_campos(ae, ea, p->tie_mode, s.bvh ? 1 : 0, st);
         c->last_launches += 2;
     }

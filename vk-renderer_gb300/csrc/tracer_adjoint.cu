@@ -99,13 +99,14 @@ __device__ __forceinline__ void gadd(double* g, int i, float v)
     if (v != 0.0f && isfinite(v)) atomicAdd(g + i, (double)v);
 }
 
-// One emitter's next-event estimate (same operations as nee_one) with its
+// One visible emitter's next-event estimate (same operations as nee_ray and
+// nee_value; rho, phi: the two random numbers of the direction L) with its
 // derivative with respect to the albedo at this bounce (componentwise, de_da)
 // and, when CAM, with respect to the camera position (de_dc[j], j = x, y, z)
 // given the tangents dP, dN of the hit point and normal.
-template <bool CAM, class TR>
-__device__ __forceinline__ V3 nee_one_grad(TR& tr, const TraceArgs& a, uint32_t si, V3 P, V3 N, const V3* dP,
-                                           const V3* dN, const Material& mat, Rng& g, V3& de_da, V3* de_dc)
+template <bool CAM>
+__device__ __forceinline__ V3 nee_grad(const TraceArgs& a, uint32_t si, V3 P, V3 N, const V3* dP, const V3* dN,
+                                       const Material& mat, float rho, float phi, V3& de_da, V3* de_dc)
 {
     const float4* rec = a.sc.sph_rec + 4 * (size_t)si;
     const float4 geo = __ldg(rec + 3);
@@ -116,14 +117,9 @@ __device__ __forceinline__ V3 nee_one_grad(TR& tr, const TraceArgs& a, uint32_t 
     const float ll = dot(l0, l0);
     const float q = sr * sr / ll;
     const float cos_a_max = sqrtf(1.0f - gclamp(q, 0.0f, 1.0f));
-    const float rho = rand01(g);
     const float cosa = gmix(cos_a_max, 1.0f, rho);
-    const float phi = (2.0f * PI) * rand01(g);
     const float sina = sqrtf(1.0f - cosa * cosa);
     const V3 L = jitter(l0, phi, sina, cosa);
-    Hit sh;
-    sh.t = t;
-    if (tr.trace(Ray{P, L}, sh, true)) return splat(0.0f);
     const float4 em = __ldg(rec + 1);
     const float q2 = t / sr + 1.0f;
     const V3 att1 = (v3(em) * 1.0f / (q2 * q2) - 0.001f) / (1.0f - 0.001f);
@@ -214,36 +210,21 @@ __device__ __forceinline__ V3 pixel_delta(float4 dl, V3 lin, uint32_t spp)
     return v3(dl.x * tm_slope(lin.x), dl.y * tm_slope(lin.y), dl.z * tm_slope(lin.z)) / (float)spp;
 }
 
-// Pass 1: the radiance loop with clamp bookkeeping.  lc[c] = last depth whose
-// clamp of acc[c] was active (-1: none); T = contributions that survive.
-template <class TR>
-__device__ __forceinline__ void primal_pass(TR& tr, const TraceArgs& a, Ray ray, Rng& g, int* lc, V3& T)
-{
-    V3 acc = splat(0.0f), mask = splat(1.0f);
-    T = splat(0.0f);
-    for (uint32_t depth = 0; depth < a.max_depth; ++depth) {
-        if (acc.x < 0.0f || acc.x > 1.0f) { lc[0] = (int)depth; T.x = 0.0f; }
-        if (acc.y < 0.0f || acc.y > 1.0f) { lc[1] = (int)depth; T.y = 0.0f; }
-        if (acc.z < 0.0f || acc.z > 1.0f) { lc[2] = (int)depth; T.z = 0.0f; }
-        acc = vclamp01(acc);
-        Hit h;
-        h.t = depth_tmax(depth);
-        const bool found = tr.trace(ray, h, false);
-        const V3 before = acc;
-        const bool cont = shade_bounce(tr, a, depth, found, h, ray, acc, mask, g);
-        T = T + (acc - before);
-        if (!cont) break;
-    }
-}
-
+// One thread per pixel; the warp's lanes go through the same jobs together,
+// bounce by bounce: with no linear image given, every sample's radiance first
+// (job 0 .. spp - 1), then pass 1 and pass 2 of every sample.  One loop body
+// holds the kernel's only closest-hit traversal and the two passes' shadow
+// rays, which the lanes trace together: with a traversal inlined at every use
+// and lanes going their own ways, two thirds of the issue slots were lost to
+// instruction fetches (160^2 x 4 spp, one light: 8.87 ms, no-instruction
+// stalls 9.7 of 17 cycles per issue).
 template <int TIE, bool BVH, bool CAM>
 __global__ void __launch_bounds__(128) k_adjoint(TraceArgs a, AdjArgs ga)
 {
     extern __shared__ int smem[];
+    const unsigned full = 0xFFFFFFFFu;
     const int tid = threadIdx.x, nthreads = blockDim.x;
-    const Stack stk{smem + tid, reinterpret_cast<float*>(smem + (size_t)a.stack_depth * nthreads) + tid, nthreads,
-                    (int)a.stack_depth};
-    // gradient sums after the stack, 8-byte aligned
+    // gradient sums after the stacks, 8-byte aligned
     double* sgrad = reinterpret_cast<double*>(smem + 2 * (size_t)a.stack_depth * nthreads);
     const uint32_t ngrad = 6 * ga.nm + 3;
     if (ga.smem_grad) {
@@ -257,163 +238,214 @@ __global__ void __launch_bounds__(128) k_adjoint(TraceArgs a, AdjArgs ga)
     Counters cnt;
 #pragma unroll
     for (int k = 0; k < C_COUNT; ++k) cnt.c[k] = 0;
-    Tracer<TIE, BVH, true> tr{a.sc, stk, cnt, a.status, a.trav_limit};
+    PathTracer<TIE, BVH, true> tr(a.sc, thread_stack(smem, a.stack_depth), cnt, a.status, a.trav_limit);
     const uint32_t x = blockIdx.x * 16 + (tid & 15);
     const uint32_t y = blockIdx.y * (nthreads >> 4) + (tid >> 4);
-    if (x < a.width && y < a.height) {
-        const size_t i = (size_t)y * a.width + x;
-        Rng g;
-        seed_rng(a, x, y, g);
-        const Ray pr = primary_ray(a, x, y);
-        V3 lin;
-        if (ga.linear) {
-            lin = v3(ga.linear[i]);
-        } else {
-            Rng g0 = g;
-            V3 acc = splat(0.0f);
-            for (uint32_t s = 0; s < a.spp; ++s) acc = acc + radiance(tr, a, pr, g0, nullptr, nullptr);
-            lin = acc / (float)a.spp;
+    bool alive = x < a.width && y < a.height;
+    const size_t i = alive ? (size_t)y * a.width + x : 0;
+    Rng g;  // at the start of a sample's pass 1 (pass 2: after it)
+    seed_rng(a, x, y, g);
+    const Ray pr = primary_ray(a, x, y);
+    V3 lin = splat(0.0f), delta = splat(0.0f), T = splat(0.0f);
+    int lc[3] = {-1, -1, -1};  // pass 1: last depth whose clamp of acc[c] was active (-1: none)
+    Rng gs = g;  // the running pass's RNG; before it, the sample's start
+    if (alive && ga.linear) lin = v3(ga.linear[i]);
+    const uint32_t spp = a.spp;
+    for (uint64_t job = ga.linear ? spp : 0; job < 3ull * spp; ++job) {
+        const int pass = job < spp ? 0 : 1 + (int)((job - spp) & 1);
+        if (job == spp) {  // the pixel's weight, once its linear value is known
+            if (!ga.linear) {
+                lin = lin / (float)spp;
+                seed_rng(a, x, y, g);
+            }
+            if (alive) delta = pixel_delta(ga.dldi[i], lin, spp);
+            alive = alive && finite3(delta) && finite3(lin);
         }
-        const V3 delta = pixel_delta(ga.dldi[i], lin, a.spp);
-        if (finite3(delta) && finite3(lin)) {
-            for (uint32_t s = 0; s < a.spp; ++s) {
-                const Rng gs = g;  // this sample's RNG state
-                int lc[3] = {-1, -1, -1};
-                V3 T;
-                primal_pass(tr, a, pr, g, lc, T);  // advances g past the sample
-                // pass 2: adjoint replay
-                Rng g2 = gs;
-                V3 mask = splat(1.0f), prefix = splat(0.0f);
-                Ray ray = pr;
-                V3 dO[3], dD[3];
+        if (!__any_sync(full, alive)) {
+            if (pass == 0) continue;  // (no lane of the warp has a pixel)
+            break;
+        }
+        Rng r = pass == 2 ? gs : g;
+        if (pass == 1) {
+            gs = g;
+            lc[0] = lc[1] = lc[2] = -1;
+            T = splat(0.0f);
+        }
+        V3 acc = splat(0.0f), mask = splat(1.0f);  // pass 2: acc = the surviving contributions so far
+        Ray ray = pr;
+        V3 dO[3], dD[3];
+        if (CAM) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                dO[j] = v3(j == 0 ? 1.0f : 0.0f, j == 1 ? 1.0f : 0.0f, j == 2 ? 1.0f : 0.0f);
+                dD[j] = splat(0.0f);
+            }
+        }
+        bool on = alive;
+        for (uint32_t depth = 0; depth < a.max_depth; ++depth) {
+            if (!__any_sync(full, on)) break;
+            Hit h;
+            bool found = false;
+            if (on) {
+                if (pass == 1) {
+                    if (acc.x < 0.0f || acc.x > 1.0f) { lc[0] = (int)depth; T.x = 0.0f; }
+                    if (acc.y < 0.0f || acc.y > 1.0f) { lc[1] = (int)depth; T.y = 0.0f; }
+                    if (acc.z < 0.0f || acc.z > 1.0f) { lc[2] = (int)depth; T.z = 0.0f; }
+                }
+                if (pass != 2) acc = vclamp01(acc);
+                h.t = depth_tmax(depth);
+                found = tr.trace(ray, h, false);
+            }
+            __syncwarp();
+            if (pass != 2) {
+                // the radiance loop; in pass 1 with the sum of what survives the clamps
+                const V3 before = acc;
+                const bool cont = shade_bounce<true, true>(tr, a, on, depth, found, h, ray, acc, mask, r);
+                if (on && pass == 1) T = T + (acc - before);
+                on = on && cont;
+                continue;
+            }
+            // pass 2: adjoint replay
+            const V3 surv = v3((int)depth >= lc[0] ? 1.0f : 0.0f, (int)depth >= lc[1] ? 1.0f : 0.0f,
+                               (int)depth >= lc[2] ? 1.0f : 0.0f);
+            const V3 w = delta * surv;
+            if (on && !found) {
+                if (a.sky_on) acc = acc + mask * a.sky * surv;
+                on = false;
+            }
+            V3 P, N;
+            Material mat;
+            int m = -1;
+            bool diffuse = false;
+            V3 dP[3], dN[3];
+            float phi = 0.0f, sa = 0.0f, ca = 0.0f;
+            V3 d;
+            if (on) {
+                surface(a.sc, ray, h, P, N, mat);
+                m = h.kind == 1 ? (int)__float_as_uint(__ldg(a.sc.tri + 3 * (size_t)h.slot).w) : -1;
+                if (CAM) {
+                    const float nd = dot(N, ray.d);
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        const V3 q = dO[j] + dD[j] * h.t;
+                        const float dt = -dot(N, q) / nd;
+                        dP[j] = q + ray.d * dt;
+                        dN[j] = h.kind == 2 ? dP[j] / __ldg(a.sc.sph_geo + h.slot).w : splat(0.0f);
+                    }
+                }
+                diffuse = mat.type == MAT_DIFFUSE;
+                if (diffuse) {
+                    const float r2 = rand01(r);
+                    phi = (2.0f * PI) * rand01(r);
+                    sa = sqrtf(r2);
+                    ca = sqrtf(1.0f - r2);
+                    d = jitter(N, phi, sa, ca) * (1.0f - mat.metalness);
+                }
+            }
+            V3 e = splat(0.0f), de_da = splat(0.0f);
+            V3 de_dc[3] = {splat(0.0f), splat(0.0f), splat(0.0f)};
+            for (uint32_t k = 0; k < a.sc.ne; ++k) {
+                if (!__any_sync(full, diffuse)) break;
+                if (diffuse) {
+                    const uint32_t si = __ldg(a.sc.emit + k);
+                    Rng r0 = r;  // the direction's two random numbers again, for the derivative
+                    Hit sh;
+                    const V3 L = nee_ray(a.sc, si, P, r, sh.t);
+                    V3 c = splat(0.0f);
+                    if (!tr.trace(Ray{P, L}, sh, true)) {
+                        const float rho = rand01(r0), ph = (2.0f * PI) * rand01(r0);
+                        c = nee_grad<CAM>(a, si, P, N, dP, dN, mat, rho, ph, de_da, de_dc);
+                    }
+                    e = e + c;
+                }
+                __syncwarp();
+            }
+            if (!on) continue;
+            if (diffuse) {
+                const bool emits = mat.emissive.x > 0.0f && mat.emissive.y > 0.0f && mat.emissive.z > 0.0f;
+                const V3 en = emits ? normalize(mat.emissive) : splat(0.0f);
+                const V3 wm = w * mask;
+                if (m >= 0) {
+                    if (emits) {  // d normalize(e) = (I - n n^T) / |e|
+                        const float il = 1.0f / length(mat.emissive);
+                        const V3 ge = (wm - en * dot(en, wm)) * il;
+                        gadd(gem, 3 * m + 0, ge.x);
+                        gadd(gem, 3 * m + 1, ge.y);
+                        gadd(gem, 3 * m + 2, ge.z);
+                    }
+                    const V3 gd = wm * de_da;
+                    gadd(gal, 3 * m + 0, gd.x);
+                    gadd(gal, 3 * m + 1, gd.y);
+                    gadd(gal, 3 * m + 2, gd.z);
+                }
+                if (CAM) {
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) gadd(gcam, j, dot(wm, de_dc[j]));
+                }
+                acc = acc + mask * (en + e) * surv;
+                if (m >= 0) {
+                    const V3 R = T - acc;
+                    if (mat.albedo.x != 0.0f) gadd(gal, 3 * m + 0, delta.x * R.x / mat.albedo.x);
+                    if (mat.albedo.y != 0.0f) gadd(gal, 3 * m + 1, delta.y * R.y / mat.albedo.y);
+                    if (mat.albedo.z != 0.0f) gadd(gal, 3 * m + 2, delta.z * R.z / mat.albedo.z);
+                }
+                mask = mask * mat.albedo;
+                const V3 rf = reflect(ray.d, N);
+                if (CAM) {
+                    float cphi, sphi;
+                    psincos(phi, sphi, cphi);
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        const V3 djd = djitter(N, dN[j], cphi, sphi, sa, 0.0f, ca, 0.0f);
+                        const V3 drf = dreflect(ray.d, dD[j], N, dN[j]);
+                        dD[j] = dnorm(rf + d, drf + djd * (1.0f - mat.metalness));
+                        dO[j] = dP[j];
+                    }
+                }
+                ray = Ray{P, normalize(rf + d)};
+            } else if (mat.type == MAT_DIELECTRIC) {
+                if (m >= 0) {
+                    const V3 ge = w * mask;
+                    gadd(gem, 3 * m + 0, ge.x);
+                    gadd(gem, 3 * m + 1, ge.y);
+                    gadd(gem, 3 * m + 2, ge.z);
+                }
+                acc = acc + mat.emissive * mask * surv;
+                if (m >= 0) {
+                    const V3 R = T - acc;
+                    if (mat.albedo.x != 0.0f) gadd(gal, 3 * m + 0, delta.x * R.x / mat.albedo.x);
+                    if (mat.albedo.y != 0.0f) gadd(gal, 3 * m + 1, delta.y * R.y / mat.albedo.y);
+                    if (mat.albedo.z != 0.0f) gadd(gal, 3 * m + 2, delta.z * R.z / mat.albedo.z);
+                }
+                mask = mask * mat.albedo;
+                const float cosine = -dot(ray.d, N) / length(ray.d);
+                const V3 reflected = reflect(ray.d, N);
+                const V3 refracted = refract(ray.d, N, mat.roughness);
+                const bool tir = refracted == splat(0.0f);
+                const float prob = tir ? 1.0f : schlick(cosine, mat.roughness);
+                const bool refl = rand01(r) < prob;
+                const V3 nd = refl ? reflected : refracted;
                 if (CAM) {
 #pragma unroll
                     for (int j = 0; j < 3; ++j) {
-                        dO[j] = v3(j == 0 ? 1.0f : 0.0f, j == 1 ? 1.0f : 0.0f, j == 2 ? 1.0f : 0.0f);
-                        dD[j] = splat(0.0f);
+                        const V3 dr = refl ? dreflect(ray.d, dD[j], N, dN[j])
+                                           : drefract(ray.d, dD[j], N, dN[j], mat.roughness);
+                        dD[j] = dnorm(nd, dr);
+                        dO[j] = dP[j];
                     }
                 }
-                for (uint32_t depth = 0; depth < a.max_depth; ++depth) {
-                    Hit h;
-                    h.t = depth_tmax(depth);
-                    const bool found = tr.trace(ray, h, false);
-                    const V3 surv = v3((int)depth >= lc[0] ? 1.0f : 0.0f, (int)depth >= lc[1] ? 1.0f : 0.0f,
-                                       (int)depth >= lc[2] ? 1.0f : 0.0f);
-                    const V3 w = delta * surv;
-                    if (!found) {
-                        if (a.sky_on) prefix = prefix + mask * a.sky * surv;
-                        break;
-                    }
-                    V3 P, N;
-                    Material mat;
-                    tr.surface(ray, h, P, N, mat);
-                    const int m = h.kind == 1 ? (int)__float_as_uint(__ldg(a.sc.tri + 3 * (size_t)h.slot).w) : -1;
-                    V3 dP[3], dN[3];
-                    if (CAM) {
-                        const float nd = dot(N, ray.d);
-#pragma unroll
-                        for (int j = 0; j < 3; ++j) {
-                            const V3 q = dO[j] + dD[j] * h.t;
-                            const float dt = -dot(N, q) / nd;
-                            dP[j] = q + ray.d * dt;
-                            dN[j] = h.kind == 2 ? dP[j] / __ldg(a.sc.sph_geo + h.slot).w : splat(0.0f);
-                        }
-                    }
-                    V3 C = splat(0.0f);
-                    if (mat.type == MAT_DIFFUSE) {
-                        const float r2 = rand01(g2);
-                        const float phi = (2.0f * PI) * rand01(g2);
-                        const float sa = sqrtf(r2), ca = sqrtf(1.0f - r2);
-                        const V3 jd = jitter(N, phi, sa, ca);
-                        const V3 d = jd * (1.0f - mat.metalness);
-                        V3 e = splat(0.0f), de_da = splat(0.0f);
-                        V3 de_dc[3] = {splat(0.0f), splat(0.0f), splat(0.0f)};
-                        for (uint32_t k = 0; k < a.sc.ne; ++k)
-                            e = e + nee_one_grad<CAM>(tr, a, __ldg(a.sc.emit + k), P, N, dP, dN, mat, g2, de_da, de_dc);
-                        const bool emits = mat.emissive.x > 0.0f && mat.emissive.y > 0.0f && mat.emissive.z > 0.0f;
-                        const V3 en = emits ? normalize(mat.emissive) : splat(0.0f);
-                        C = mask * (en + e);
-                        const V3 wm = w * mask;
-                        if (m >= 0) {
-                            if (emits) {  // d normalize(e) = (I - n n^T) / |e|
-                                const float il = 1.0f / length(mat.emissive);
-                                const V3 ge = (wm - en * dot(en, wm)) * il;
-                                gadd(gem, 3 * m + 0, ge.x);
-                                gadd(gem, 3 * m + 1, ge.y);
-                                gadd(gem, 3 * m + 2, ge.z);
-                            }
-                            const V3 gd = wm * de_da;
-                            gadd(gal, 3 * m + 0, gd.x);
-                            gadd(gal, 3 * m + 1, gd.y);
-                            gadd(gal, 3 * m + 2, gd.z);
-                        }
-                        if (CAM) {
-#pragma unroll
-                            for (int j = 0; j < 3; ++j) gadd(gcam, j, dot(wm, de_dc[j]));
-                        }
-                        prefix = prefix + C * surv;
-                        if (m >= 0) {
-                            const V3 R = T - prefix;
-                            if (mat.albedo.x != 0.0f) gadd(gal, 3 * m + 0, delta.x * R.x / mat.albedo.x);
-                            if (mat.albedo.y != 0.0f) gadd(gal, 3 * m + 1, delta.y * R.y / mat.albedo.y);
-                            if (mat.albedo.z != 0.0f) gadd(gal, 3 * m + 2, delta.z * R.z / mat.albedo.z);
-                        }
-                        mask = mask * mat.albedo;
-                        const V3 rf = reflect(ray.d, N);
-                        if (CAM) {
-                            float cphi, sphi;
-                            psincos(phi, sphi, cphi);
-#pragma unroll
-                            for (int j = 0; j < 3; ++j) {
-                                const V3 djd = djitter(N, dN[j], cphi, sphi, sa, 0.0f, ca, 0.0f);
-                                const V3 drf = dreflect(ray.d, dD[j], N, dN[j]);
-                                dD[j] = dnorm(rf + d, drf + djd * (1.0f - mat.metalness));
-                                dO[j] = dP[j];
-                            }
-                        }
-                        ray = Ray{P, normalize(rf + d)};
-                    } else if (mat.type == MAT_DIELECTRIC) {
-                        C = mat.emissive * mask;
-                        if (m >= 0) {
-                            const V3 ge = w * mask;
-                            gadd(gem, 3 * m + 0, ge.x);
-                            gadd(gem, 3 * m + 1, ge.y);
-                            gadd(gem, 3 * m + 2, ge.z);
-                        }
-                        prefix = prefix + C * surv;
-                        if (m >= 0) {
-                            const V3 R = T - prefix;
-                            if (mat.albedo.x != 0.0f) gadd(gal, 3 * m + 0, delta.x * R.x / mat.albedo.x);
-                            if (mat.albedo.y != 0.0f) gadd(gal, 3 * m + 1, delta.y * R.y / mat.albedo.y);
-                            if (mat.albedo.z != 0.0f) gadd(gal, 3 * m + 2, delta.z * R.z / mat.albedo.z);
-                        }
-                        mask = mask * mat.albedo;
-                        const float cosine = -dot(ray.d, N) / length(ray.d);
-                        const V3 reflected = reflect(ray.d, N);
-                        const V3 refracted = refract(ray.d, N, mat.roughness);
-                        const bool tir = refracted == splat(0.0f);
-                        const float prob = tir ? 1.0f : schlick(cosine, mat.roughness);
-                        const bool refl = rand01(g2) < prob;
-                        const V3 nd = refl ? reflected : refracted;
-                        if (CAM) {
-#pragma unroll
-                            for (int j = 0; j < 3; ++j) {
-                                const V3 dr = refl ? dreflect(ray.d, dD[j], N, dN[j])
-                                                   : drefract(ray.d, dD[j], N, dN[j], mat.roughness);
-                                dD[j] = dnorm(nd, dr);
-                                dO[j] = dP[j];
-                            }
-                        }
-                        ray = Ray{P, normalize(nd)};
-                    }
-                    if (depth >= a.rr_start) {
-                        const float p = max3(mask);
-                        if (rand01(g2) > p) break;
-                        mask = mask * (1.0f / p);
-                    }
-                }
+                ray = Ray{P, normalize(nd)};
+            }
+            if (depth >= a.rr_start) {
+                const float p = max3(mask);
+                if (rand01(r) > p)
+                    on = false;
+                else
+                    mask = mask * (1.0f / p);
             }
         }
+        if (pass == 0) lin = lin + acc;
+        if (pass != 2) g = r;  // past the sample
     }
     flush_counters(a, cnt);
     if (ga.smem_grad) {
@@ -544,7 +576,7 @@ __device__ __forceinline__ bool adj_replay_bounce(TR& tr, const TraceArgs& a, co
     if (found) {
         V3 P, N;
         Material mat;
-        tr.surface(p.ray, h, P, N, mat);
+        surface(a.sc, p.ray, h, P, N, mat);
         const int m = h.kind == 1 ? (int)__float_as_uint(__ldg(a.sc.tri + 3 * (size_t)h.slot).w) : -1;
         if (mat.type == MAT_DIFFUSE) {
             const float r2 = rand01(p.g);
@@ -627,7 +659,7 @@ __device__ __forceinline__ bool adj_advance(TR& tr, const TraceArgs& a, const Ad
         if (p.acc.z < 0.0f || p.acc.z > 1.0f) { p.lc[2] = (int)p.depth; p.T.z = 0.0f; }
         p.acc = vclamp01(p.acc);
         const V3 before = p.acc;
-        const bool cont = shade_bounce<false>(tr, a, p.depth, found, h, p.ray, p.acc, p.mask, p.g);  // no emitters
+        const bool cont = shade_bounce<false>(tr, a, true, p.depth, found, h, p.ray, p.acc, p.mask, p.g);  // no emitters
         p.T = p.T + (p.acc - before);
         if (log) log[p.depth] = hit_pack(h);
         p.depth++;
@@ -711,18 +743,7 @@ __global__ void __launch_bounds__(128) wf_adj_finish(TraceArgs a, WfState s, Adj
     Counters cnt;
 #pragma unroll
     for (int k = 0; k < C_COUNT; ++k) cnt.c[k] = 0;
-    const Stack stk{smem + threadIdx.x, reinterpret_cast<float*>(smem + (size_t)a.stack_depth * blockDim.x) + threadIdx.x,
-                    (int)blockDim.x, (int)a.stack_depth};
-    // closest hits: the per-thread 8-wide traversal where the scene has one
-    // (c3's 256^2 adjoint: 0.47 ms against 0.74 with the plain binary
-    // traversal), else the plain traversal, which tests a hit leaf child as
-    // soon as its parent is visited (on c3's short, latency-bound chains it
-    // beat the pre-encoded binary traversal, 1.35 against 1.42 ms)
-    Tracer<TIE, BVH, STATS> tr{a.sc, stk, cnt, a.status, a.trav_limit};
-    // triangle-only scenes with an 8-wide BVH: the forward finishing kernel's
-    // per-thread 8-wide traversal, its stack over the same shared memory
-    // (stack_depth 8-byte entries per thread; nothing here traces shadow rays)
-    const PairStack pstk{reinterpret_cast<int2*>(smem) + threadIdx.x, (int)blockDim.x, (int)a.stack_depth};
+    PathTracer<TIE, BVH, STATS> tr(a.sc, thread_stack(smem, a.stack_depth), cnt, a.status, a.trav_limit);
     const uint32_t threads = gridDim.x * blockDim.x;
     uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x;
     while (qi < n) {
@@ -733,10 +754,7 @@ __global__ void __launch_bounds__(128) wf_adj_finish(TraceArgs a, WfState s, Adj
         for (;;) {
             Hit h;
             h.t = depth_tmax(p.depth);
-            if (BVH && a.sc.tri_cw8 != nullptr)
-                closest_cw8<STATS>(a.sc, p.ray, h, pstk, a.status, a.trav_limit, cnt);
-            else
-                tr.trace(p.ray, h, false);
+            tr.trace(p.ray, h, false);
             if (!adj_advance(tr, a, w, pid, x, y, h, p, w.pix + pid, s.prim0 + pid)) break;
         }
         qi = n > threads ? threads + atomicAdd(&s.count[2], 1u) : n;

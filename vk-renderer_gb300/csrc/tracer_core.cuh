@@ -188,6 +188,7 @@ struct Tracer {
             BoxRay br = make_boxray(ray);
             done = traverse<0>(sc.tri_nodes, sc.n_tri_nodes, ray, br, h, tmax, any);
         } else {
+#pragma unroll 1
             for (uint32_t i = 0; i < sc.nt && !done; ++i) done = test_tri(ray, i, h, tmax, any);
         }
         if (!done) {
@@ -195,9 +196,11 @@ struct Tracer {
                 BoxRay br = make_boxray(ray);
                 done = traverse<1>(sc.sph_nodes, sc.n_sph_nodes, ray, br, h, tmax, any);
             } else {
+#pragma unroll 1
                 for (uint32_t i = 0; i < sc.ns && !done; ++i) done = test_sphere(ray, i, h, tmax, any);
             }
         }
+#pragma unroll 1
         for (uint32_t i = 0; i < sc.np && !done; ++i) {
             count(C_PLANES);
             const float4* p = sc.planes + 4 * (size_t)i;
@@ -216,31 +219,31 @@ struct Tracer {
         if (!shadow) count(C_HITS);  // closest-hit rays that hit (each reads a material record)
         return true;
     }
-
-    // Surface data of a hit (Tracer.comp:384-392, :404-408, :420-424).
-    __device__ __forceinline__ void surface(const Ray& ray, const Hit& h, V3& P, V3& N, Material& m)
-    {
-        P = ray.o + h.t * ray.d;
-        if (h.kind == 1) {
-            const float4* t = sc.tri + 3 * (size_t)h.slot;
-            const float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t + 2);
-            const V3 u = v3(b), v = v3(c);
-            N = v3((u.y * v.z) - (u.z * v.y), (u.z * v.x) - (u.x * v.z), (u.x * v.y) - (u.y * v.x));
-            m = load_material(sc.mats + 3 * (size_t)__float_as_uint(a.w));
-        } else if (h.kind == 2) {
-            const float4 g = __ldg(sc.sph_geo + h.slot);
-            N = (P - v3(g)) / g.w;
-            m = load_material(sc.sph_rec + 4 * (size_t)__ldg(sc.sph_id + h.slot));
-        } else {
-            const float4* p = sc.planes + 4 * (size_t)h.slot;
-            N = v3(__ldg(p + 3));
-            m = load_material(p);
-        }
-    }
 };
 
+// Surface data of a hit (Tracer.comp:384-392, :404-408, :420-424).
+__device__ __forceinline__ void surface(const DevScene& sc, const Ray& ray, const Hit& h, V3& P, V3& N, Material& m)
+{
+    P = ray.o + h.t * ray.d;
+    if (h.kind == 1) {
+        const float4* t = sc.tri + 3 * (size_t)h.slot;
+        const float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t + 2);
+        const V3 u = v3(b), v = v3(c);
+        N = v3((u.y * v.z) - (u.z * v.y), (u.z * v.x) - (u.x * v.z), (u.x * v.y) - (u.y * v.x));
+        m = load_material(sc.mats + 3 * (size_t)__float_as_uint(a.w));
+    } else if (h.kind == 2) {
+        const float4 g = __ldg(sc.sph_geo + h.slot);
+        N = (P - v3(g)) / g.w;
+        m = load_material(sc.sph_rec + 4 * (size_t)__ldg(sc.sph_id + h.slot));
+    } else {
+        const float4* p = sc.planes + 4 * (size_t)h.slot;
+        N = v3(__ldg(p + 3));
+        m = load_material(p);
+    }
+}
+
 // Tracer.comp:256-263
-__device__ __forceinline__ V3 jitter(V3 d, float phi, float sina, float cosa)
+static __device__ __noinline__ V3 jitter(V3 d, float phi, float sina, float cosa)
 {
     const V3 w = normalize(d);
     const V3 u = normalize(cross(v3(w.y, w.z, w.x), w));
@@ -250,12 +253,18 @@ __device__ __forceinline__ V3 jitter(V3 d, float phi, float sina, float cosa)
     return (u * c + v * s) * sina + w * cosa;
 }
 
+// powf, rand01's cosine and jitter are out of line: the kernels that shade hold
+// several copies of each otherwise, and lose a third of their issue slots to
+// instruction fetches (the reference's frame, k_plain: 1506 us inlined, 1379
+// out of line with the primitive loops not unrolled either, 1611 at first).
+static __device__ __noinline__ float pow_call(float x, float y) { return powf(x, y); }
+
 // Tracer.comp:265-272
 __device__ __forceinline__ float schlick(float cosine, float ior)
 {
     float r0 = (1.0f - ior) / (1.0f + ior);
     r0 = r0 * r0;
-    return r0 + (1.0f - r0) * powf(1.0f - cosine, 5.0f);
+    return r0 + (1.0f - r0) * pow_call(1.0f - cosine, 5.0f);
 }
 
 // Tracer.comp:279-312
@@ -283,22 +292,25 @@ __device__ __forceinline__ float geometry_smith(V3 N, V3 V, V3 L, float roughnes
 }
 
 // One emitter's next-event contribution (Tracer.comp:458-504) for a diffuse
-// hit; consumes two random numbers whether or not the light is visible.
-template <class TR>
-__device__ __forceinline__ V3 nee_one(TR& tr, const TraceArgs& a, uint32_t si, V3 P, V3 N, const Material& mat, Rng& g)
+// hit, in two parts around its shadow ray.  nee_ray: the direction to a
+// random point of the light's cone, and the distance to the light; consumes
+// two random numbers whether or not the light is visible.
+__device__ __forceinline__ V3 nee_ray(const DevScene& sc, uint32_t si, V3 P, Rng& g, float& t)
 {
-    const float4* rec = a.sc.sph_rec + 4 * (size_t)si;
-    const float4 geo = __ldg(rec + 3);
+    const float4 geo = __ldg(sc.sph_rec + 4 * (size_t)si + 3);
     const V3 sP = v3(geo);
     const float sr = geo.w;
-    const float t = length(sP - P) - sr;
+    t = length(sP - P) - sr;
     const V3 l0 = sP - P;
     const float cos_a_max = sqrtf(1.0f - gclamp(sr * sr / dot(l0, l0), 0.0f, 1.0f));
     const float cosa = gmix(cos_a_max, 1.0f, rand01(g));
-    const V3 L = jitter(l0, (2.0f * PI) * rand01(g), sqrtf(1.0f - cosa * cosa), cosa);
-    Hit sh;
-    sh.t = t;
-    if (tr.trace(Ray{P, L}, sh, true)) return splat(0.0f);
+    return jitter(l0, (2.0f * PI) * rand01(g), sqrtf(1.0f - cosa * cosa), cosa);
+}
+// nee_value: the contribution of the light at distance t along L, visible.
+__device__ __forceinline__ V3 nee_value(const TraceArgs& a, uint32_t si, V3 P, V3 N, const Material& mat, V3 L, float t)
+{
+    const float4* rec = a.sc.sph_rec + 4 * (size_t)si;
+    const float sr = __ldg(rec + 3).w;
     const float4 em = __ldg(rec + 1);
     const float q = t / sr + 1.0f;
     V3 attenuation = v3(em) * 1.0f / (q * q);
@@ -311,7 +323,7 @@ __device__ __forceinline__ V3 nee_one(TR& tr, const TraceArgs& a, uint32_t si, V
     const float NDF = distribution_ggx(N, H, mat.roughness);
     const float G = geometry_smith(N, V, L, mat.roughness);
     const float cth = gmax(dot(H, V), 0.0f);
-    const V3 F = F0 + (1.0f - F0) * powf(1.0f - cth, 5.0f);
+    const V3 F = F0 + (1.0f - F0) * pow_call(1.0f - cth, 5.0f);
     V3 kD = 1.0f - F;
     kD = kD * (1.0f - mat.metalness);
     const V3 numerator = NDF * G * F;
@@ -329,29 +341,56 @@ __device__ __forceinline__ float depth_tmax(uint32_t depth)
 }
 
 // The part of one depth iteration of radiance (Tracer.comp:445-549) that
-// follows trace_ray: sky on a miss, material scatter with next-event
-// estimation, Russian roulette.  Updates acc, mask and ray; returns false
-// when the path ends (miss or roulette).  acc must already be clamped
-// (Tracer.comp:441; the clamp does not affect the trace, so it may run before
-// or after it).  NEE = false leaves out the next-event code for scenes
-// without emissive spheres (its loop would run no iteration there).
-template <bool NEE = true, class TR>
-__device__ __forceinline__ bool shade_bounce(TR& tr, const TraceArgs& a, uint32_t depth, bool found, const Hit& h,
-                                             Ray& ray, V3& acc, V3& mask, Rng& g)
+// follows trace_ray, for a lane that is `on`: sky on a miss, material scatter
+// with next-event estimation, Russian roulette.  Updates acc, mask and ray;
+// returns false when the path ends (miss or roulette) or the lane is off.
+// acc must already be clamped (Tracer.comp:441; the clamp does not affect the
+// trace, so it may run before or after it).  NEE = false leaves out the
+// next-event code for scenes without emissive spheres (its loop would run no
+// iteration there).
+//
+// SYNC (with NEE): every lane of the warp calls this together, and the lanes
+// trace each emitter's shadow ray together.  Called by lanes on their own,
+// the shadow rays of some run while the others wait, or trace something else
+// of the same warp: 3.5 of 32 lanes active in the finishing kernel of a
+// 640x360 frame with two lights, and most issue slots lost to instruction
+// fetches of a kernel with five copies of the traversal.
+template <bool NEE = true, bool SYNC = false, class TR>
+__device__ __forceinline__ bool shade_bounce(TR& tr, const TraceArgs& a, bool on, uint32_t depth, bool found,
+                                             const Hit& h, Ray& ray, V3& acc, V3& mask, Rng& g)
 {
-    if (!found) {
-        if (a.sky_on) acc = acc + mask * a.sky;
-        return false;
-    }
-    V3 P, N;
+    const bool hit = on && found;
+    if (on && !found && a.sky_on) acc = acc + mask * a.sky;
+    V3 P, N, d;
     Material mat;
-    tr.surface(ray, h, P, N, mat);
-    if (mat.type == MAT_DIFFUSE) {
-        const float r2 = rand01(g);
-        const V3 d = jitter(N, (2.0f * PI) * rand01(g), sqrtf(r2), sqrtf(1.0f - r2)) * (1.0f - mat.metalness);
-        V3 e = splat(0.0f);
-        if (NEE)
-            for (uint32_t k = 0; k < a.sc.ne; ++k) e = e + nee_one(tr, a, __ldg(a.sc.emit + k), P, N, mat, g);
+    bool diffuse = false;
+    if (hit) {
+        surface(a.sc, ray, h, P, N, mat);
+        diffuse = mat.type == MAT_DIFFUSE;
+        if (diffuse) {
+            const float r2 = rand01(g);
+            d = jitter(N, (2.0f * PI) * rand01(g), sqrtf(r2), sqrtf(1.0f - r2)) * (1.0f - mat.metalness);
+        }
+    }
+    V3 e = splat(0.0f);
+    if (NEE) {
+        for (uint32_t k = 0;; ++k) {
+            const bool mine = diffuse && k < a.sc.ne;
+            if (!(SYNC ? __any_sync(0xFFFFFFFFu, mine) : mine)) break;
+            if (mine) {
+                const uint32_t si = __ldg(a.sc.emit + k);
+                Hit sh;
+                const V3 L = nee_ray(a.sc, si, P, g, sh.t);
+                const float t = sh.t;
+                V3 c = splat(0.0f);
+                if (!tr.trace(Ray{P, L}, sh, true)) c = nee_value(a, si, P, N, mat, L, t);
+                e = e + c;
+            }
+            if (SYNC) __syncwarp();
+        }
+    }
+    if (!hit) return false;
+    if (diffuse) {
         const bool emits = mat.emissive.x > 0.0f && mat.emissive.y > 0.0f && mat.emissive.z > 0.0f;
         const V3 emissive = emits ? normalize(mat.emissive) : splat(0.0f);
         acc = acc + mask * (emissive + e);
@@ -372,27 +411,6 @@ __device__ __forceinline__ bool shade_bounce(TR& tr, const TraceArgs& a, uint32_
         mask = mask * (1.0f / p);
     }
     return true;
-}
-
-// Tracer.comp:433-553 (radiance), extensions: rr_start, sky, max_depth.
-// prim0 / t0 receive the first ray's hit when non-null.
-template <class TR>
-__device__ __forceinline__ V3 radiance(TR& tr, const TraceArgs& a, Ray ray, Rng& g, uint32_t* prim0, float* t0)
-{
-    V3 acc = splat(0.0f);
-    V3 mask = splat(1.0f);
-    for (uint32_t depth = 0; depth < a.max_depth; ++depth) {
-        acc = vclamp01(acc);
-        Hit h;
-        h.t = depth_tmax(depth);
-        const bool found = tr.trace(ray, h, false);
-        if (prim0 && depth == 0) {
-            *prim0 = found ? h.prim : NO_PRIM;
-            *t0 = found ? h.t : -1.0f;
-        }
-        if (!shade_bounce(tr, a, depth, found, h, ray, acc, mask, g)) break;
-    }
-    return acc;
 }
 
 __device__ __forceinline__ unsigned char unorm8(float x)
@@ -429,7 +447,7 @@ __device__ __forceinline__ void resolve_pixel(const TraceArgs& a, uint32_t x, ui
     if (a.linear) a.linear[(size_t)y * a.width + x] = make_float4(accum.x, accum.y, accum.z, 1.0f);
     accum = accum / (accum + splat(1.0f));
     const float gam = 1.0f / 2.2f;
-    accum = v3(powf(accum.x, gam), powf(accum.y, gam), powf(accum.z, gam));
+    accum = v3(pow_call(accum.x, gam), pow_call(accum.y, gam), pow_call(accum.z, gam));
     const float dither = rand01(g) / 64.0f;
     const float4 c = make_float4(accum.x + dither, accum.y + dither, accum.z + dither, 1.0f);
     const size_t i = (size_t)y * a.width + x;

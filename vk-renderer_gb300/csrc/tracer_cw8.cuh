@@ -162,26 +162,31 @@ struct alignas(16) W8Lane {
 };
 static_assert(sizeof(W8Lane) == 48, "lane record is 48 bytes");
 
-// Closest hit of one ray by one thread over the 8-wide BVH of a
-// triangle-only scene, for the finishing kernel: the extend kernel's node
-// visit and triangle test (strict ties), without the warp's phases -- a
-// node's leaves are tested right after the visit -- so the same hit.  h.t
-// holds tmax on entry; on a miss h.kind = 0 and h.prim = NO_PRIM.  stk: the
-// thread's stack of node groups (8-byte entries, interleaved by thread).
+// trace_ray of one ray by one thread over a scene with BVHs (strict ties):
+// the triangles over the 8-wide BVH where the scene has one (the extend
+// kernel's node visit and triangle test, a node's leaves tested right after
+// the visit), else, and the spheres, over the binary BVHs, then the planes.
+// The same hit as every other traversal.  h.t holds tmax on entry; on a miss
+// h.kind = 0 and h.prim = NO_PRIM.  shadow: any hit will do.  stk: the
+// thread's stack (8-byte entries, interleaved by thread), at least as deep as
+// either BVH.
 template <bool STATS>
-__device__ __forceinline__ bool closest_cw8(const DevScene& sc, const Ray& ray, Hit& h, const PairStack& stk,
-                                            int* status, uint32_t trav_limit, Counters& cnt)
+__device__ __forceinline__ bool trace_bvh(const DevScene& sc, const Ray& ray, Hit& h, bool shadow, const PairStack& stk,
+                                          int* status, uint32_t trav_limit, Counters& cnt)
 {
-    if (STATS) cnt.c[C_CLOSEST]++;
-    Hit b;
-    b.t = h.t;
-    b.prim = 0;  // see accept_strict
-    b.kind = 0;
-    b.slot = 0;
+    if (STATS) {
+        cnt.c[C_SHADOW] += shadow ? 1 : 0;
+        cnt.c[C_CLOSEST] += shadow ? 0 : 1;
+    }
+    Lane L;
+    L.h.t = h.t;
+    L.h.prim = 0;  // see accept_strict
+    L.h.kind = 0;
+    L.h.slot = 0;
     if (!isnan3(ray.d)) {
-        if (sc.n_tri_nodes > 0 && sc.nt > 0) {
-            const W8Ray cr = make_w8ray(ray);
-            const float4* nodes = sc.tri_cw8;
+        const W8Ray cr = make_w8ray(ray);
+        const bool wide = sc.tri_cw8 != nullptr;
+        if (wide) {
             uint2 G = w8_root();
             int sp = 0;
             uint32_t steps = 0;
@@ -206,24 +211,53 @@ __device__ __forceinline__ bool closest_cw8(const DevScene& sc, const Ray& ray, 
                     }
                 }
                 uint2 P;
-                w8_visit(nodes, idx, cr, b.t, G, P);
-                if (STATS) cnt.c[C_NODES] += 4;
+                w8_visit(sc.tri_cw8, idx, cr, L.h.t, G, P);
+                if (STATS) cnt.c[C_NODES] += 3;
                 while (w8_any(P)) {
                     bool two;
                     const uint32_t k = w8_next_leaf(P, two);
-                    cw8_test_tri2<STATS>(sc.tri_cw8_prims, k, two, ray, b, cnt);
+                    cw8_test_tri2<STATS>(sc.tri_cw8_prims, k, two, ray, L.h, cnt);
                 }
+                if (shadow && L.h.kind) break;
             }
         }
-        planes_pass<STATS>(sc, ray, b, cnt);
+        L.br = cr.br;
+        for (L.pass = wide ? 1 : 0; L.pass < 2 && !(shadow && L.h.kind); ++L.pass) {
+            const bool any = L.pass == 0 ? (sc.n_tri_nodes > 0 && sc.nt > 0) : (sc.n_sph_nodes > 0 && sc.ns > 0);
+            if (any) enc_pass<STATS>(sc, ray, L, shadow, stk, status, trav_limit, cnt);
+        }
+        planes_pass<STATS>(sc, ray, L.h, cnt, shadow);
     }
-    h = b;
+    h = L.h;
     if (h.kind == 0) {
         h.prim = NO_PRIM;
         return false;
     }
-    if (STATS) cnt.c[C_HITS]++;
+    if (STATS && !shadow) cnt.c[C_HITS]++;
     return true;
+}
+
+// The per-thread trace_ray of the path kernels: trace_bvh on scenes with
+// BVHs, else the linear scan.
+template <int TIE, bool BVH, bool STATS>
+struct PathTracer : Tracer<TIE, false, STATS> {
+    PairStack pstk;
+    __device__ __forceinline__ PathTracer(const DevScene& sc, const PairStack& p, Counters& cnt, int* status,
+                                          uint32_t trav_limit)
+        : Tracer<TIE, false, STATS>{sc, Stack{nullptr, nullptr, 0, 0}, cnt, status, trav_limit}, pstk(p)
+    {
+    }
+    __device__ __forceinline__ bool trace(const Ray& ray, Hit& h, bool shadow)
+    {
+        if (BVH) return trace_bvh<STATS>(this->sc, ray, h, shadow, pstk, this->status, this->trav_limit, this->cnt);
+        return Tracer<TIE, false, STATS>::trace(ray, h, shadow);
+    }
+};
+
+// A thread's stack in a block's dynamic shared memory: depth 8-byte entries a thread.
+__device__ __forceinline__ PairStack thread_stack(int* smem, uint32_t depth)
+{
+    return PairStack{reinterpret_cast<int2*>(smem) + threadIdx.x, (int)blockDim.x, (int)depth};
 }
 
 }  // namespace vkt

@@ -170,14 +170,18 @@ __device__ __forceinline__ void ldg256u(const void* p, uint32_t (&w)[8])
 struct Rng {
     float salt, cx, cy;
 };
-__device__ __forceinline__ float rand01(Rng& g)
+static __device__ __noinline__ float rand_at(float cx, float cy, float salt)
 {
-    g.salt = g.salt + 1.0f;
-    float ax = (g.cx + g.salt) * 5.0f;
-    float ay = (g.cy + g.salt) * 5.0f;
+    float ax = (cx + salt) * 5.0f;
+    float ay = (cy + salt) * 5.0f;
     float dp = ax * 23.14069263277926f + ay * 2.665144142690225f;
     float v = pcos(dp) * 12345.6789f;
     return v - floorf(v);
+}
+__device__ __forceinline__ float rand01(Rng& g)
+{
+    g.salt = g.salt + 1.0f;
+    return rand_at(g.cx, g.cy, g.salt);
 }
 
 // ------------------------------------------------------------ scene data --

@@ -47,50 +47,58 @@ __device__ __forceinline__ Ray primary_ray_at(const TraceArgs& a, float ux, floa
     return Ray{a.fr.cpos, normalize(dir)};
 }
 
-// Closest hit of a path ray: over the compressed 8-wide BVH where the scene
-// has one (the same hit, fewer dependent fetches), else the plain traversal.
-template <class TR>
-__device__ __forceinline__ bool closest(TR& tr, const TraceArgs& a, const PairStack& pstk, const Ray& ray, Hit& h,
-                                        Counters& cnt)
+// The pixel (x, y) on both sides of an outline: its forward value for the
+// primary rays r[0] and r[1] (through other image points than the pixel's own
+// sample point) whose closest hits h0[k] are given (found0[k]: it hit): every
+// sample (the pixel's random numbers) through the radiance loop
+// (Tracer.comp:433-553), Reinhard, gamma 1/2.2 and the dither, as
+// resolve_pixel (:578-590).  Every sample starts with the same primary ray, so
+// its hit is traced once, by the caller.  Returns the values' difference,
+// first minus second.  One loop runs both sides' samples bounce after bounce.
+// SYNC: as shade_bounce; lanes that are not `on` take part without a pixel.
+template <bool SYNC, class TR>
+__device__ __forceinline__ V3 pixel_difference(TR& tr, const TraceArgs& a, bool on, uint32_t x, uint32_t y,
+                                               const Ray (&r)[2], const bool (&found0)[2], const Hit (&h0)[2])
 {
-    if (a.sc.tri_cw8 != nullptr) return closest_cw8<false>(a.sc, ray, h, pstk, a.status, a.trav_limit, cnt);
-    return tr.trace(ray, h, false);
-}
-
-// The forward value of pixel (x, y) for the primary ray r (through another
-// image point than the pixel's own sample point) whose closest hit h0 is
-// given (found0: it hit): every sample (the pixel's random numbers) through
-// the radiance loop (Tracer.comp:433-553), Reinhard, gamma 1/2.2 and the
-// dither, as resolve_pixel (:578-590).  Every sample starts with the same
-// primary ray, so its hit is traced once, by the caller.
-template <class TR>
-__device__ __forceinline__ V3 pixel_value_from(TR& tr, const TraceArgs& a, const PairStack& pstk, uint32_t x,
-                                               uint32_t y, const Ray& r, bool found0, const Hit& h0, Counters& cnt)
-{
+    V3 diff = splat(0.0f), accum = splat(0.0f), acc = splat(0.0f), mask = splat(1.0f);
     Rng g;
     seed_rng(a, x, y, g);
-    V3 accum = splat(0.0f);
-    for (uint32_t s = 0; s < a.spp; ++s) {
-        V3 acc = splat(0.0f), mask = splat(1.0f);
-        Ray ray = r;
-        for (uint32_t depth = 0; depth < a.max_depth; ++depth) {
+    uint32_t sample = 0, depth = 0;
+    bool second = false;
+    Ray ray = r[0];
+    for (;;) {
+        if (!(SYNC ? __any_sync(0xFFFFFFFFu, on) : on)) break;
+        Hit h = second ? h0[1] : h0[0];
+        bool found = second ? found0[1] : found0[0];
+        if (on) {
             acc = vclamp01(acc);
-            Hit h = h0;
-            bool found = found0;
             if (depth > 0) {
                 h.t = depth_tmax(depth);
-                found = closest(tr, a, pstk, ray, h, cnt);
+                found = tr.trace(ray, h, false);
             }
-            if (!shade_bounce(tr, a, depth, found, h, ray, acc, mask, g)) break;
         }
+        if (SYNC) __syncwarp();
+        const bool cont = shade_bounce<true, SYNC>(tr, a, on, depth, found, h, ray, acc, mask, g);
+        if (!on || (cont && ++depth < a.max_depth)) continue;
         accum = accum + acc;
+        depth = 0;
+        acc = splat(0.0f);
+        mask = splat(1.0f);
+        if (++sample == a.spp) {
+            V3 v = accum / (float)a.spp;
+            v = v / (v + splat(1.0f));
+            const float gam = 1.0f / 2.2f;
+            v = v3(powf(v.x, gam), powf(v.y, gam), powf(v.z, gam)) + splat(rand01(g) / 64.0f);
+            diff = second ? diff - v : v;
+            on = !second;
+            second = true;
+            sample = 0;
+            accum = splat(0.0f);
+            seed_rng(a, x, y, g);
+        }
+        ray = second ? r[1] : r[0];
     }
-    accum = accum / (float)a.spp;
-    accum = accum / (accum + splat(1.0f));
-    const float gam = 1.0f / 2.2f;
-    accum = v3(powf(accum.x, gam), powf(accum.y, gam), powf(accum.z, gam));
-    const float dither = rand01(g) / 64.0f;
-    return accum + splat(dither);
+    return diff;
 }
 
 // The camera-space coefficients q = (lambda, mu, nu) of X:
@@ -109,20 +117,21 @@ __device__ __forceinline__ V3 cam_coeffs(const EdgeArgs& e, const TraceArgs& a, 
 // (I_inside - I_outside), the pixel evaluated for primary rays through the
 // inside point (ix, iy), whose closest hit hin is known, and the outside
 // point (ox, oy).
-template <class TR>
-__device__ __forceinline__ float part_weight(TR& tr, const TraceArgs& a, const PairStack& pstk, const EdgeArgs& e,
-                                             uint32_t px, uint32_t py, float ix, float iy, float ox, float oy,
-                                             const Hit& hin, Counters& cnt)
+template <bool SYNC, class TR>
+__device__ __forceinline__ float part_weight(TR& tr, const TraceArgs& a, const EdgeArgs& e, bool on, uint32_t px,
+                                             uint32_t py, float ix, float iy, float ox, float oy, const Hit& hin)
 {
     const float4 dl = __ldg(e.dldi + (size_t)py * a.width + px);
-    const Ray rin = primary_ray_at(a, ix, iy);
-    const Ray rout = primary_ray_at(a, ox, oy);
-    Hit hout;
-    hout.t = depth_tmax(0);
-    const bool fout = closest(tr, a, pstk, rout, hout, cnt);
-    const V3 vin = pixel_value_from(tr, a, pstk, px, py, rin, true, hin, cnt);
-    const V3 vout = pixel_value_from(tr, a, pstk, px, py, rout, fout, hout, cnt);
-    return dl.x * (vin.x - vout.x) + dl.y * (vin.y - vout.y) + dl.z * (vin.z - vout.z);
+    const Ray r[2] = {primary_ray_at(a, ix, iy), primary_ray_at(a, ox, oy)};
+    Hit h0[2] = {hin, hin};
+    bool found0[2] = {true, false};
+    if (on) {
+        h0[1].t = depth_tmax(0);
+        found0[1] = tr.trace(r[1], h0[1], false);
+    }
+    if (SYNC) __syncwarp();
+    const V3 d = pixel_difference<SYNC>(tr, a, on, px, py, r, found0, h0);
+    return dl.x * d.x + dl.y * d.y + dl.z * d.z;
 }
 
 // Block sum of the three camera-axis contributions in FP64, added to e.gcam.
@@ -160,13 +169,7 @@ __global__ void __launch_bounds__(128) k_edge_campos(TraceArgs a, EdgeArgs e)
     Counters cnt;
 #pragma unroll
     for (int k = 0; k < C_COUNT; ++k) cnt.c[k] = 0;
-    Tracer<TIE, BVH, false> tr{a.sc,
-                               Stack{smem + tid, reinterpret_cast<float*>(smem + (size_t)a.stack_depth * blockDim.x) + tid,
-                                     (int)blockDim.x, (int)a.stack_depth},
-                               cnt, a.status, a.trav_limit};
-    // the 8-wide traversal's stack of node groups, after the plain traversal's
-    const PairStack pstk{reinterpret_cast<int2*>(smem + 2 * (size_t)a.stack_depth * blockDim.x) + tid,
-                         (int)blockDim.x, (int)a.stack_depth};
+    PathTracer<TIE, BVH, false> tr(a.sc, thread_stack(smem, a.stack_depth), cnt, a.status, a.trav_limit);
     float contrib[3] = {0.0f, 0.0f, 0.0f};
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + tid;
     const uint64_t total = (uint64_t)a.sc.nt * 3u * e.samples;
@@ -247,7 +250,7 @@ __global__ void __launch_bounds__(128) k_edge_campos(TraceArgs a, EdgeArgs e)
                             if (dot(e1, cross(rin.d, e2)) >= EPSILON) {
                                 Hit hin;
                                 hin.t = depth_tmax(0);
-                                if (closest(tr, a, pstk, rin, hin, cnt) && hin.prim == tri_id) {
+                                if (tr.trace(rin, hin, false) && hin.prim == tri_id) {
                                     // velocity factors of the part: (n . du/dc_j) * its length,
                                     // at the 3D point (1 / lambda is linear along the image)
                                     float vel[3];
@@ -275,7 +278,7 @@ __global__ void __launch_bounds__(128) k_edge_campos(TraceArgs a, EdgeArgs e)
                                                            __uint_as_float(px | py << 16));
                                         r[2] = make_float4(vel[0], vel[1], vel[2], 0.0f);
                                     } else {
-                                        const float w = part_weight(tr, a, pstk, e, px, py, ix, iy, ox, oy, hin, cnt);
+                                        const float w = part_weight<false>(tr, a, e, true, px, py, ix, iy, ox, oy, hin);
                                         if (w != 0.0f && isfinite(w)) {
 #pragma unroll
                                             for (int j = 0; j < 3; ++j) contrib[j] += w * vel[j];
@@ -301,7 +304,8 @@ __global__ void __launch_bounds__(128) k_edge_campos(TraceArgs a, EdgeArgs e)
 }
 
 // The visible parts the walk handed over: one per thread (grid-stride), the
-// pixel on both sides of each; block sums in FP64.
+// pixel on both sides of each; block sums in FP64.  The warp's lanes go
+// through both sides' samples bounce by bounce together.
 template <int TIE, bool BVH>
 __global__ void __launch_bounds__(128) k_edge_values(TraceArgs a, EdgeArgs e)
 {
@@ -311,17 +315,14 @@ __global__ void __launch_bounds__(128) k_edge_values(TraceArgs a, EdgeArgs e)
     Counters cnt;
 #pragma unroll
     for (int k = 0; k < C_COUNT; ++k) cnt.c[k] = 0;
-    Tracer<TIE, BVH, false> tr{a.sc,
-                               Stack{smem + tid, reinterpret_cast<float*>(smem + (size_t)a.stack_depth * blockDim.x) + tid,
-                                     (int)blockDim.x, (int)a.stack_depth},
-                               cnt, a.status, a.trav_limit};
-    const PairStack pstk{reinterpret_cast<int2*>(smem + 2 * (size_t)a.stack_depth * blockDim.x) + tid,
-                         (int)blockDim.x, (int)a.stack_depth};
+    PathTracer<TIE, BVH, false> tr(a.sc, thread_stack(smem, a.stack_depth), cnt, a.status, a.trav_limit);
     float contrib[3] = {0.0f, 0.0f, 0.0f};
     const uint32_t found = *e.nsegs;
     const uint32_t n = found < e.seg_cap ? found : e.seg_cap;
-    for (uint32_t r = blockIdx.x * blockDim.x + tid; r < n; r += gridDim.x * blockDim.x) {
-        const float4* rec = e.segs + (size_t)kEdgeSegFloat4 * r;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+        const uint32_t r = base + tid;
+        const bool on = r < n;
+        const float4* rec = e.segs + (size_t)kEdgeSegFloat4 * (on ? r : 0);
         const float4 pts = rec[0], hr = rec[1], vel = rec[2];
         Hit hin;
         hin.t = hr.x;
@@ -329,8 +330,8 @@ __global__ void __launch_bounds__(128) k_edge_values(TraceArgs a, EdgeArgs e)
         hin.slot = __float_as_uint(hr.z);
         hin.kind = 1;
         const uint32_t pp = __float_as_uint(hr.w);
-        const float w = part_weight(tr, a, pstk, e, pp & 0xFFFFu, pp >> 16, pts.x, pts.y, pts.z, pts.w, hin, cnt);
-        if (w != 0.0f && isfinite(w)) {
+        const float w = part_weight<true>(tr, a, e, on, pp & 0xFFFFu, pp >> 16, pts.x, pts.y, pts.z, pts.w, hin);
+        if (on && w != 0.0f && isfinite(w)) {
             contrib[0] += w * vel.x;
             contrib[1] += w * vel.y;
             contrib[2] += w * vel.z;
@@ -343,7 +344,7 @@ template <int TIE, bool BVH>
 static cudaError_t edge_t(const TraceArgs& a, const EdgeArgs& e, cudaStream_t st)
 {
     const uint32_t block = 128;
-    const size_t smem = 2 * (size_t)a.stack_depth * block * 8;  // plain and 8-wide traversal stacks
+    const size_t smem = BVH ? (size_t)a.stack_depth * block * 8 : 0;
     auto k = k_edge_campos<TIE, BVH>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const uint64_t n = (uint64_t)a.sc.nt * 3u * e.samples;

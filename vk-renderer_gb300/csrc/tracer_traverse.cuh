@@ -2,7 +2,7 @@
 // kernel's lanes, the forward and adjoint finishing kernels): the encoded
 // child references, strict-tie acceptance, a lane's traversal state, the
 // shared-memory stack, the plane scan, primitive tests, and one thread's
-// closest hit over the pre-encoded BVHs.
+// pass over a pre-encoded BVH.
 #pragma once
 
 #include "tracer_core.cuh"
@@ -39,10 +39,13 @@ struct Lane {
 };
 
 // Planes after the BVHs (unbounded; scanned linearly, Tracer.comp:414-428).
+// any: stop at the first hit.
 template <bool STATS>
-__device__ __forceinline__ void planes_pass(const DevScene& sc, const Ray& ray, Hit& h, Counters& cnt)
+__device__ __forceinline__ void planes_pass(const DevScene& sc, const Ray& ray, Hit& h, Counters& cnt,
+                                            bool any = false)
 {
-    for (uint32_t i = 0; i < sc.np; ++i) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < sc.np && !(any && h.kind); ++i) {
         if (STATS) cnt.c[C_PLANES]++;
         const float4 q = __ldg(sc.planes + 4 * (size_t)i + 3);
         const float tt = plane_intersect(ray, v3(q), q.w);
@@ -115,75 +118,54 @@ __device__ __forceinline__ void test_prim_sc(const DevScene& sc, Lane& L, const 
     }
 }
 
-// Closest hit of one ray by one thread over the pre-encoded BVHs, for the
-// finishing kernels: the extend kernel's node step, leaf test and acceptance
-// (strict ties) without the warp's phases -- a leaf is tested as soon as it is
-// reached -- so the same hit as extend and as the plain traversal.  h.t holds
-// tmax on entry; on a miss h.kind = 0 and h.prim = NO_PRIM, as Tracer::trace.
+// One ray's pass over a pre-encoded binary BVH by one thread (L.pass: 0
+// triangles, 1 spheres): the extend kernel's node step, leaf test and
+// acceptance (strict ties) without the warp's phases -- a leaf is tested as
+// soon as it is reached -- so the same hit.  any: stop at the first hit.
 template <bool STATS>
-__device__ __forceinline__ bool closest_enc(const DevScene& sc, const Ray& ray, Hit& h, const PairStack& stk,
-                                            int* status, uint32_t trav_limit, Counters& cnt)
+__device__ __forceinline__ void enc_pass(const DevScene& sc, const Ray& ray, Lane& L, bool any, const PairStack& stk,
+                                         int* status, uint32_t trav_limit, Counters& cnt)
 {
-    if (STATS) cnt.c[C_CLOSEST]++;
-    Lane L;
-    L.h.t = h.t;
-    L.h.prim = 0;  // see accept_strict
-    L.h.kind = 0;
-    L.h.slot = 0;
-    if (!isnan3(ray.d)) {
-        L.br = make_boxray(ray);
-        for (int pass = 0; pass < 2; ++pass) {
-            const bool any = pass == 0 ? (sc.n_tri_nodes > 0 && sc.nt > 0) : (sc.n_sph_nodes > 0 && sc.ns > 0);
-            if (!any) continue;
-            L.pass = pass;
-            L.prims = pass == 0 ? sc.tri : sc.sph_geo;
-            L.nodes = pass == 0 ? sc.tri_enc : sc.sph_enc;
-            L.sp = 0;
-            uint32_t steps = 0;
-            float4 rlo, rhi;
-            ldg256(L.nodes, rlo, rhi);
-            if (STATS) cnt.c[C_NODES]++;
-            float tn;
-            int cur = box_hit(L.br, rlo, rhi, L.h.t, tn) ? __float_as_int(rlo.w) : 0;
-            while (cur != 0) {
-                if (cur < 0) {
-                    int first, count;
-                    leaf_dec(cur, first, count);
-                    for (int k = 0; k < count; ++k) test_prim_sc<STATS>(sc, L, ray, first + k, cnt);
-                    cur = pop(L, stk);
-                    continue;
-                }
-                if (++steps > trav_limit) {
-                    atomicCAS(status, ST_OK, ST_TRAVERSAL_LIMIT);
-                    break;
-                }
-                const float4* c = L.nodes + 2 * (size_t)cur;
-                float4 lo0, hi0, lo1, hi1;
-                ldg256(c, lo0, hi0);
-                ldg256(c + 2, lo1, hi1);
-                if (STATS) cnt.c[C_NODES] += 2;
-                float t0, t1;
-                const bool h0 = box_hit(L.br, lo0, hi0, L.h.t, t0);
-                const bool h1 = box_hit(L.br, lo1, hi1, L.h.t, t1);
-                if (!h0 && !h1) {
-                    cur = pop(L, stk);
-                } else {
-                    const bool swap = h1 && (!h0 || t1 < t0);
-                    const int e0 = __float_as_int(lo0.w), e1 = __float_as_int(lo1.w);
-                    cur = swap ? e1 : e0;
-                    if (h0 && h1) push(L, stk, swap ? e0 : e1, swap ? t0 : t1, status);
-                }
-            }
+    L.prims = L.pass == 0 ? sc.tri : sc.sph_geo;
+    L.nodes = L.pass == 0 ? sc.tri_enc : sc.sph_enc;
+    L.sp = 0;
+    uint32_t steps = 0;
+    float4 rlo, rhi;
+    ldg256(L.nodes, rlo, rhi);
+    if (STATS) cnt.c[C_NODES]++;
+    float tn;
+    int cur = box_hit(L.br, rlo, rhi, L.h.t, tn) ? __float_as_int(rlo.w) : 0;
+    while (cur != 0) {
+        if (cur < 0) {
+            int first, count;
+            leaf_dec(cur, first, count);
+#pragma unroll 1
+            for (int k = 0; k < count; ++k) test_prim_sc<STATS>(sc, L, ray, first + k, cnt);
+            if (any && L.h.kind) return;
+            cur = pop(L, stk);
+            continue;
         }
-        planes_pass<STATS>(sc, ray, L.h, cnt);
+        if (++steps > trav_limit) {
+            atomicCAS(status, ST_OK, ST_TRAVERSAL_LIMIT);
+            return;
+        }
+        const float4* c = L.nodes + 2 * (size_t)cur;
+        float4 lo0, hi0, lo1, hi1;
+        ldg256(c, lo0, hi0);
+        ldg256(c + 2, lo1, hi1);
+        if (STATS) cnt.c[C_NODES] += 2;
+        float t0, t1;
+        const bool h0 = box_hit(L.br, lo0, hi0, L.h.t, t0);
+        const bool h1 = box_hit(L.br, lo1, hi1, L.h.t, t1);
+        if (!h0 && !h1) {
+            cur = pop(L, stk);
+        } else {
+            const bool swap = h1 && (!h0 || t1 < t0);
+            const int e0 = __float_as_int(lo0.w), e1 = __float_as_int(lo1.w);
+            cur = swap ? e1 : e0;
+            if (h0 && h1) push(L, stk, swap ? e0 : e1, swap ? t0 : t1, status);
+        }
     }
-    h = L.h;
-    if (h.kind == 0) {
-        h.prim = NO_PRIM;
-        return false;
-    }
-    if (STATS) cnt.c[C_HITS]++;
-    return true;
 }
 
 }  // namespace vkt

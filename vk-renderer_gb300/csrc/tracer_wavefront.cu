@@ -606,18 +606,22 @@ __device__ __forceinline__ void store_path(const WfState& s, uint32_t pid, const
 // sample and pixel bookkeeping (:578-592): the next depth, else the pixel's
 // next sample (its RNG continues where the last sample stopped), else the
 // resolve.  Returns true while the pixel has another ray to trace: p.ray, with
-// tmax depth_tmax(p.depth).  NEE: as shade_bounce.
+// tmax depth_tmax(p.depth).  NEE: as shade_bounce, every lane of the warp
+// calling this together, those with a path being on.
 template <bool NEE, class TR>
-__device__ __forceinline__ bool advance_path(TR& tr, const TraceArgs& A, uint32_t x, uint32_t y, const Hit& h,
+__device__ __forceinline__ bool advance_path(TR& tr, const TraceArgs& A, bool on, uint32_t x, uint32_t y, const Hit& h,
                                              PathRegs& p)
 {
-    const bool found = h.kind != 0;
-    if (p.sample == 0 && p.depth == 0) {
-        p.prim0 = found ? h.prim : NO_PRIM;
-        p.t0 = found ? h.t : -1.0f;
+    const bool found = on && h.kind != 0;
+    if (on) {
+        if (p.sample == 0 && p.depth == 0) {
+            p.prim0 = found ? h.prim : NO_PRIM;
+            p.t0 = found ? h.t : -1.0f;
+        }
+        p.acc = vclamp01(p.acc);
     }
-    p.acc = vclamp01(p.acc);
-    const bool cont = shade_bounce<NEE>(tr, A, p.depth, found, h, p.ray, p.acc, p.mask, p.g);
+    const bool cont = shade_bounce<NEE, NEE>(tr, A, on, p.depth, found, h, p.ray, p.acc, p.mask, p.g);
+    if (!on) return false;
     p.depth++;
     if (cont && p.depth < A.max_depth) return true;
     p.accum = p.accum + p.acc;
@@ -645,30 +649,28 @@ __global__ void __launch_bounds__(256) wf_shade(TraceArgs a, WfState s, int qsel
     Counters cnt;
 #pragma unroll
     for (int k = 0; k < C_COUNT; ++k) cnt.c[k] = 0;
-    const Stack stk{smem + threadIdx.x, reinterpret_cast<float*>(smem + (size_t)a.stack_depth * blockDim.x) + threadIdx.x,
-                    (int)blockDim.x, (int)a.stack_depth};
+    const PairStack stk = thread_stack(smem, a.stack_depth);  // shadow rays'
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         const uint32_t qi = base + threadIdx.x;
-        bool again = false;
-        uint32_t pid = 0;
-        if (qi < n) {
-            pid = queue[qi];
-            const TraceArgs& A = SCENE_ARGS(MULTI, a, slots, MULTI ? s.scene_of[pid] : 0);
-            Tracer<TIE, BVH, STATS> tr{A.sc, stk, cnt, a.status, A.trav_limit};
-            const uint32_t p = pid - A.pixel_base;
-            const uint32_t x = p % A.width, y = p / A.width;
-            PathRegs ps;
+        const bool on = qi < n;
+        const uint32_t pid = on ? queue[qi] : 0;
+        const TraceArgs& A = SCENE_ARGS(MULTI, a, slots, MULTI && on ? s.scene_of[pid] : 0);
+        PathTracer<TIE, BVH, STATS> tr(A.sc, stk, cnt, a.status, A.trav_limit);
+        const uint32_t p = pid - (on ? A.pixel_base : 0);
+        const uint32_t x = p % A.width, y = p / A.width;
+        PathRegs ps;
+        Hit h;
+        if (on) {
             load_path(s, A, pid, x, y, ps);
             const uint4 hr = s.hit[pid];
-            Hit h;
             h.t = __uint_as_float(hr.x);
             h.prim = hr.y;
             h.slot = hr.z;
             h.kind = (int)hr.w;
-            again = advance_path<NEE>(tr, A, x, y, h, ps);
-            if (again) store_path(s, pid, ps);
         }
+        const bool again = advance_path<NEE>(tr, A, on, x, y, h, ps);
+        if (again) store_path(s, pid, ps);
         warp_append(again, pid, next, &s.count[qsel ^ 1]);
     }
     if (STATS) flush_counters(a, cnt);
@@ -682,7 +684,8 @@ __global__ void __launch_bounds__(256) wf_shade(TraceArgs a, WfState s, int qsel
 // for whole frames with fewer pixels than that: the paths then need no
 // launches per round and do not wait each round for that round's slowest ray.
 // The operations per pixel are those of extend + shade, in the same order, so
-// the results are identical.
+// the results are identical.  A warp's lanes go from bounce to bounce
+// together (640x360 x 4 frame with two lights: 7.18 ms each on its own).
 // First path of a thread: queue entry = its global index; later ones from the
 // cursor count[2] (zeroed by the generate or shade that wrote the queue),
 // offset by the number of threads.
@@ -695,35 +698,37 @@ __global__ void __launch_bounds__(128) wf_finish(TraceArgs a, WfState s, int qse
     Counters cnt;
 #pragma unroll
     for (int k = 0; k < C_COUNT; ++k) cnt.c[k] = 0;
-    const Stack stk{smem + threadIdx.x, reinterpret_cast<float*>(smem + (size_t)a.stack_depth * blockDim.x) + threadIdx.x,
-                    (int)blockDim.x, (int)a.stack_depth};
-    // the closest-hit traversal's stack (8-byte entries interleaved by thread)
-    // after the shadow rays' (stk: 4-byte entries interleaved by thread, used
-    // only with NEE), so no thread's entries overlap another's
-    const size_t pbase = NEE ? 2 * (size_t)a.stack_depth * blockDim.x : 0;  // in ints
-    const PairStack pstk{reinterpret_cast<int2*>(smem + pbase) + threadIdx.x, (int)blockDim.x, (int)a.stack_depth};
+    const PairStack stk = thread_stack(smem, a.stack_depth);
     const uint32_t threads = gridDim.x * blockDim.x;
     uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x;
-    while (qi < n) {
-        const uint32_t pid = queue[qi];
-        const TraceArgs& A = SCENE_ARGS(MULTI, a, slots, MULTI ? s.scene_of[pid] : 0);
-        Tracer<TIE, BVH, STATS> tr{A.sc, stk, cnt, a.status, A.trav_limit};
+    uint32_t pid = 0, scene = 0, x = 0, y = 0;
+    PathRegs ps;
+    bool on = false;
+    auto take = [&]() {  // the path of queue entry qi, if there is one
+        on = qi < n;
+        if (!on) return;
+        pid = queue[qi];
+        scene = MULTI ? s.scene_of[pid] : 0;
+        const TraceArgs& A = SCENE_ARGS(MULTI, a, slots, scene);
         const uint32_t p = pid - A.pixel_base;
-        const uint32_t x = p % A.width, y = p / A.width;
-        PathRegs ps;
+        x = p % A.width;
+        y = p / A.width;
         load_path(s, A, pid, x, y, ps);
-        for (;;) {
-            Hit h;
+    };
+    take();
+    while (__any_sync(0xFFFFFFFFu, on)) {
+        const TraceArgs& A = SCENE_ARGS(MULTI, a, slots, scene);
+        PathTracer<TIE, BVH, STATS> tr(A.sc, stk, cnt, a.status, A.trav_limit);
+        Hit h;
+        if (on) {
             h.t = depth_tmax(ps.depth);
-            if (BVH && A.sc.tri_cw8 != nullptr)  // triangle-only scenes with an 8-wide BVH
-                closest_cw8<STATS>(A.sc, ps.ray, h, pstk, a.status, A.trav_limit, cnt);
-            else if (BVH)
-                closest_enc<STATS>(A.sc, ps.ray, h, pstk, a.status, A.trav_limit, cnt);
-            else
-                tr.trace(ps.ray, h, false);
-            if (!advance_path<NEE>(tr, A, x, y, h, ps)) break;
+            tr.trace(ps.ray, h, false);
         }
-        qi = n > threads ? threads + atomicAdd(&s.count[2], 1u) : n;
+        __syncwarp();
+        if (!advance_path<NEE>(tr, A, on, x, y, h, ps) && on) {
+            qi = n > threads ? threads + atomicAdd(&s.count[2], 1u) : n;
+            take();
+        }
     }
     if (STATS) flush_counters(a, cnt);
 }
@@ -779,24 +784,20 @@ template <int TIE, bool BVH, bool STATS, bool MULTI>
 static cudaError_t shade_t(const TraceArgs& a, const WfState& s, const WfConfig& c, int qsel, cudaStream_t st)
 {
     auto k = c.has_emitters ? wf_shade<TIE, BVH, STATS, MULTI, true> : wf_shade<TIE, BVH, STATS, MULTI, false>;
-    const size_t smem = (BVH && c.has_emitters) ? (size_t)a.stack_depth * 256 * 8 : 0;
+    const size_t smem = (BVH && c.has_emitters) ? (size_t)a.stack_depth * 256 * 8 : 0;  // shadow rays' stack
     smem_attr(k, smem);
     k<<<c.shade_grid, 256, smem, st>>>(a, s, qsel, c.slots);
     return cudaGetLastError();
 }
 
-// Dynamic shared memory of the finishing kernel (128 threads): the closest-hit
-// stack and, with next-event estimation, the shadow rays' stack before it.
-static size_t wf_finish_smem(bool bvh, bool nee, size_t stack_depth)
-{
-    return bvh ? stack_depth * 128 * 8 * (nee ? 2 : 1) : 0;
-}
+// Dynamic shared memory of the finishing kernel (128 threads): the stacks.
+static size_t wf_finish_smem(bool bvh, size_t stack_depth) { return bvh ? stack_depth * 128 * 8 : 0; }
 
 template <int TIE, bool BVH, bool STATS, bool MULTI>
 static cudaError_t finish_t(const TraceArgs& a, const WfState& s, const WfConfig& c, int qsel, cudaStream_t st)
 {
     auto k = c.has_emitters ? wf_finish<TIE, BVH, STATS, MULTI, true> : wf_finish<TIE, BVH, STATS, MULTI, false>;
-    const size_t smem = wf_finish_smem(BVH, c.has_emitters != 0, a.stack_depth);
+    const size_t smem = wf_finish_smem(BVH, a.stack_depth);
     smem_attr(k, smem);
     k<<<c.finish_grid, 128, smem, st>>>(a, s, qsel, c.slots);
     return cudaGetLastError();
@@ -854,7 +855,7 @@ cudaError_t wf_launch_finish(const TraceArgs& a, const WfState& s, const WfConfi
 int wf_finish_blocks_per_sm(const WfConfig& c, uint32_t stack_depth)
 {
     const bool nee = c.has_emitters != 0;
-    const size_t smem = wf_finish_smem(c.bvh != 0, nee, stack_depth);
+    const size_t smem = wf_finish_smem(c.bvh != 0, stack_depth);
     if (c.multi) return c.stats ? finish_occ<TIE_STRICT, true, true, true>(smem, nee)
                                 : finish_occ<TIE_STRICT, true, false, true>(smem, nee);
     if (c.tie == TIE_REFERENCE) return c.stats ? finish_occ<TIE_REFERENCE, false, true, false>(smem, nee)
