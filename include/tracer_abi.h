@@ -209,7 +209,8 @@ typedef struct tracer_trace_params {
                                them to the end of its pixel (remaining bounces and samples) instead of
                                further rounds; a frame with fewer pixels than this runs no round at all.
                                0 = auto: twice the extend kernel's resident threads, no round below once
-                               that; 1 = never.  Same images either way. */
+                               that, or at any size on triangle-only scenes whose rays are short (an
+                               estimate from the BVH); 1 = never.  Same images either way. */
 } tracer_trace_params;
 
 typedef struct tracer_stats {

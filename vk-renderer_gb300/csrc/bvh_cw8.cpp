@@ -191,11 +191,12 @@ void append_prims(const tracer_bvh_node* nodes, uint32_t n, std::vector<uint32_t
 }  // namespace
 
 bool build_cw8(const tracer_bvh_node* nodes, uint32_t num_nodes, std::vector<Cw8Node>& out,
-               std::vector<uint32_t>& order_out, uint32_t* depth_out)
+               std::vector<uint32_t>& order_out, uint32_t* depth_out, double* cost_out)
 {
     out.clear();
     order_out.clear();
     if (depth_out) *depth_out = 0;
+    if (cost_out) *cost_out = 0.0;
     if (!nodes || num_nodes == 0) return true;
     for (uint32_t i = 0; i < num_nodes; ++i) {
         const tracer_bvh_node& n = nodes[i];
@@ -207,6 +208,8 @@ bool build_cw8(const tracer_bvh_node* nodes, uint32_t num_nodes, std::vector<Cw8
     // Which binary nodes become 8-wide nodes, which leaf children: the least
     // expected cost, bottom up (children are stored after their parents).
     const std::vector<Cut> cuts = plan_cuts(nodes, num_nodes);
+    const double root_area = area(nodes[0]);
+    if (cost_out && root_area > 0.0) *cost_out = cuts[0].cost[1] / root_area;
     struct Work {
         uint32_t wide, bin, level;
     };

@@ -60,9 +60,11 @@ constexpr uint32_t kCw8MaxNodePrims = 24;
 // primitive k.  *depth_out = levels of 8-wide nodes (the traversal stack
 // holds at most one entry per level).  Returns false (no 8-wide BVH) when a
 // leaf holds more than 6 primitives or a coordinate's magnitude exceeds 1e6
-// (the quantised slab test's range).
+// (the quantised slab test's range).  *cost_out = the plan's cost over the
+// root's surface area: what a random ray through the root box is expected to
+// visit, in nodes.
 bool build_cw8(const tracer_bvh_node* nodes, uint32_t num_nodes, std::vector<Cw8Node>& out,
-               std::vector<uint32_t>& order_out, uint32_t* depth_out);
+               std::vector<uint32_t>& order_out, uint32_t* depth_out, double* cost_out = nullptr);
 
 // The node the kernels read, 96 bytes (three 256-bit loads), as 24
 // little-endian words: a Cw8Node's boxes with the grid written out as floats

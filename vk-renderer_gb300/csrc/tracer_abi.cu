@@ -58,6 +58,7 @@ struct SceneBuffers {
     bool wide = false;        // 4-wide nodes present
     uint32_t cw8_depth = 0;   // levels of the 8-wide BVH (0: none)
     uint32_t n_cw8_nodes = 0;
+    double cw8_cost = 0.0;    // expected node visits of a ray (build_cw8)
     bool cw8 = false;         // the extend kernel may use it (triangle-only scenes)
     bool bvh = false;
     bool loaded = false;
@@ -144,6 +145,7 @@ struct tracer_ctx {
     SceneBuffers batch;                 // arena: every scene's arrays back to back
     std::vector<DevScene> batch_scenes; // pointers into the arena, one per scene
     std::vector<uint32_t> batch_depth, batch_nodes;
+    std::vector<double> batch_cost;     // per scene, as SceneBuffers::cw8_cost
     bool batch_emitters = false;
     DevBuf<TraceArgs> batch_slots;
     TraceArgs* pinned_slots = nullptr;
@@ -291,6 +293,17 @@ cudaEvent_t prof_event(tracer_ctx* c, size_t i)
     return c->prof_events[i];
 }
 
+// Triangle-only scenes without lights whose rays visit at most this many 8-wide
+// nodes (build_cw8's estimate) run no rounds: the finishing kernel alone was
+// faster by (frame 640x360 x 4 spp / 1280x720 x 4 / 1920x1080 x 8) 1.95 / 1.90 /
+// 1.84 on a soup of 500 triangles (estimate 5.1), 1.66 / 1.58 / 1.51 on 2k (9.0),
+// 1.31 / 1.22 / 1.15 on 10k (16.8); 1.35 / 1.54 / 1.25 on a height field of 2k
+// (7.2), 1.37 / 1.33 / 1.04 on 20k (10.4), 1.21 / 1.15 / 0.91 on 200k (13.8);
+// slower from 1.05 / 0.96 / 0.86 on a soup of 30k (27) to 0.91 / 0.63 / 0.54 on
+// 200k (66).
+constexpr double kCheapRays = 20.0;
+bool cheap_rays(double cost) { return cost > 0.0 && cost <= kCheapRays; }
+
 // Launches the wavefront: generate, then rounds of extend + shade until the
 // path queue is empty (read back a few rounds behind the launches) or
 // max_rounds is reached (no path needs more than spp * max_depth rounds).
@@ -305,10 +318,14 @@ cudaEvent_t prof_event(tracer_ctx* c, size_t i)
 // finishing kernel traces every pixel after generate (c3's 256^2 adjoint:
 // 1.33 ms with four rounds first; a 640x360 frame of c1's scene, 230k
 // pixels: 5.0 ms without rounds against 4.5 with them).
+// cheap: the scene's rays are short, so that a round's launches and path state
+// cost more than its traversals gain from the extend kernel: with the
+// automatic tail no round runs either (kCheapRays).
 // With adj, the adjoint's generate, shade and finishing stages run instead of
 // the forward's (a.linear = the forward image).
 int run_wavefront(tracer_ctx* c, const TraceArgs& a, WfConfig& wc, size_t nslots, uint64_t max_rounds,
-                  uint32_t stack, uint32_t wavefront, uint32_t tail, cudaStream_t st, const AdjWf* adj = nullptr)
+                  uint32_t stack, uint32_t wavefront, uint32_t tail, bool cheap, cudaStream_t st,
+                  const AdjWf* adj = nullptr)
 {
     WfState ws{c->wf_ray_o.p, c->wf_ray_d.p, c->wf_hit.p, c->wf_acc.p, c->wf_mask.p, c->wf_accum.p,
                c->wf_prim0.p, {c->wf_q0.p, c->wf_q1.p}, c->wf_count.p, c->wf_scene.p};
@@ -319,7 +336,7 @@ int run_wavefront(tracer_ctx* c, const TraceArgs& a, WfConfig& wc, size_t nslots
     const size_t sg = (nslots + 255) / 256;
     wc.shade_grid = (uint32_t)(sg < (size_t)c->sm_count * 8 ? sg : (size_t)c->sm_count * 8);
     const uint32_t resident = wc.extend_grid * wc.block;
-    const uint32_t no_rounds_below = tail == 0 ? resident : tail;
+    const uint64_t no_rounds_below = tail != 0 ? tail : cheap ? UINT64_MAX : resident;
     if (tail == 0) tail = 2 * resident;
     const int fin_per = tail <= 1 ? 0 : adj ? wf_adj_finish_blocks_per_sm(a, wc) : wf_finish_blocks_per_sm(wc, stack);
     if (fin_per <= 0) tail = 0;
@@ -493,7 +510,7 @@ int pick_width(tracer_ctx* c, const tracer_trace_params* p, uint32_t& stack, int
 // The binary leaves are split to single triangles first.  Returns false when
 // the scene gets none (bvh_cw8.h).
 bool make_cw8(const std::vector<tracer_bvh_node>& tnodes, const std::vector<float4>& tri, std::vector<W8Node>& nodes,
-              std::vector<float4>& prims, uint32_t& depth)
+              std::vector<float4>& prims, uint32_t& depth, double& cost)
 {
     if (tnodes.empty()) return false;
     for (const tracer_bvh_node& n : tnodes)
@@ -513,7 +530,7 @@ bool make_cw8(const std::vector<tracer_bvh_node>& tnodes, const std::vector<floa
     split_leaves(tnodes.data(), (uint32_t)tnodes.size(), reinterpret_cast<const double(*)[6]>(box.data()), split,
                  slot_of);
     std::vector<Cw8Node> coded;
-    if (!build_cw8(split.data(), (uint32_t)split.size(), coded, order, &depth) || !pack_w8(coded, nodes)) return false;
+    if (!build_cw8(split.data(), (uint32_t)split.size(), coded, order, &depth, &cost) || !pack_w8(coded, nodes)) return false;
     for (uint32_t& s : order) s = slot_of[s];
     prims.assign(4 * order.size(), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
     for (size_t k = 0; k < order.size(); ++k) {
@@ -768,7 +785,8 @@ int tracer_upload_scene(tracer_ctx* c, const tracer_scene_desc* d)
     std::vector<W8Node> cw8;
     std::vector<float4> cw8_prims;
     uint32_t cw8_depth = 0;
-    const bool cw8_ok = s.bvh && s.nt > 0 && make_cw8(tnodes, tri, cw8, cw8_prims, cw8_depth);
+    double cw8_cost = 0.0;
+    const bool cw8_ok = s.bvh && s.nt > 0 && make_cw8(tnodes, tri, cw8, cw8_prims, cw8_depth, cw8_cost);
 
     cudaError_t e = upload(s.tri, tri.data(), tri.size());
     if (e == cudaSuccess) e = upload(s.mats, reinterpret_cast<const float4*>(d->materials), 3 * (size_t)s.nm);
@@ -796,6 +814,7 @@ int tracer_upload_scene(tracer_ctx* c, const tracer_scene_desc* d)
     s.wide = wide_ok;
     s.cw8 = cw8_ok && s.ns == 0;
     s.cw8_depth = cw8_ok ? cw8_depth : 0u;
+    s.cw8_cost = cw8_cost;
     s.n_cw8_nodes = cw8_ok ? (uint32_t)cw8.size() : 0u;
     s.loaded = true;
     ++c->scene_version;
@@ -942,8 +961,10 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
         if (wc.wide == WF_WIDTH_8) wc.cw8_stack = s.cw8_depth;
         if (binary_asked(p)) a.sc.tri_cw8 = a.sc.tri_cw8_prims = nullptr;
         else wstack = std::max(wstack, s.cw8_depth);
+        wc.finish_w8 = s.cw8 && !binary_asked(p);
         a.stack_depth = wstack;
-        r = run_wavefront(c, a, wc, npx, (uint64_t)p->spp * p->max_depth + 1, wstack, p->wavefront, p->tail_paths, st);
+        r = run_wavefront(c, a, wc, npx, (uint64_t)p->spp * p->max_depth + 1, wstack, p->wavefront, p->tail_paths,
+                          wc.wide == WF_WIDTH_8 && cheap_rays(s.cw8_cost), st);
         if (r != TRACER_OK) return r;
     }
     if (c->profiling) cudaEventRecord(c->prof_end, st);
@@ -1233,6 +1254,7 @@ extern "C" int tracer_trace_noalloc(tracer_ctx* c, const tracer_frame* f, const 
     wc.bvh = s.bvh ? 1 : 0;
     wc.stats = 0;
     wc.has_emitters = s.ne > 0;
+    wc.finish_w8 = s.cw8 && !binary_asked(p);
     wc.block = 128;
     int per = wf_extend_blocks_per_sm(wc, stack);
     if (per <= 0) return fail(c, TRACER_ERR_INVALID_ARG, "extend kernel cannot be resident (stack %u)", stack);
@@ -1282,6 +1304,7 @@ struct PackedScene {
     std::vector<W8Node> cw8;
     std::vector<float4> cw8_prims;
     uint32_t depth = 0, wide_depth = 0, cw8_depth = 0;
+    double cw8_cost = 0.0;
     bool wide = false, cw8_ok = false;
     int status = TRACER_OK;
 };
@@ -1357,7 +1380,7 @@ void pack_scene(const tracer_scene_desc& d, PackedScene& out)
         const float* em = d.spheres[i].mat.emissive;
         if (!(em[0] == 0.0f && em[1] == 0.0f && em[2] == 0.0f)) out.emit.push_back(i);
     }
-    out.cw8_ok = d.num_triangles > 0 && make_cw8(out.tnodes, out.tri, out.cw8, out.cw8_prims, out.cw8_depth);
+    out.cw8_ok = d.num_triangles > 0 && make_cw8(out.tnodes, out.tri, out.cw8, out.cw8_prims, out.cw8_depth, out.cw8_cost);
     if (!out.cw8_ok) out.cw8_depth = 0;
 }
 
@@ -1478,6 +1501,7 @@ extern "C" int tracer_upload_scenes(tracer_ctx* c, const tracer_scene_desc* desc
     c->batch_scenes.assign(n, DevScene{});
     c->batch_depth.assign(n, 0);
     c->batch_nodes.assign(n, 0);
+    c->batch_cost.assign(n, 0.0);
     c->batch_emitters = false;
     for (uint32_t k = 0; k < n; ++k) {
         const tracer_scene_desc& d = descs[k];
@@ -1497,6 +1521,7 @@ extern "C" int tracer_upload_scenes(tracer_ctx* c, const tracer_scene_desc* desc
         b.wide_depth = std::max(b.wide_depth, p.wide_depth);
         b.cw8_depth = std::max(b.cw8_depth, p.cw8_depth);
         c->batch_depth[k] = p.depth;
+        c->batch_cost[k] = p.cw8_cost;
         c->batch_nodes[k] = (uint32_t)std::max(std::max(p.tnodes.size(), p.snodes.size()), p.cw8.size());
         c->batch_emitters = c->batch_emitters || !p.emit.empty();
     }
@@ -1648,13 +1673,18 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
         wc.stats = stats;
         wc.multi = 1;
         wc.has_emitters = c->batch_emitters;
+        wc.finish_w8 = c->batch.cw8 && !binary_asked(&p0);
         wc.block = block;
         wc.wide = wide;
         if (wide == WF_WIDTH_8) wc.cw8_stack = c->batch.cw8_depth;
         wc.slots = c->batch_slots.p;
         wc.nslots = n;
+        // the scenes' estimates, each weighted by its pixels
+        double cost = 0.0;
+        for (uint32_t k = 0; k < n; ++k) cost += c->batch_cost[k] * params[k].width * params[k].height / (double)total;
+        const bool cheap = wide == WF_WIDTH_8 && cheap_rays(cost);
         if (!use_graph) {
-            r = run_wavefront(c, a, wc, total, max_rounds, stack, p0.wavefront, p0.tail_paths, st);
+            r = run_wavefront(c, a, wc, total, max_rounds, stack, p0.wavefront, p0.tail_paths, cheap, st);
             if (r != TRACER_OK) return r;
         } else {
             WfState ws{c->wf_ray_o.p, c->wf_ray_d.p, c->wf_hit.p, c->wf_acc.p, c->wf_mask.p, c->wf_accum.p,
@@ -1667,7 +1697,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
             wc.shade_grid = (uint32_t)(sg < (size_t)c->sm_count * 8 ? sg : (size_t)c->sm_count * 8);
             // the graph bakes in sizes, launch shapes and buffer addresses
             std::vector<uint64_t> key = {n, total, max_rounds, block, stack, (uint64_t)stats, wc.extend_grid,
-                                         (uint64_t)wide, (uint64_t)binary_asked(&p0), p0.tail_paths,
+                                         (uint64_t)wide, (uint64_t)binary_asked(&p0), (uint64_t)cheap, p0.tail_paths,
                                          (uint64_t)(uintptr_t)c->wf_ray_o.p, (uint64_t)(uintptr_t)c->batch_slots.p,
                                          (uint64_t)(uintptr_t)c->b_rgba8.p, (uint64_t)(uintptr_t)c->b_rgba32f.p,
                                          (uint64_t)(uintptr_t)c->b_hit.p, mask};
@@ -1682,7 +1712,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
                 // run of this batch reaches (launched here, with read-backs).
                 // Any frame is still traced completely: the finishing kernel
                 // runs whatever paths are queued after that round.
-                r = run_wavefront(c, a, wc, total, max_rounds, stack, p0.wavefront, p0.tail_paths, st);
+                r = run_wavefront(c, a, wc, total, max_rounds, stack, p0.wavefront, p0.tail_paths, cheap, st);
                 if (r != TRACER_OK) return r;
                 const int fin_per = c->last_finish ? wf_finish_blocks_per_sm(wc, stack) : 0;
                 const uint64_t rounds = fin_per > 0 ? c->last_handover : max_rounds;
@@ -1901,13 +1931,15 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
         if (wc.wide == WF_WIDTH_8) wc.cw8_stack = s.cw8_depth;
         if (binary_asked(p)) a.sc.tri_cw8 = a.sc.tri_cw8_prims = nullptr;
         else wstack = std::max(wstack, s.cw8_depth);
+        wc.finish_w8 = s.cw8 && !binary_asked(p);
         a.stack_depth = wstack;
         const AdjWf aw{dldi, lin, ab.grad.p, s.nm, ab.pix.p, use_log ? ab.log.p : nullptr};
         c->last_kernel = TRACER_KERNEL_WAVEFRONT;
         c->last_launches = 1;  // + generate, rounds; the FP64-to-float conversion
         if (c->profiling) cudaEventRecord(c->prof_begin, st);
         // a sample takes at most max_depth rounds in each pass
-        r = run_wavefront(c, a, wc, npx, 2 * (uint64_t)p->spp * p->max_depth + 1, wstack, p->wavefront, p->tail_paths, st, &aw);
+        r = run_wavefront(c, a, wc, npx, 2 * (uint64_t)p->spp * p->max_depth + 1, wstack, p->wavefront, p->tail_paths,
+                          wc.wide == WF_WIDTH_8 && cheap_rays(s.cw8_cost), st, &aw);
         if (r != TRACER_OK) return r;
     } else {
         c->last_kernel = 3;

@@ -733,8 +733,8 @@ __global__ void __launch_bounds__(256) wf_adj_shade(TraceArgs a, WfState s, AdjW
 // The adjoint's finishing kernel (as wf_finish for the forward): each thread
 // runs queued paths to the end of their pixels -- both passes of every
 // remaining sample (pass 2 from the hit log when there is one) -- with the
-// per-thread traversal for the closest hits.
-template <int TIE, bool BVH, bool STATS>
+// per-thread traversal for the closest hits.  W8: as wf_finish.
+template <int TIE, bool BVH, bool STATS, bool W8>
 __global__ void __launch_bounds__(128) wf_adj_finish(TraceArgs a, WfState s, AdjWf w, int qsel)
 {
     extern __shared__ int smem[];
@@ -743,21 +743,33 @@ __global__ void __launch_bounds__(128) wf_adj_finish(TraceArgs a, WfState s, Adj
     Counters cnt;
 #pragma unroll
     for (int k = 0; k < C_COUNT; ++k) cnt.c[k] = 0;
-    PathTracer<TIE, BVH, STATS> tr(a.sc, thread_stack(smem, a.stack_depth), cnt, a.status, a.trav_limit);
+    PathTracer<TIE, BVH, STATS, W8> tr(a.sc, thread_stack(smem, a.stack_depth), cnt, a.status, a.trav_limit);
     const uint32_t threads = gridDim.x * blockDim.x;
     uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x;
-    while (qi < n) {
-        const uint32_t pid = queue[qi];
-        const uint32_t x = pid % a.width, y = pid / a.width;
-        AdjPath p;
+    uint32_t pid = 0, x = 0, y = 0;
+    AdjPath p;
+    bool on = false;
+    auto take = [&]() {  // the path of queue entry qi, if there is one
+        on = qi < n;
+        if (!on) return;
+        pid = queue[qi];
+        x = pid % a.width;
+        y = pid / a.width;
         adj_load(s, a, pid, x, y, p);
-        for (;;) {
-            Hit h;
+    };
+    take();
+    while (__any_sync(0xFFFFFFFFu, on)) {
+        Hit h;
+        if (on) {
             h.t = depth_tmax(p.depth);
             tr.trace(p.ray, h, false);
-            if (!adj_advance(tr, a, w, pid, x, y, h, p, w.pix + pid, s.prim0 + pid)) break;
         }
-        qi = n > threads ? threads + atomicAdd(&s.count[2], 1u) : n;
+        __syncwarp();
+        if (on && !adj_advance(tr, a, w, pid, x, y, h, p, w.pix + pid, s.prim0 + pid)) {
+            qi = n > threads ? threads + atomicAdd(&s.count[2], 1u) : n;
+            take();
+        }
+        __syncwarp();
     }
     if (STATS) flush_counters(a, cnt);
 }
@@ -781,59 +793,41 @@ cudaError_t wf_launch_adj_shade(const TraceArgs& a, const WfState& s, const AdjW
     return cudaGetLastError();
 }
 
-template <int TIE, bool BVH, bool STATS>
-static size_t adj_finish_smem(const TraceArgs& a)
-{
-    const size_t smem = BVH ? (size_t)a.stack_depth * 128 * 8 : 0;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(wf_adj_finish<TIE, BVH, STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return smem;
-}
+using AdjFinishKernel = void (*)(TraceArgs, WfState, AdjWf, int);
 
+// The kernel for the configuration and its dynamic shared memory.
 template <int TIE, bool BVH, bool STATS>
-static cudaError_t adj_finish_t(const TraceArgs& a, const WfState& s, const AdjWf& w, const WfConfig& c, int qsel,
-                                cudaStream_t st)
+static AdjFinishKernel adj_finish_kernel(const TraceArgs& a, const WfConfig& c, size_t& smem)
 {
-    wf_adj_finish<TIE, BVH, STATS><<<c.finish_grid, 128, adj_finish_smem<TIE, BVH, STATS>(a), st>>>(a, s, w, qsel);
-    return cudaGetLastError();
-}
-
-template <int TIE, bool BVH, bool STATS>
-static int adj_finish_occ(const TraceArgs& a)
-{
-    int n = 0;
-    const size_t smem = adj_finish_smem<TIE, BVH, STATS>(a);
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_adj_finish<TIE, BVH, STATS>, 128, smem) == cudaSuccess
-               ? n
-               : 0;
+    const AdjFinishKernel k = BVH && c.finish_w8 ? wf_adj_finish<TIE, BVH, STATS, BVH> : wf_adj_finish<TIE, BVH, STATS, false>;
+    smem = BVH ? (size_t)a.stack_depth * 128 * 8 : 0;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return k;
 }
 
 template <bool STATS>
-static cudaError_t adj_finish_s(const TraceArgs& a, const WfState& s, const AdjWf& w, const WfConfig& c, int qsel,
-                                cudaStream_t st)
+static AdjFinishKernel adj_finish_s(const TraceArgs& a, const WfConfig& c, size_t& smem)
 {
-    if (c.tie == TIE_REFERENCE) return adj_finish_t<TIE_REFERENCE, false, STATS>(a, s, w, c, qsel, st);
-    if (c.bvh) return adj_finish_t<TIE_STRICT, true, STATS>(a, s, w, c, qsel, st);
-    return adj_finish_t<TIE_STRICT, false, STATS>(a, s, w, c, qsel, st);
-}
-
-template <bool STATS>
-static int adj_finish_occ_s(const TraceArgs& a, const WfConfig& c)
-{
-    if (c.tie == TIE_REFERENCE) return adj_finish_occ<TIE_REFERENCE, false, STATS>(a);
-    if (c.bvh) return adj_finish_occ<TIE_STRICT, true, STATS>(a);
-    return adj_finish_occ<TIE_STRICT, false, STATS>(a);
+    if (c.tie == TIE_REFERENCE) return adj_finish_kernel<TIE_REFERENCE, false, STATS>(a, c, smem);
+    if (c.bvh) return adj_finish_kernel<TIE_STRICT, true, STATS>(a, c, smem);
+    return adj_finish_kernel<TIE_STRICT, false, STATS>(a, c, smem);
 }
 
 cudaError_t wf_launch_adj_finish(const TraceArgs& a, const WfState& s, const AdjWf& w, const WfConfig& c, int qsel,
                                  cudaStream_t st)
 {
-    return c.stats ? adj_finish_s<true>(a, s, w, c, qsel, st) : adj_finish_s<false>(a, s, w, c, qsel, st);
+    size_t smem = 0;
+    const AdjFinishKernel k = c.stats ? adj_finish_s<true>(a, c, smem) : adj_finish_s<false>(a, c, smem);
+    k<<<c.finish_grid, 128, smem, st>>>(a, s, w, qsel);
+    return cudaGetLastError();
 }
 
 int wf_adj_finish_blocks_per_sm(const TraceArgs& a, const WfConfig& c)
 {
-    return c.stats ? adj_finish_occ_s<true>(a, c) : adj_finish_occ_s<false>(a, c);
+    size_t smem = 0;
+    const AdjFinishKernel k = c.stats ? adj_finish_s<true>(a, c, smem) : adj_finish_s<false>(a, c, smem);
+    int n = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 128, smem) == cudaSuccess ? n : 0;
 }
 
 template <int TIE, bool BVH, bool CAM>

@@ -162,15 +162,58 @@ struct alignas(16) W8Lane {
 };
 static_assert(sizeof(W8Lane) == 48, "lane record is 48 bytes");
 
-// trace_ray of one ray by one thread over a scene with BVHs (strict ties):
-// the triangles over the 8-wide BVH where the scene has one (the extend
+// One ray's pass over the triangles' 8-wide BVH by one thread: the extend
 // kernel's node visit and triangle test, a node's leaves tested right after
-// the visit), else, and the spheres, over the binary BVHs, then the planes.
-// The same hit as every other traversal.  h.t holds tmax on entry; on a miss
-// h.kind = 0 and h.prim = NO_PRIM.  shadow: any hit will do.  stk: the
-// thread's stack (8-byte entries, interleaved by thread), at least as deep as
-// either BVH.
+// the visit.  any: stop at the first hit.
 template <bool STATS>
+__device__ __forceinline__ void w8_pass(const DevScene& sc, const Ray& ray, const W8Ray& cr, Hit& h, bool any,
+                                        const PairStack& stk, int* status, uint32_t trav_limit, Counters& cnt)
+{
+    uint2 G = w8_root();
+    int sp = 0;
+    uint32_t steps = 0;
+    for (;;) {
+        if (!w8_any(G)) {
+            if (sp == 0) break;
+            --sp;
+            const int2 e = stk.e[sp * stk.stride];
+            G = make_uint2((uint32_t)e.x, (uint32_t)e.y);
+        }
+        if (++steps > trav_limit) {
+            atomicCAS(status, ST_OK, ST_TRAVERSAL_LIMIT);
+            break;
+        }
+        const uint32_t idx = w8_next(G, cr);
+        if (w8_any(G)) {
+            if (sp >= stk.cap) {
+                atomicCAS(status, ST_OK, ST_STACK_OVERFLOW);
+            } else {
+                stk.e[sp * stk.stride] = make_int2((int)G.x, (int)G.y);
+                ++sp;
+            }
+        }
+        uint2 P;
+        w8_visit(sc.tri_cw8, idx, cr, h.t, G, P);
+        if (STATS) cnt.c[C_NODES] += 3;
+        while (w8_any(P)) {
+            bool two;
+            const uint32_t k = w8_next_leaf(P, two);
+            cw8_test_tri2<STATS>(sc.tri_cw8_prims, k, two, ray, h, cnt);
+        }
+        if (any && h.kind) break;
+    }
+}
+
+// trace_ray of one ray by one thread over a scene with BVHs (strict ties):
+// the triangles over the 8-wide BVH where the scene has one, else, and the
+// spheres, over the binary BVHs, then the planes.  The same hit as every
+// other traversal.  h.t holds tmax on entry; on a miss h.kind = 0 and h.prim =
+// NO_PRIM.  shadow: any hit will do.  stk: the thread's stack (8-byte entries,
+// interleaved by thread), at least as deep as either BVH.
+// W8: a triangle-only scene with an 8-wide BVH and a closest hit: no binary
+// passes, whose code and registers cost the finishing kernels a tenth (256^2
+// adjoint 593 against 527 us).
+template <bool STATS, bool W8>
 __device__ __forceinline__ bool trace_bvh(const DevScene& sc, const Ray& ray, Hit& h, bool shadow, const PairStack& stk,
                                           int* status, uint32_t trav_limit, Counters& cnt)
 {
@@ -185,46 +228,14 @@ __device__ __forceinline__ bool trace_bvh(const DevScene& sc, const Ray& ray, Hi
     L.h.slot = 0;
     if (!isnan3(ray.d)) {
         const W8Ray cr = make_w8ray(ray);
-        const bool wide = sc.tri_cw8 != nullptr;
-        if (wide) {
-            uint2 G = w8_root();
-            int sp = 0;
-            uint32_t steps = 0;
-            for (;;) {
-                if (!w8_any(G)) {
-                    if (sp == 0) break;
-                    --sp;
-                    const int2 e = stk.e[sp * stk.stride];
-                    G = make_uint2((uint32_t)e.x, (uint32_t)e.y);
-                }
-                if (++steps > trav_limit) {
-                    atomicCAS(status, ST_OK, ST_TRAVERSAL_LIMIT);
-                    break;
-                }
-                const uint32_t idx = w8_next(G, cr);
-                if (w8_any(G)) {
-                    if (sp >= stk.cap) {
-                        atomicCAS(status, ST_OK, ST_STACK_OVERFLOW);
-                    } else {
-                        stk.e[sp * stk.stride] = make_int2((int)G.x, (int)G.y);
-                        ++sp;
-                    }
-                }
-                uint2 P;
-                w8_visit(sc.tri_cw8, idx, cr, L.h.t, G, P);
-                if (STATS) cnt.c[C_NODES] += 3;
-                while (w8_any(P)) {
-                    bool two;
-                    const uint32_t k = w8_next_leaf(P, two);
-                    cw8_test_tri2<STATS>(sc.tri_cw8_prims, k, two, ray, L.h, cnt);
-                }
-                if (shadow && L.h.kind) break;
+        const bool wide = W8 || sc.tri_cw8 != nullptr;
+        if (wide) w8_pass<STATS>(sc, ray, cr, L.h, shadow, stk, status, trav_limit, cnt);
+        if (!W8) {
+            L.br = cr.br;
+            for (L.pass = wide ? 1 : 0; L.pass < 2 && !(shadow && L.h.kind); ++L.pass) {
+                const bool any = L.pass == 0 ? (sc.n_tri_nodes > 0 && sc.nt > 0) : (sc.n_sph_nodes > 0 && sc.ns > 0);
+                if (any) enc_pass<STATS>(sc, ray, L, shadow, stk, status, trav_limit, cnt);
             }
-        }
-        L.br = cr.br;
-        for (L.pass = wide ? 1 : 0; L.pass < 2 && !(shadow && L.h.kind); ++L.pass) {
-            const bool any = L.pass == 0 ? (sc.n_tri_nodes > 0 && sc.nt > 0) : (sc.n_sph_nodes > 0 && sc.ns > 0);
-            if (any) enc_pass<STATS>(sc, ray, L, shadow, stk, status, trav_limit, cnt);
         }
         planes_pass<STATS>(sc, ray, L.h, cnt, shadow);
     }
@@ -239,7 +250,7 @@ __device__ __forceinline__ bool trace_bvh(const DevScene& sc, const Ray& ray, Hi
 
 // The per-thread trace_ray of the path kernels: trace_bvh on scenes with
 // BVHs, else the linear scan.
-template <int TIE, bool BVH, bool STATS>
+template <int TIE, bool BVH, bool STATS, bool W8 = false>
 struct PathTracer : Tracer<TIE, false, STATS> {
     PairStack pstk;
     __device__ __forceinline__ PathTracer(const DevScene& sc, const PairStack& p, Counters& cnt, int* status,
@@ -249,7 +260,8 @@ struct PathTracer : Tracer<TIE, false, STATS> {
     }
     __device__ __forceinline__ bool trace(const Ray& ray, Hit& h, bool shadow)
     {
-        if (BVH) return trace_bvh<STATS>(this->sc, ray, h, shadow, pstk, this->status, this->trav_limit, this->cnt);
+        if (BVH)
+            return trace_bvh<STATS, W8>(this->sc, ray, h, shadow, pstk, this->status, this->trav_limit, this->cnt);
         return Tracer<TIE, false, STATS>::trace(ray, h, shadow);
     }
 };

@@ -685,11 +685,15 @@ __global__ void __launch_bounds__(256) wf_shade(TraceArgs a, WfState s, int qsel
 // launches per round and do not wait each round for that round's slowest ray.
 // The operations per pixel are those of extend + shade, in the same order, so
 // the results are identical.  A warp's lanes go from bounce to bounce
-// together (640x360 x 4 frame with two lights: 7.18 ms each on its own).
+// together (640x360 x 4 frame with two lights: 2.25 ms, 7.18 each on its own).
 // First path of a thread: queue entry = its global index; later ones from the
 // cursor count[2] (zeroed by the generate or shade that wrote the queue),
 // offset by the number of threads.
-template <int TIE, bool BVH, bool STATS, bool MULTI, bool NEE>
+// W8: triangle-only scenes with an 8-wide BVH, without lights.  (Lanes with
+// finished rays shading while the others' walks wait, once 13, 10 or 8 of 16
+// are finished, instead of all: 720p mesh 3354, 3449, 3554 against 3481 us, but
+// a 10k-triangle soup 1240, 1377, 1384 against 1146.)
+template <int TIE, bool BVH, bool STATS, bool MULTI, bool NEE, bool W8>
 __global__ void __launch_bounds__(128) wf_finish(TraceArgs a, WfState s, int qsel, const TraceArgs* slots)
 {
     extern __shared__ int smem[];
@@ -718,7 +722,7 @@ __global__ void __launch_bounds__(128) wf_finish(TraceArgs a, WfState s, int qse
     take();
     while (__any_sync(0xFFFFFFFFu, on)) {
         const TraceArgs& A = SCENE_ARGS(MULTI, a, slots, scene);
-        PathTracer<TIE, BVH, STATS> tr(A.sc, stk, cnt, a.status, A.trav_limit);
+        PathTracer<TIE, BVH, STATS, W8> tr(A.sc, stk, cnt, a.status, A.trav_limit);
         Hit h;
         if (on) {
             h.t = depth_tmax(ps.depth);
@@ -793,10 +797,20 @@ static cudaError_t shade_t(const TraceArgs& a, const WfState& s, const WfConfig&
 // Dynamic shared memory of the finishing kernel (128 threads): the stacks.
 static size_t wf_finish_smem(bool bvh, size_t stack_depth) { return bvh ? stack_depth * 128 * 8 : 0; }
 
+using FinishKernel = void (*)(TraceArgs, WfState, int, const TraceArgs*);
+
+template <int TIE, bool BVH, bool STATS, bool MULTI>
+static FinishKernel finish_kernel(const WfConfig& c)
+{
+    if (c.has_emitters) return wf_finish<TIE, BVH, STATS, MULTI, true, false>;
+    if (BVH && c.finish_w8) return wf_finish<TIE, BVH, STATS, MULTI, false, BVH>;
+    return wf_finish<TIE, BVH, STATS, MULTI, false, false>;
+}
+
 template <int TIE, bool BVH, bool STATS, bool MULTI>
 static cudaError_t finish_t(const TraceArgs& a, const WfState& s, const WfConfig& c, int qsel, cudaStream_t st)
 {
-    auto k = c.has_emitters ? wf_finish<TIE, BVH, STATS, MULTI, true> : wf_finish<TIE, BVH, STATS, MULTI, false>;
+    const FinishKernel k = finish_kernel<TIE, BVH, STATS, MULTI>(c);
     const size_t smem = wf_finish_smem(BVH, a.stack_depth);
     smem_attr(k, smem);
     k<<<c.finish_grid, 128, smem, st>>>(a, s, qsel, c.slots);
@@ -804,9 +818,9 @@ static cudaError_t finish_t(const TraceArgs& a, const WfState& s, const WfConfig
 }
 
 template <int TIE, bool BVH, bool STATS, bool MULTI>
-static int finish_occ(size_t smem, bool nee)
+static int finish_occ(size_t smem, const WfConfig& c)
 {
-    auto k = nee ? wf_finish<TIE, BVH, STATS, MULTI, true> : wf_finish<TIE, BVH, STATS, MULTI, false>;
+    const FinishKernel k = finish_kernel<TIE, BVH, STATS, MULTI>(c);
     smem_attr(k, smem);
     int n = 0;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 128, smem) == cudaSuccess ? n : 0;
@@ -854,16 +868,15 @@ cudaError_t wf_launch_finish(const TraceArgs& a, const WfState& s, const WfConfi
 
 int wf_finish_blocks_per_sm(const WfConfig& c, uint32_t stack_depth)
 {
-    const bool nee = c.has_emitters != 0;
     const size_t smem = wf_finish_smem(c.bvh != 0, stack_depth);
-    if (c.multi) return c.stats ? finish_occ<TIE_STRICT, true, true, true>(smem, nee)
-                                : finish_occ<TIE_STRICT, true, false, true>(smem, nee);
-    if (c.tie == TIE_REFERENCE) return c.stats ? finish_occ<TIE_REFERENCE, false, true, false>(smem, nee)
-                                               : finish_occ<TIE_REFERENCE, false, false, false>(smem, nee);
-    if (c.bvh) return c.stats ? finish_occ<TIE_STRICT, true, true, false>(smem, nee)
-                              : finish_occ<TIE_STRICT, true, false, false>(smem, nee);
-    return c.stats ? finish_occ<TIE_STRICT, false, true, false>(smem, nee)
-                   : finish_occ<TIE_STRICT, false, false, false>(smem, nee);
+    if (c.multi) return c.stats ? finish_occ<TIE_STRICT, true, true, true>(smem, c)
+                                : finish_occ<TIE_STRICT, true, false, true>(smem, c);
+    if (c.tie == TIE_REFERENCE) return c.stats ? finish_occ<TIE_REFERENCE, false, true, false>(smem, c)
+                                               : finish_occ<TIE_REFERENCE, false, false, false>(smem, c);
+    if (c.bvh) return c.stats ? finish_occ<TIE_STRICT, true, true, false>(smem, c)
+                              : finish_occ<TIE_STRICT, true, false, false>(smem, c);
+    return c.stats ? finish_occ<TIE_STRICT, false, true, false>(smem, c)
+                   : finish_occ<TIE_STRICT, false, false, false>(smem, c);
 }
 
 template <int TIE, bool STATS, bool MULTI, int BLOCK>
