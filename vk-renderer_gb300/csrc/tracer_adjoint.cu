@@ -284,8 +284,6 @@ __global__ void __launch_bounds__(128) k_adjoint(TraceArgs a, AdjArgs ga)
         bool on = alive;
         for (uint32_t depth = 0; depth < a.max_depth; ++depth) {
             if (!__any_sync(full, on)) break;
-            Hit h;
-            bool found = false;
             if (on) {
                 if (pass == 1) {
                     if (acc.x < 0.0f || acc.x > 1.0f) { lc[0] = (int)depth; T.x = 0.0f; }
@@ -293,75 +291,58 @@ __global__ void __launch_bounds__(128) k_adjoint(TraceArgs a, AdjArgs ga)
                     if (acc.z < 0.0f || acc.z > 1.0f) { lc[2] = (int)depth; T.z = 0.0f; }
                 }
                 if (pass != 2) acc = vclamp01(acc);
-                h.t = depth_tmax(depth);
-                found = tr.trace(ray, h, false);
             }
-            __syncwarp();
+            const V3 surv = pass != 2 ? splat(1.0f)
+                                      : v3((int)depth >= lc[0] ? 1.0f : 0.0f, (int)depth >= lc[1] ? 1.0f : 0.0f,
+                                           (int)depth >= lc[2] ? 1.0f : 0.0f);
+            const V3 before = acc;
+            Bounce b;
+            int m = -1;
+            V3 dP[3], dN[3], de_da = splat(0.0f);
+            V3 de_dc[3] = {splat(0.0f), splat(0.0f), splat(0.0f)};
+            Hit h0;
+            h0.t = depth_tmax(depth);
+            trace_rays(
+                tr, a, on, false, false, h0, ray, r, b,
+                [&](bool found, const Hit& h) {
+                    bounce_begin(a, on, found, h, ray, surv, acc, mask, r, b);
+                    if (pass != 2 || !b.hit) return;
+                    m = h.kind == 1 ? (int)__float_as_uint(__ldg(a.sc.tri + 3 * (size_t)h.slot).w) : -1;
+                    if (CAM) {
+                        const float nd = dot(b.N, ray.d);
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            const V3 q = dO[j] + dD[j] * h.t;
+                            const float dt = -dot(b.N, q) / nd;
+                            dP[j] = q + ray.d * dt;
+                            dN[j] = h.kind == 2 ? dP[j] / __ldg(a.sc.sph_geo + h.slot).w : splat(0.0f);
+                        }
+                    }
+                },
+                [&](uint32_t si, V3 L, float t, Rng g0) {
+                    V3 c;
+                    if (pass != 2) {
+                        c = nee_value(a, si, b.P, b.N, b.mat, L, t);
+                    } else {  // the direction's two random numbers again, for the derivative
+                        const float rho = rand01(g0), ph = (2.0f * PI) * rand01(g0);
+                        c = nee_grad<CAM>(a, si, b.P, b.N, dP, dN, b.mat, rho, ph, de_da, de_dc);
+                    }
+                    b.e = b.e + c;
+                });
             if (pass != 2) {
                 // the radiance loop; in pass 1 with the sum of what survives the clamps
-                const V3 before = acc;
-                const bool cont = shade_bounce<true, true>(tr, a, on, depth, found, h, ray, acc, mask, r);
+                const bool cont = bounce_end(a, b, depth, ray, acc, mask, r);
                 if (on && pass == 1) T = T + (acc - before);
                 on = on && cont;
                 continue;
             }
             // pass 2: adjoint replay
-            const V3 surv = v3((int)depth >= lc[0] ? 1.0f : 0.0f, (int)depth >= lc[1] ? 1.0f : 0.0f,
-                               (int)depth >= lc[2] ? 1.0f : 0.0f);
+            on = b.hit;
             const V3 w = delta * surv;
-            if (on && !found) {
-                if (a.sky_on) acc = acc + mask * a.sky * surv;
-                on = false;
-            }
-            V3 P, N;
-            Material mat;
-            int m = -1;
-            bool diffuse = false;
-            V3 dP[3], dN[3];
-            float phi = 0.0f, sa = 0.0f, ca = 0.0f;
-            V3 d;
-            if (on) {
-                surface(a.sc, ray, h, P, N, mat);
-                m = h.kind == 1 ? (int)__float_as_uint(__ldg(a.sc.tri + 3 * (size_t)h.slot).w) : -1;
-                if (CAM) {
-                    const float nd = dot(N, ray.d);
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        const V3 q = dO[j] + dD[j] * h.t;
-                        const float dt = -dot(N, q) / nd;
-                        dP[j] = q + ray.d * dt;
-                        dN[j] = h.kind == 2 ? dP[j] / __ldg(a.sc.sph_geo + h.slot).w : splat(0.0f);
-                    }
-                }
-                diffuse = mat.type == MAT_DIFFUSE;
-                if (diffuse) {
-                    const float r2 = rand01(r);
-                    phi = (2.0f * PI) * rand01(r);
-                    sa = sqrtf(r2);
-                    ca = sqrtf(1.0f - r2);
-                    d = jitter(N, phi, sa, ca) * (1.0f - mat.metalness);
-                }
-            }
-            V3 e = splat(0.0f), de_da = splat(0.0f);
-            V3 de_dc[3] = {splat(0.0f), splat(0.0f), splat(0.0f)};
-            for (uint32_t k = 0; k < a.sc.ne; ++k) {
-                if (!__any_sync(full, diffuse)) break;
-                if (diffuse) {
-                    const uint32_t si = __ldg(a.sc.emit + k);
-                    Rng r0 = r;  // the direction's two random numbers again, for the derivative
-                    Hit sh;
-                    const V3 L = nee_ray(a.sc, si, P, r, sh.t);
-                    V3 c = splat(0.0f);
-                    if (!tr.trace(Ray{P, L}, sh, true)) {
-                        const float rho = rand01(r0), ph = (2.0f * PI) * rand01(r0);
-                        c = nee_grad<CAM>(a, si, P, N, dP, dN, mat, rho, ph, de_da, de_dc);
-                    }
-                    e = e + c;
-                }
-                __syncwarp();
-            }
+            const V3 &P = b.P, &N = b.N, &d = b.d, &e = b.e;
+            const Material& mat = b.mat;
             if (!on) continue;
-            if (diffuse) {
+            if (b.diffuse) {
                 const bool emits = mat.emissive.x > 0.0f && mat.emissive.y > 0.0f && mat.emissive.z > 0.0f;
                 const V3 en = emits ? normalize(mat.emissive) : splat(0.0f);
                 const V3 wm = w * mask;
@@ -393,10 +374,10 @@ __global__ void __launch_bounds__(128) k_adjoint(TraceArgs a, AdjArgs ga)
                 const V3 rf = reflect(ray.d, N);
                 if (CAM) {
                     float cphi, sphi;
-                    psincos(phi, sphi, cphi);
+                    psincos(b.phi, sphi, cphi);
 #pragma unroll
                     for (int j = 0; j < 3; ++j) {
-                        const V3 djd = djitter(N, dN[j], cphi, sphi, sa, 0.0f, ca, 0.0f);
+                        const V3 djd = djitter(N, dN[j], cphi, sphi, b.sina, 0.0f, b.cosa, 0.0f);
                         const V3 drf = dreflect(ray.d, dD[j], N, dN[j]);
                         dD[j] = dnorm(rf + d, drf + djd * (1.0f - mat.metalness));
                         dO[j] = dP[j];

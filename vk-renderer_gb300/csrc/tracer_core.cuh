@@ -340,70 +340,60 @@ __device__ __forceinline__ float depth_tmax(uint32_t depth)
     return 3000.0f / (dp1 * dp1);
 }
 
-// The part of one depth iteration of radiance (Tracer.comp:445-549) that
-// follows trace_ray, for a lane that is `on`: sky on a miss, material scatter
-// with next-event estimation, Russian roulette.  Updates acc, mask and ray;
-// returns false when the path ends (miss or roulette) or the lane is off.
-// acc must already be clamped (Tracer.comp:441; the clamp does not affect the
-// trace, so it may run before or after it).  NEE = false leaves out the
-// next-event code for scenes without emissive spheres (its loop would run no
-// iteration there).
-//
-// SYNC (with NEE): every lane of the warp calls this together, and the lanes
-// trace each emitter's shadow ray together.  Called by lanes on their own,
-// the shadow rays of some run while the others wait, or trace something else
-// of the same warp: 3.5 of 32 lanes active in the finishing kernel of a
-// 640x360 frame with two lights, and most issue slots lost to instruction
-// fetches of a kernel with five copies of the traversal.
-template <bool NEE = true, bool SYNC = false, class TR>
-__device__ __forceinline__ bool shade_bounce(TR& tr, const TraceArgs& a, bool on, uint32_t depth, bool found,
-                                             const Hit& h, Ray& ray, V3& acc, V3& mask, Rng& g)
-{
-    const bool hit = on && found;
-    if (on && !found && a.sky_on) acc = acc + mask * a.sky;
-    V3 P, N, d;
+// A path's state in one depth iteration of radiance (Tracer.comp:445-549)
+// between its closest hit and its next ray: the hit's surface and, for a
+// diffuse one, the scatter jitter and the sum of the next-event estimates.
+struct Bounce {
+    V3 P, N, d, e;
     Material mat;
-    bool diffuse = false;
-    if (hit) {
-        surface(a.sc, ray, h, P, N, mat);
-        diffuse = mat.type == MAT_DIFFUSE;
-        if (diffuse) {
+    float phi, sina, cosa;  // of the jitter d
+    bool hit, diffuse;
+};
+
+// The closest hit's part, for a lane that is `on`: sky on a miss (surv: the
+// share of it that counts; 1 but in the adjoint replay), else the surface and
+// the diffuse lobe's random numbers.
+__device__ __forceinline__ void bounce_begin(const TraceArgs& a, bool on, bool found, const Hit& h, const Ray& ray,
+                                             V3 surv, V3& acc, const V3& mask, Rng& g, Bounce& b)
+{
+    b.hit = on && found;
+    b.diffuse = false;
+    b.e = splat(0.0f);
+    if (on && !found && a.sky_on) acc = acc + mask * a.sky * surv;
+    if (b.hit) {
+        surface(a.sc, ray, h, b.P, b.N, b.mat);
+        b.diffuse = b.mat.type == MAT_DIFFUSE;
+        if (b.diffuse) {
             const float r2 = rand01(g);
-            d = jitter(N, (2.0f * PI) * rand01(g), sqrtf(r2), sqrtf(1.0f - r2)) * (1.0f - mat.metalness);
+            b.phi = (2.0f * PI) * rand01(g);
+            b.sina = sqrtf(r2);
+            b.cosa = sqrtf(1.0f - r2);
+            b.d = jitter(b.N, b.phi, b.sina, b.cosa) * (1.0f - b.mat.metalness);
         }
     }
-    V3 e = splat(0.0f);
-    if (NEE) {
-        for (uint32_t k = 0;; ++k) {
-            const bool mine = diffuse && k < a.sc.ne;
-            if (!(SYNC ? __any_sync(0xFFFFFFFFu, mine) : mine)) break;
-            if (mine) {
-                const uint32_t si = __ldg(a.sc.emit + k);
-                Hit sh;
-                const V3 L = nee_ray(a.sc, si, P, g, sh.t);
-                const float t = sh.t;
-                V3 c = splat(0.0f);
-                if (!tr.trace(Ray{P, L}, sh, true)) c = nee_value(a, si, P, N, mat, L, t);
-                e = e + c;
-            }
-            if (SYNC) __syncwarp();
-        }
-    }
-    if (!hit) return false;
-    if (diffuse) {
+}
+
+// After the next-event estimates: material scatter, Russian roulette.  Updates
+// acc, mask and ray; returns false when the path ends or the lane has no hit.
+__device__ __forceinline__ bool bounce_end(const TraceArgs& a, const Bounce& b, uint32_t depth, Ray& ray, V3& acc,
+                                           V3& mask, Rng& g)
+{
+    if (!b.hit) return false;
+    const Material& mat = b.mat;
+    if (b.diffuse) {
         const bool emits = mat.emissive.x > 0.0f && mat.emissive.y > 0.0f && mat.emissive.z > 0.0f;
         const V3 emissive = emits ? normalize(mat.emissive) : splat(0.0f);
-        acc = acc + mask * (emissive + e);
+        acc = acc + mask * (emissive + b.e);
         mask = mask * mat.albedo;
-        ray = Ray{P, normalize(reflect(ray.d, N) + d)};
+        ray = Ray{b.P, normalize(reflect(ray.d, b.N) + b.d)};
     } else if (mat.type == MAT_DIELECTRIC) {
         acc = acc + mat.emissive * mask;
         mask = mask * mat.albedo;
-        const float cosine = -dot(ray.d, N) / length(ray.d);
-        const V3 reflected = reflect(ray.d, N);
-        const V3 refracted = refract(ray.d, N, mat.roughness);
+        const float cosine = -dot(ray.d, b.N) / length(ray.d);
+        const V3 reflected = reflect(ray.d, b.N);
+        const V3 refracted = refract(ray.d, b.N, mat.roughness);
         const float prob = (refracted == splat(0.0f)) ? 1.0f : schlick(cosine, mat.roughness);
-        ray = Ray{P, normalize(rand01(g) < prob ? reflected : refracted)};
+        ray = Ray{b.P, normalize(rand01(g) < prob ? reflected : refracted)};
     }  // other types: the shader's switch has no default; the ray is left as it was
     if (depth >= a.rr_start) {
         const float p = max3(mask);
@@ -411,6 +401,99 @@ __device__ __forceinline__ bool shade_bounce(TR& tr, const TraceArgs& a, bool on
         mask = mask * (1.0f / p);
     }
     return true;
+}
+
+// One depth iteration after its closest hit, for a lane that is `on`.  acc must
+// already be clamped (Tracer.comp:441; the clamp does not affect the trace, so
+// it may run before or after it).  NEE = false leaves out the next-event code
+// for scenes without emissive spheres (its loop would run no iteration there).
+//
+// SYNC (with NEE): every lane of the warp calls this together, and the lanes
+// trace each emitter's shadow ray together.  Called by lanes on their own,
+// the shadow rays of some run while the others wait, or trace something else
+// of the same warp: 3.5 of 32 lanes active in the finishing kernel of a
+// 640x360 frame with two lights.
+template <bool NEE = true, bool SYNC = false, class TR>
+__device__ __forceinline__ bool shade_bounce(TR& tr, const TraceArgs& a, bool on, uint32_t depth, bool found,
+                                             const Hit& h, Ray& ray, V3& acc, V3& mask, Rng& g)
+{
+    Bounce b;
+    bounce_begin(a, on, found, h, ray, splat(1.0f), acc, mask, g, b);
+    if (NEE) {
+#pragma unroll 1
+        for (uint32_t k = 0;; ++k) {
+            const bool mine = b.diffuse && k < a.sc.ne;
+            if (!(SYNC ? __any_sync(0xFFFFFFFFu, mine) : mine)) break;
+            if (mine) {
+                const uint32_t si = __ldg(a.sc.emit + k);
+                Hit sh;
+                const V3 L = nee_ray(a.sc, si, b.P, g, sh.t);
+                const float t = sh.t;
+                V3 c = splat(0.0f);
+                if (!tr.trace(Ray{b.P, L}, sh, true)) c = nee_value(a, si, b.P, b.N, b.mat, L, t);
+                b.e = b.e + c;
+            }
+            if (SYNC) __syncwarp();
+        }
+    }
+    return bounce_end(a, b, depth, ray, acc, mask, g);
+}
+
+// The rays of one depth iteration, traced by a whole warp in one loop: the
+// closest hit, then each emitter's shadow ray, so that the kernel holds one
+// copy of the traversal.  With two, on scenes with lights, the finishing kernel
+// waited 7 of 11 cycles per issue for instructions: a 640x360 frame with two
+// lights took 3.74 ms, with one 2.80.  (k_plain keeps two: it is smaller, at
+// its register limit, and 6 % slower this way.)
+//   given    the lane has its closest hit in h already (found)
+//   first(found, h)            sees the closest hit; fills P, N, mat, diffuse of b
+//   light(si, L, t, g0)        an emitter that the surface sees; g0: the random
+//                              numbers of its direction L are the next two
+template <class TR, class First, class Light>
+__device__ __forceinline__ void trace_rays(TR& tr, const TraceArgs& a, bool on, bool given, bool found, Hit h,
+                                           const Ray& ray, Rng& g, Bounce& b, const First& first, const Light& light)
+{
+    bool go = on;
+    V3 L;
+    float t = 0.0f;
+    uint32_t si = 0;
+    Ray r = ray;
+    Rng g0 = g;
+#pragma unroll 1
+    for (uint32_t k = 0;; ++k) {
+        bool hit = found;
+        if (go && !(given && k == 0)) hit = tr.trace(r, h, k > 0);
+        __syncwarp();
+        if (k == 0)
+            first(hit, h);
+        else if (go && !hit)
+            light(si, L, t, g0);
+        go = b.diffuse && k < a.sc.ne;
+        if (!__any_sync(0xFFFFFFFFu, go)) break;
+        if (go) {
+            si = __ldg(a.sc.emit + k);
+            g0 = g;
+            L = nee_ray(a.sc, si, b.P, g, t);
+            r = Ray{b.P, L};
+            h.t = t;
+        }
+    }
+}
+
+// A whole depth iteration by a whole warp, its rays in trace_rays.
+template <class TR, class F>
+__device__ __forceinline__ bool trace_bounce(TR& tr, const TraceArgs& a, bool on, bool given, bool found0, const Hit& h0,
+                                             uint32_t depth, Ray& ray, V3& acc, V3& mask, Rng& g, const F& first_hit)
+{
+    Bounce b;
+    trace_rays(
+        tr, a, on, given, found0, h0, ray, g, b,
+        [&](bool found, const Hit& h) {
+            if (on) first_hit(found, h);
+            bounce_begin(a, on, found, h, ray, splat(1.0f), acc, mask, g, b);
+        },
+        [&](uint32_t si, V3 L, float t, const Rng&) { b.e = b.e + nee_value(a, si, b.P, b.N, b.mat, L, t); });
+    return bounce_end(a, b, depth, ray, acc, mask, g);
 }
 
 __device__ __forceinline__ unsigned char unorm8(float x)

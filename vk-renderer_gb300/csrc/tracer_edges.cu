@@ -49,16 +49,16 @@ __device__ __forceinline__ Ray primary_ray_at(const TraceArgs& a, float ux, floa
 
 // The pixel (x, y) on both sides of an outline: its forward value for the
 // primary rays r[0] and r[1] (through other image points than the pixel's own
-// sample point) whose closest hits h0[k] are given (found0[k]: it hit): every
-// sample (the pixel's random numbers) through the radiance loop
-// (Tracer.comp:433-553), Reinhard, gamma 1/2.2 and the dither, as
-// resolve_pixel (:578-590).  Every sample starts with the same primary ray, so
-// its hit is traced once, by the caller.  Returns the values' difference,
-// first minus second.  One loop runs both sides' samples bounce after bounce.
+// sample point), r[0] with its closest hit hin: every sample (the pixel's
+// random numbers) through the radiance loop (Tracer.comp:433-553), Reinhard,
+// gamma 1/2.2 and the dither, as resolve_pixel (:578-590).  Every sample starts
+// with the same primary ray, so the hit of r[1] is traced once, in the first
+// sample.  Returns the values' difference, first minus second.  One loop runs
+// both sides' samples bounce after bounce.
 // SYNC: as shade_bounce; lanes that are not `on` take part without a pixel.
 template <bool SYNC, class TR>
 __device__ __forceinline__ V3 pixel_difference(TR& tr, const TraceArgs& a, bool on, uint32_t x, uint32_t y,
-                                               const Ray (&r)[2], const bool (&found0)[2], const Hit (&h0)[2])
+                                               const Ray (&r)[2], const Hit& hin)
 {
     V3 diff = splat(0.0f), accum = splat(0.0f), acc = splat(0.0f), mask = splat(1.0f);
     Rng g;
@@ -66,19 +66,28 @@ __device__ __forceinline__ V3 pixel_difference(TR& tr, const TraceArgs& a, bool 
     uint32_t sample = 0, depth = 0;
     bool second = false;
     Ray ray = r[0];
+    Hit first = hin;  // this side's primary hit
+    bool found0 = true;
     for (;;) {
         if (!(SYNC ? __any_sync(0xFFFFFFFFu, on) : on)) break;
-        Hit h = second ? h0[1] : h0[0];
-        bool found = second ? found0[1] : found0[0];
-        if (on) {
-            acc = vclamp01(acc);
-            if (depth > 0) {
-                h.t = depth_tmax(depth);
-                found = tr.trace(ray, h, false);
+        if (on) acc = vclamp01(acc);
+        const bool given = depth == 0 && !(second && sample == 0);
+        const auto keep = [&](bool found, const Hit& h) {
+            if (depth == 0) {
+                found0 = found;
+                first = h;
             }
+        };
+        Hit h = first;
+        if (!given) h.t = depth_tmax(depth);
+        bool cont;
+        if (SYNC) {
+            cont = trace_bounce(tr, a, on, given, found0, h, depth, ray, acc, mask, g, keep);
+        } else {
+            const bool found = given ? found0 : tr.trace(ray, h, false);
+            keep(found, h);
+            cont = shade_bounce<true, false>(tr, a, on, depth, found, h, ray, acc, mask, g);
         }
-        if (SYNC) __syncwarp();
-        const bool cont = shade_bounce<true, SYNC>(tr, a, on, depth, found, h, ray, acc, mask, g);
         if (!on || (cont && ++depth < a.max_depth)) continue;
         accum = accum + acc;
         depth = 0;
@@ -123,14 +132,7 @@ __device__ __forceinline__ float part_weight(TR& tr, const TraceArgs& a, const E
 {
     const float4 dl = __ldg(e.dldi + (size_t)py * a.width + px);
     const Ray r[2] = {primary_ray_at(a, ix, iy), primary_ray_at(a, ox, oy)};
-    Hit h0[2] = {hin, hin};
-    bool found0[2] = {true, false};
-    if (on) {
-        h0[1].t = depth_tmax(0);
-        found0[1] = tr.trace(r[1], h0[1], false);
-    }
-    if (SYNC) __syncwarp();
-    const V3 d = pixel_difference<SYNC>(tr, a, on, px, py, r, found0, h0);
+    const V3 d = pixel_difference<SYNC>(tr, a, on, px, py, r, hin);
     return dl.x * d.x + dl.y * d.y + dl.z * d.z;
 }
 

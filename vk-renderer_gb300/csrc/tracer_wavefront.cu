@@ -601,27 +601,19 @@ __device__ __forceinline__ void store_path(const WfState& s, uint32_t pid, const
     s.prim0[pid] = p.prim0;
 }
 
-// The rest of one depth iteration after its closest hit h (Tracer.comp:441-549:
-// clamp, sky, scatter, next-event estimation, Russian roulette), then the
-// sample and pixel bookkeeping (:578-592): the next depth, else the pixel's
-// next sample (its RNG continues where the last sample stopped), else the
-// resolve.  Returns true while the pixel has another ray to trace: p.ray, with
-// tmax depth_tmax(p.depth).  NEE: as shade_bounce, every lane of the warp
-// calling this together, those with a path being on.
-template <bool NEE, class TR>
-__device__ __forceinline__ bool advance_path(TR& tr, const TraceArgs& A, bool on, uint32_t x, uint32_t y, const Hit& h,
-                                             PathRegs& p)
+// The pixel's primary hit, for the primary-hit image.
+__device__ __forceinline__ void note_primary(PathRegs& p, bool found, const Hit& h)
 {
-    const bool found = on && h.kind != 0;
-    if (on) {
-        if (p.sample == 0 && p.depth == 0) {
-            p.prim0 = found ? h.prim : NO_PRIM;
-            p.t0 = found ? h.t : -1.0f;
-        }
-        p.acc = vclamp01(p.acc);
+    if (p.sample == 0 && p.depth == 0) {
+        p.prim0 = found ? h.prim : NO_PRIM;
+        p.t0 = found ? h.t : -1.0f;
     }
-    const bool cont = shade_bounce<NEE, NEE>(tr, A, on, p.depth, found, h, p.ray, p.acc, p.mask, p.g);
-    if (!on) return false;
+}
+
+// After a bounce (cont: its path goes on): the next depth, else the pixel's
+// next sample, else the resolve.  Returns true while the pixel has a ray.
+__device__ __forceinline__ bool next_ray(const TraceArgs& A, uint32_t x, uint32_t y, bool cont, PathRegs& p)
+{
     p.depth++;
     if (cont && p.depth < A.max_depth) return true;
     p.accum = p.accum + p.acc;
@@ -635,6 +627,26 @@ __device__ __forceinline__ bool advance_path(TR& tr, const TraceArgs& A, bool on
     }
     resolve_pixel(A, x, y, p.accum, p.g, p.prim0, p.t0);
     return false;
+}
+
+// The rest of one depth iteration after its closest hit h (Tracer.comp:441-549:
+// clamp, sky, scatter, next-event estimation, Russian roulette), then the
+// sample and pixel bookkeeping (:578-592): the next depth, else the pixel's
+// next sample (its RNG continues where the last sample stopped), else the
+// resolve.  Returns true while the pixel has another ray to trace: p.ray, with
+// tmax depth_tmax(p.depth).  NEE: as shade_bounce, every lane of the warp
+// calling this together, those with a path being on.
+template <bool NEE, class TR>
+__device__ __forceinline__ bool advance_path(TR& tr, const TraceArgs& A, bool on, uint32_t x, uint32_t y, const Hit& h,
+                                             PathRegs& p)
+{
+    const bool found = on && h.kind != 0;
+    if (on) {
+        note_primary(p, found, h);
+        p.acc = vclamp01(p.acc);
+    }
+    const bool cont = shade_bounce<NEE, NEE>(tr, A, on, p.depth, found, h, p.ray, p.acc, p.mask, p.g);
+    return on && next_ray(A, x, y, cont, p);
 }
 
 // ------------------------------------------------------------------- shade --
@@ -724,12 +736,19 @@ __global__ void __launch_bounds__(128) wf_finish(TraceArgs a, WfState s, int qse
         const TraceArgs& A = SCENE_ARGS(MULTI, a, slots, scene);
         PathTracer<TIE, BVH, STATS, W8> tr(A.sc, stk, cnt, a.status, A.trav_limit);
         Hit h;
-        if (on) {
-            h.t = depth_tmax(ps.depth);
-            tr.trace(ps.ray, h, false);
+        h.t = on ? depth_tmax(ps.depth) : 0.0f;
+        bool again;
+        if (NEE) {
+            if (on) ps.acc = vclamp01(ps.acc);
+            const bool cont = trace_bounce(tr, A, on, false, false, h, ps.depth, ps.ray, ps.acc, ps.mask, ps.g,
+                                           [&](bool found, const Hit& first) { note_primary(ps, found, first); });
+            again = on && next_ray(A, x, y, cont, ps);
+        } else {
+            if (on) tr.trace(ps.ray, h, false);
+            __syncwarp();
+            again = advance_path<false>(tr, A, on, x, y, h, ps);
         }
-        __syncwarp();
-        if (!advance_path<NEE>(tr, A, on, x, y, h, ps) && on) {
+        if (on && !again) {
             qi = n > threads ? threads + atomicAdd(&s.count[2], 1u) : n;
             take();
         }
