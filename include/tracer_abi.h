@@ -175,7 +175,11 @@ typedef struct tracer_scene_desc {
 
 #define TRACER_KERNEL_AUTO 0      /* WAVEFRONT for BVH scenes with >= 2^16 pixel x spp x depth when the
                                      scene has an 8-wide BVH (and bvh_width is 0 or 8), >= 2^22 otherwise;
-                                     else PLAIN (tracer_trace_adjoint: WAVEFRONT wherever it applies) */
+                                     else PLAIN (tracer_trace_adjoint: WAVEFRONT wherever it applies).
+                                     PLAIN too at any size on scenes that it traces faster (with spheres,
+                                     or triangle-only ones of short rays), unless the call sets bvh_width,
+                                     tail_paths, wavefront, block or stack_depth, collects statistics or is
+                                     profiled; the images are the same */
 #define TRACER_KERNEL_PLAIN 1     /* one thread per pixel, nested sample/bounce loops */
 #define TRACER_KERNEL_WAVEFRONT 2 /* persistent extend kernel + shade kernel over path queues */
 
@@ -343,7 +347,8 @@ int tracer_readback_scene(tracer_ctx* ctx, uint32_t scene, int aov, void* host_d
 
 /* Per-kernel GPU time of the last trace, measured with CUDA events when
  * profiling is on (off by default; the reference has only an FPS counter,
- * Source/Main.cpp:152-163). */
+ * Source/Main.cpp:152-163).  While it is on, TRACER_KERNEL_AUTO keeps to the
+ * wavefront's stages on scenes where the plain kernel is the faster one. */
 typedef struct tracer_timings {
     float total_ms;     /* whole trace */
     float extend_ms;    /* wavefront: sum over rounds of the extend (traversal) kernel */

@@ -304,6 +304,20 @@ cudaEvent_t prof_event(tracer_ctx* c, size_t i)
 constexpr double kCheapRays = 20.0;
 bool cheap_rays(double cost) { return cost > 0.0 && cost <= kCheapRays; }
 
+// BVH scenes whose frames the plain kernel traces faster than the wavefront at
+// every size (its stages and path state cost more than they gain): scenes with
+// spheres, and triangle-only ones of short rays (kCheapRays; above, rounds win
+// on large frames: soup of 30k 2.74 / 2.39 ms).  Plain / wavefront as this line
+// was drawn, 1280x720 x 4 spp x depth 6, ms: height field of 20k triangles
+// 0.86 / 1.07, of 200k 1.67 / 1.81, soup of 10k 1.13 / 1.12; 20k triangles and
+// 30 spheres 3.48 / 5.13, 12k and 200 with 2 lights 14.2 / 21.3, 60k and 200
+// with 2 lights 33.4 / 44.1; 40 spheres 0.26 / 0.60, 2000 3.02 / 3.28.
+bool plain_suits(const SceneBuffers& s)
+{
+    if (s.cw8) return cheap_rays(s.cw8_cost);
+    return s.nt == 0 || s.tri_cw8.p;
+}
+
 // Launches the wavefront: generate, then rounds of extend + shade until the
 // path queue is empty (read back a few rounds behind the launches) or
 // max_rounds is reached (no path needs more than spp * max_depth rounds).
@@ -847,21 +861,20 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
         return fail(c, TRACER_ERR_INVALID_ARG, "unknown tie mode %d", p->tie_mode);
     if (p->tie_mode == TRACER_TIES_REFERENCE && c->scene.bvh)
         return fail(c, TRACER_ERR_INVALID_ARG, "reference ties depend on scan order and need a linear-scan scene");
-    // AUTO: the wavefront on BVH scenes with enough path bounces in flight --
-    // from 2^16 where the scene has an 8-wide BVH (its traversal, in the
-    // extend and finishing kernels, wins even on small frames), from 2^22
-    // otherwise; the plain kernel on linear-scan scenes and small frames.
-    // Measured (plain / wavefront ms), 8-wide: c3 scene 128^2 x 4 spp x
-    // depth 4 (2^18 bounces) 0.48 / 0.30, 256^2 x 4 x 4 0.59 / 0.38, 512^2
-    // 1.42 / 0.91; c1 scene 128^2 x 4 x 8 2.63 / 1.63, 256^2 x 4 x 8 2.95 /
-    // 1.83, 640x360 x 4 x 8 8.06 / 3.08, 1920x1080 x 16 x 8 222 / 58; c4
-    // scene 256^2 x 4 x 12 6.22 / 3.80.  Binary only: c0 (spheres) 512^2 x 1
-    // x 2 0.067 / 0.118; the reference's own 10-primitive frame (linear) 1.6
-    // / 2.2.
+    // AUTO: the plain kernel on linear-scan scenes, small frames and scenes that
+    // it traces faster (plain_suits); else the wavefront, from 2^16 path bounces
+    // where the scene has an 8-wide BVH, from 2^22 otherwise (c1 scene, plain /
+    // wavefront ms: 256^2 x 4 spp x depth 8 2.95 / 1.83, 640x360 x 4 x 8 8.06 /
+    // 3.08, 1920x1080 x 16 x 8 222 / 58).  A call that asks for something of the
+    // wavefront, for statistics or, with profiling on, for its stages' times
+    // keeps the rule on bounces.
     const uint64_t bounces = (uint64_t)p->width * p->height * p->spp * p->max_depth;
     const bool cw8_auto = c->scene.cw8 && (p->bvh_width == 0 || p->bvh_width == 8);
+    const bool asked = p->bvh_width || p->tail_paths || p->wavefront || p->block || p->stack_depth || p->stats ||
+                       c->profiling || (p->aov_mask & (1u << TRACER_AOV_STATS));
     const int kernel = p->kernel != TRACER_KERNEL_AUTO ? p->kernel
-                       : (c->scene.bvh && bounces >= (cw8_auto ? (1ull << 16) : (1ull << 22)))
+                       : (c->scene.bvh && bounces >= (cw8_auto ? (1ull << 16) : (1ull << 22)) &&
+                          (asked || !plain_suits(c->scene)))
                            ? TRACER_KERNEL_WAVEFRONT
                            : TRACER_KERNEL_PLAIN;
     if (kernel != TRACER_KERNEL_PLAIN && kernel != TRACER_KERNEL_WAVEFRONT)
@@ -940,7 +953,8 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
     if (c->profiling) cudaEventRecord(c->prof_begin, st);
 
     if (kernel == TRACER_KERNEL_PLAIN) {
-        LaunchConfig lc{block, stats, p->tie_mode, s.bvh ? 1 : 0};
+        LaunchConfig lc{block, stats, p->tie_mode, s.bvh ? 1 : 0, s.cw8 ? 1 : 0, (uint32_t)c->sm_count};
+        if (s.cw8 && !stats) a.stack_depth = std::max(1u, s.cw8_depth);  // all that its triangles-only form pushes to
         e = launch_plain(a, lc, st);
         c->last_launches = 1;
     } else {
@@ -1267,20 +1281,20 @@ extern "C" int tracer_trace_noalloc(tracer_ctx* c, const tracer_frame* f, const 
     // The status word starts at zero; the generate kernel resets the queue
     // counters; statistics are not collected here.
     cudaError_t e = cudaMemsetAsync(a.status, 0, sizeof(int), st);
-    if (e == cudaSuccess) e = wf_launch_generate(a, ws, wc, st);
     // No queue length is read back to the host.  With fewer pixels than the
     // point below which tracer_trace runs no round (tail_paths, or with the
     // automatic threshold the extend kernel's resident threads -- always the
-    // case here, the image being at most TRACER_NOALLOC_MAX_PIXELS), the
-    // finishing kernel traces every pixel in one launch; otherwise every round
-    // is launched, and a round with an empty queue returns at once.
+    // case here, the image being at most TRACER_NOALLOC_MAX_PIXELS), the plain
+    // kernel traces every pixel in one launch (320x180 x 4 spp: soup of 500
+    // triangles 64 us, generate and finishing kernel 73; of 30k 471, 461);
+    // otherwise every round is launched, and a round with an empty queue
+    // returns at once.
     const uint32_t no_rounds_below = p->tail_paths ? p->tail_paths : wc.extend_grid * wc.block;
-    const int fin_per = npx < no_rounds_below ? wf_finish_blocks_per_sm(wc, stack) : 0;
-    if (fin_per > 0) {
-        const size_t blocks = (npx + 127) / 128, cap = (size_t)fin_per * c->sm_count;
-        wc.finish_grid = (uint32_t)(blocks < cap ? blocks : cap);
-        if (e == cudaSuccess) e = wf_launch_finish(a, ws, wc, 0, st);
+    if (npx < no_rounds_below) {
+        LaunchConfig lc{128, 0, p->tie_mode, s.bvh ? 1 : 0, wc.finish_w8 ? 1 : 0, (uint32_t)c->sm_count};
+        if (e == cudaSuccess) e = launch_plain(a, lc, st);
     } else {
+        if (e == cudaSuccess) e = wf_launch_generate(a, ws, wc, st);
         const uint32_t rounds = p->spp * p->max_depth + 1;
         for (uint32_t k = 0; k < rounds && e == cudaSuccess; ++k) {
             e = wf_launch_extend(a, ws, wc, (int)(k & 1), st);
@@ -1656,7 +1670,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
     if (c->profiling) cudaEventRecord(c->prof_begin, st);
 
     if (kernel == TRACER_KERNEL_PLAIN) {
-        LaunchConfig lc{block, stats, TRACER_TIES_STRICT, 1};
+        LaunchConfig lc{block, stats, TRACER_TIES_STRICT, 1, 0, (uint32_t)c->sm_count};
         for (uint32_t k = 0; k < n && e == cudaSuccess; ++k) {
             e = launch_plain(slots[k], lc, st);
             c->last_launches++;

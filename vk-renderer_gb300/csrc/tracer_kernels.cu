@@ -16,11 +16,11 @@ namespace vkt {
 
 // With statistics, the canonical traversal (its node visiting order is the
 // oracle's); without, the path kernels' faster one, which finds the same hits.
-template <int TIE, bool BVH, bool STATS>
-using PlainTracer = std::conditional_t<STATS, Tracer<TIE, BVH, STATS>, PathTracer<TIE, BVH, STATS>>;
+template <int TIE, bool BVH, bool STATS, bool W8>
+using PlainTracer = std::conditional_t<STATS, Tracer<TIE, BVH, STATS>, PathTracer<TIE, BVH, STATS, W8>>;
 
-template <int TIE, bool BVH, bool STATS>
-__device__ __forceinline__ PlainTracer<TIE, BVH, STATS> plain_tracer(const TraceArgs& a, int* smem, Counters& cnt)
+template <int TIE, bool BVH, bool STATS, bool W8>
+__device__ __forceinline__ PlainTracer<TIE, BVH, STATS, W8> plain_tracer(const TraceArgs& a, int* smem, Counters& cnt)
 {
     if constexpr (STATS) {
         const int n = blockDim.x, tid = threadIdx.x;
@@ -28,7 +28,7 @@ __device__ __forceinline__ PlainTracer<TIE, BVH, STATS> plain_tracer(const Trace
             a.sc, Stack{smem + tid, reinterpret_cast<float*>(smem + (size_t)a.stack_depth * n) + tid, n, (int)a.stack_depth},
             cnt, a.status, a.trav_limit};
     } else {
-        return PathTracer<TIE, BVH, STATS>(a.sc, thread_stack(smem, a.stack_depth), cnt, a.status, a.trav_limit);
+        return PathTracer<TIE, BVH, STATS, W8>(a.sc, thread_stack(smem, a.stack_depth), cnt, a.status, a.trav_limit);
     }
 }
 
@@ -36,11 +36,16 @@ __device__ __forceinline__ PlainTracer<TIE, BVH, STATS> plain_tracer(const Trace
 // closest hit, then the lanes shade together (shadow rays too).  All lanes
 // finish a sample before any starts the next, so that primary rays, the
 // coherent ones, are traced together (the reference's frame: 1.56 ms against
-// 1.76 for lanes that go straight on).  Linear scans are bound by issue and
-// instruction fetches at low occupancy: 64 registers, 1.56 ms against 1.63 at
-// 80 and 1.91 at 105.  With BVHs 80 registers: c0's frame 49 us, 54 at 128.
-template <int TIE, bool BVH, bool STATS>
-__global__ void __launch_bounds__(256, BVH ? 3 : 4) k_plain(TraceArgs a)
+// 1.76 for lanes that go straight on).
+//
+// Bound by issue and instruction fetches, so a kernel holds only what its
+// scenes need: no next-event code without lights (NEE; 1280x720 x 4 spp of 20k
+// triangles, 30 spheres: 3.42 ms, 3.70 with it), no binary traversal on
+// triangle-only scenes (W8), and with BVHs and lights one copy of the
+// traversal (trace_rays: 12k triangles, 200 spheres, 2 lights: 14.2 ms, 29.1
+// with two).
+template <int TIE, bool BVH, bool STATS, bool NEE, bool W8, int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS) k_plain(TraceArgs a)
 {
     extern __shared__ int smem[];
     const int tid = threadIdx.x;
@@ -48,7 +53,7 @@ __global__ void __launch_bounds__(256, BVH ? 3 : 4) k_plain(TraceArgs a)
     Counters cnt;
 #pragma unroll
     for (int k = 0; k < C_COUNT; ++k) cnt.c[k] = 0;
-    PlainTracer<TIE, BVH, STATS> tr = plain_tracer<TIE, BVH, STATS>(a, smem, cnt);
+    PlainTracer<TIE, BVH, STATS, W8> tr = plain_tracer<TIE, BVH, STATS, W8>(a, smem, cnt);
     const uint32_t x = blockIdx.x * 16 + (tid & 15);
     const uint32_t y = blockIdx.y * (nthreads >> 4) + (tid >> 4);
     bool alive = x < a.width && y < a.height;
@@ -66,19 +71,26 @@ __global__ void __launch_bounds__(256, BVH ? 3 : 4) k_plain(TraceArgs a)
         mask = splat(1.0f);
         for (depth = 0; depth < a.max_depth; ++depth) {
             if (!__any_sync(0xFFFFFFFFu, on)) break;
-            Hit h;
-            bool found = false;
-            if (on) {
-                acc = vclamp01(acc);
-                h.t = depth_tmax(depth);
-                found = tr.trace(ray, h, false);
+            const auto primary = [&](bool found, const Hit& h) {
                 if (sample == 0 && depth == 0) {
                     prim0 = found ? h.prim : NO_PRIM;
                     t0 = found ? h.t : -1.0f;
                 }
+            };
+            Hit h;
+            h.t = depth_tmax(depth);
+            if (on) acc = vclamp01(acc);
+            if (BVH && NEE) {
+                on = trace_bounce(tr, a, on, false, false, h, depth, ray, acc, mask, g, primary);
+            } else {
+                bool found = false;
+                if (on) {
+                    found = tr.trace(ray, h, false);
+                    primary(found, h);
+                }
+                __syncwarp();
+                on = shade_bounce<NEE, NEE>(tr, a, on, depth, found, h, ray, acc, mask, g);
             }
-            __syncwarp();
-            on = shade_bounce<true, true>(tr, a, on, depth, found, h, ray, acc, mask, g);
         }
         accum = accum + acc;
     }
@@ -86,21 +98,44 @@ __global__ void __launch_bounds__(256, BVH ? 3 : 4) k_plain(TraceArgs a)
     if (STATS) flush_counters(a, cnt);
 }
 
-template <int TIE, bool BVH, bool STATS>
-static cudaError_t launch_t(const TraceArgs& a, const LaunchConfig& lc, cudaStream_t s)
+template <int TIE, bool BVH, bool STATS, bool NEE, bool W8, int BLOCKS>
+static cudaError_t launch_k(const TraceArgs& a, const LaunchConfig& lc, cudaStream_t s)
 {
     const size_t smem = (size_t)a.stack_depth * lc.block * 8;
-    auto k = k_plain<TIE, BVH, STATS>;
+    auto k = k_plain<TIE, BVH, STATS, NEE, W8, BLOCKS>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     dim3 grid((a.width + 15) / 16, (a.height + (lc.block / 16) - 1) / (lc.block / 16));
     k<<<grid, lc.block, smem, s>>>(a);
     return cudaGetLastError();
 }
 
+// The register budget, as resident blocks of 256.  Frames that fit two such
+// blocks per SM have no use for a third: 104-127 registers with BVHs, where a
+// soup of 10k triangles at 320x180 x 4 spp took 225 us (232 at three blocks,
+// 247 at four), a lit scene of 12.7k primitives 2.79 ms (3.09, 3.16); linear
+// scans three, the reference's scene at that size 215 us (229 at four).
+// Larger ones: four, three on triangle-only scenes (1280x720 x 4 spp, three /
+// four: height field of 20k triangles 0.86 / 0.90 ms; 64 spheres 1.23 / 1.11,
+// the lit scene 15.3 / 14.2).
+template <int TIE, bool BVH, bool NEE, bool W8>
+static cudaError_t launch_sized(const TraceArgs& a, const LaunchConfig& lc, cudaStream_t s)
+{
+    constexpr int kSmall = BVH ? 2 : NEE ? 3 : 4, kLarge = W8 ? 3 : 4;
+    if ((uint64_t)a.width * a.height <= 512ull * lc.sms) return launch_k<TIE, BVH, false, NEE, W8, kSmall>(a, lc, s);
+    return launch_k<TIE, BVH, false, NEE, W8, kLarge>(a, lc, s);
+}
+
 template <int TIE, bool BVH>
 static cudaError_t launch_s(const TraceArgs& a, const LaunchConfig& lc, cudaStream_t s)
 {
-    return lc.stats ? launch_t<TIE, BVH, true>(a, lc, s) : launch_t<TIE, BVH, false>(a, lc, s);
+    constexpr int kStats = BVH ? 3 : 4;
+    if (lc.stats)
+        return a.sc.ne ? launch_k<TIE, BVH, true, true, false, kStats>(a, lc, s)
+                       : launch_k<TIE, BVH, true, false, false, kStats>(a, lc, s);
+    if (a.sc.ne) return launch_sized<TIE, BVH, true, false>(a, lc, s);
+    if constexpr (BVH)
+        if (lc.w8) return launch_sized<TIE, BVH, false, true>(a, lc, s);
+    return launch_sized<TIE, BVH, false, false>(a, lc, s);
 }
 
 // Reads n 16-byte words `passes` times with loads that are cached in L2 only

@@ -16,6 +16,8 @@ struct LaunchConfig {
     int stats;
     int tie;
     int bvh;
+    int w8;        // the scene's triangles have an 8-wide BVH and it has no spheres
+    uint32_t sms;  // of the device
 };
 
 cudaError_t launch_plain(const TraceArgs& a, const LaunchConfig& lc, cudaStream_t s);
