@@ -36,7 +36,12 @@ __device__ __forceinline__ PlainTracer<TIE, BVH, STATS, W8> plain_tracer(const T
 // closest hit, then the lanes shade together (shadow rays too).  All lanes
 // finish a sample before any starts the next, so that primary rays, the
 // coherent ones, are traced together (the reference's frame: 1.56 ms against
-// 1.76 for lanes that go straight on).
+// 1.76 for lanes that go straight on).  Every sample of a pixel starts with
+// the same ray (no jitter, Tracer.comp:568-574), so its hit is found once (not
+// with statistics, which count the reference's rays): 1280x720 x 4 spp, soup of
+// 10k triangles 1.15 -> 0.64 ms, height field of 200k 1.65 -> 1.31, 20k
+// triangles and 30 spheres 3.52 -> 2.65, lit scene of 12k 14.3 -> 13.4; 1 to 3 %
+// slower at 1 spp, by registers.
 //
 // Bound by issue and instruction fetches, so a kernel holds only what its
 // scenes need: no next-event code without lights (NEE; 1280x720 x 4 spp of 20k
@@ -63,7 +68,9 @@ __global__ void __launch_bounds__(256, BLOCKS) k_plain(TraceArgs a)
     Ray ray = pr;
     V3 accum = splat(0.0f), acc = splat(0.0f), mask = splat(1.0f);
     uint32_t prim0 = NO_PRIM, sample = 0, depth = 0;
-    float t0 = -1.0f;
+    float t0 = -1.0f;  // with prim0, kind0, slot0: the primary hit
+    int kind0 = 0;
+    uint32_t slot0 = 0;
     for (; sample < a.spp; ++sample) {
         bool on = alive;
         ray = pr;
@@ -71,20 +78,23 @@ __global__ void __launch_bounds__(256, BLOCKS) k_plain(TraceArgs a)
         mask = splat(1.0f);
         for (depth = 0; depth < a.max_depth; ++depth) {
             if (!__any_sync(0xFFFFFFFFu, on)) break;
+            // the primary ray is the same in every sample: traced once
+            const bool given = !STATS && sample > 0 && depth == 0;
             const auto primary = [&](bool found, const Hit& h) {
                 if (sample == 0 && depth == 0) {
                     prim0 = found ? h.prim : NO_PRIM;
                     t0 = found ? h.t : -1.0f;
+                    kind0 = h.kind;
+                    slot0 = h.slot;
                 }
             };
-            Hit h;
-            h.t = depth_tmax(depth);
+            Hit h{given ? t0 : depth_tmax(depth), prim0, kind0, slot0};
             if (on) acc = vclamp01(acc);
             if (BVH && NEE) {
-                on = trace_bounce(tr, a, on, false, false, h, depth, ray, acc, mask, g, primary);
+                on = trace_bounce(tr, a, on, given, kind0 != 0, h, depth, ray, acc, mask, g, primary);
             } else {
-                bool found = false;
-                if (on) {
+                bool found = kind0 != 0;
+                if (on && !given) {
                     found = tr.trace(ray, h, false);
                     primary(found, h);
                 }
@@ -113,14 +123,14 @@ static cudaError_t launch_k(const TraceArgs& a, const LaunchConfig& lc, cudaStre
 // blocks per SM have no use for a third: 104-127 registers with BVHs, where a
 // soup of 10k triangles at 320x180 x 4 spp took 225 us (232 at three blocks,
 // 247 at four), a lit scene of 12.7k primitives 2.79 ms (3.09, 3.16); linear
-// scans three, the reference's scene at that size 215 us (229 at four).
+// scans with lights too, the reference's scene at that size 206 us (229 at four).
 // Larger ones: four, three on triangle-only scenes (1280x720 x 4 spp, three /
 // four: height field of 20k triangles 0.86 / 0.90 ms; 64 spheres 1.23 / 1.11,
 // the lit scene 15.3 / 14.2).
 template <int TIE, bool BVH, bool NEE, bool W8>
 static cudaError_t launch_sized(const TraceArgs& a, const LaunchConfig& lc, cudaStream_t s)
 {
-    constexpr int kSmall = BVH ? 2 : NEE ? 3 : 4, kLarge = W8 ? 3 : 4;
+    constexpr int kSmall = BVH || NEE ? 2 : 4, kLarge = W8 ? 3 : 4;
     if ((uint64_t)a.width * a.height <= 512ull * lc.sms) return launch_k<TIE, BVH, false, NEE, W8, kSmall>(a, lc, s);
     return launch_k<TIE, BVH, false, NEE, W8, kLarge>(a, lc, s);
 }
