@@ -126,7 +126,7 @@ struct tracer_ctx {
     uint32_t last_mask = 0;
     // wavefront path state (scratch, one slot per pixel)
     DevBuf<float4> wf_ray_o, wf_ray_d, wf_acc, wf_mask, wf_accum;
-    DevBuf<uint4> wf_hit;
+    DevBuf<uint4> wf_hit, wf_hit0;
     DevBuf<uint32_t> wf_prim0, wf_q0, wf_q1, wf_count, wf_scene;
     uint32_t* pinned_counts = nullptr;  // lagged queue lengths read by the launch loop
     std::vector<cudaEvent_t> count_events;
@@ -262,6 +262,7 @@ void release_wavefront(tracer_ctx* c)
     c->wf_mask.release();
     c->wf_accum.release();
     c->wf_hit.release();
+    c->wf_hit0.release();
     c->wf_prim0.release();
     c->wf_q0.release();
     c->wf_q1.release();
@@ -276,6 +277,7 @@ cudaError_t ensure_wavefront(tracer_ctx* c, size_t npx)
     if (e == cudaSuccess) e = dalloc(c->wf_mask, npx);
     if (e == cudaSuccess) e = dalloc(c->wf_accum, npx);
     if (e == cudaSuccess) e = dalloc(c->wf_hit, npx);
+    if (e == cudaSuccess) e = dalloc(c->wf_hit0, npx);
     if (e == cudaSuccess) e = dalloc(c->wf_prim0, npx);
     if (e == cudaSuccess) e = dalloc(c->wf_q0, npx);
     if (e == cudaSuccess) e = dalloc(c->wf_q1, npx);
@@ -342,7 +344,7 @@ int run_wavefront(tracer_ctx* c, const TraceArgs& a, WfConfig& wc, size_t nslots
                   const AdjWf* adj = nullptr)
 {
     WfState ws{c->wf_ray_o.p, c->wf_ray_d.p, c->wf_hit.p, c->wf_acc.p, c->wf_mask.p, c->wf_accum.p,
-               c->wf_prim0.p, {c->wf_q0.p, c->wf_q1.p}, c->wf_count.p, c->wf_scene.p};
+               c->wf_prim0.p, {c->wf_q0.p, c->wf_q1.p}, c->wf_count.p, wc.stats ? nullptr : c->wf_hit0.p, c->wf_scene.p};
     int per = wf_extend_blocks_per_sm(wc, stack);
     if (per <= 0) return fail(c, TRACER_ERR_INVALID_ARG, "extend kernel cannot be resident (stack %u)", stack);
     if (wavefront && (int)wavefront < per) per = (int)wavefront;
@@ -1155,7 +1157,8 @@ constexpr size_t kNaOffHit = kNaOffRayD + kNaF4;
 constexpr size_t kNaOffAcc = kNaOffHit + kNaF4;
 constexpr size_t kNaOffMask = kNaOffAcc + kNaF4;
 constexpr size_t kNaOffAccum = kNaOffMask + kNaF4;
-constexpr size_t kNaOffPrim0 = kNaOffAccum + kNaF4;
+constexpr size_t kNaOffHit0 = kNaOffAccum + kNaF4;
+constexpr size_t kNaOffPrim0 = kNaOffHit0 + kNaF4;
 constexpr size_t kNaOffQ0 = kNaOffPrim0 + kNaU32;
 constexpr size_t kNaOffQ1 = kNaOffQ0 + kNaU32;
 constexpr size_t kNaOffCount = kNaOffQ1 + kNaU32;     // 4 x u32
@@ -1261,7 +1264,8 @@ extern "C" int tracer_trace_noalloc(tracer_ctx* c, const tracer_frame* f, const 
                reinterpret_cast<float4*>(base + kNaOffMask), reinterpret_cast<float4*>(base + kNaOffAccum),
                reinterpret_cast<uint32_t*>(base + kNaOffPrim0),
                {reinterpret_cast<uint32_t*>(base + kNaOffQ0), reinterpret_cast<uint32_t*>(base + kNaOffQ1)},
-               reinterpret_cast<uint32_t*>(base + kNaOffCount), nullptr};
+               reinterpret_cast<uint32_t*>(base + kNaOffCount), reinterpret_cast<uint4*>(base + kNaOffHit0),
+               nullptr};
     WfConfig wc;
     std::memset(&wc, 0, sizeof wc);
     wc.tie = p->tie_mode;
@@ -1702,7 +1706,8 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
             if (r != TRACER_OK) return r;
         } else {
             WfState ws{c->wf_ray_o.p, c->wf_ray_d.p, c->wf_hit.p, c->wf_acc.p, c->wf_mask.p, c->wf_accum.p,
-                       c->wf_prim0.p, {c->wf_q0.p, c->wf_q1.p}, c->wf_count.p, c->wf_scene.p};
+                       c->wf_prim0.p, {c->wf_q0.p, c->wf_q1.p}, c->wf_count.p, wc.stats ? nullptr : c->wf_hit0.p,
+                       c->wf_scene.p};
             int per = wf_extend_blocks_per_sm(wc, stack);
             if (per <= 0) return fail(c, TRACER_ERR_INVALID_ARG, "extend kernel cannot be resident");
             if (p0.wavefront && (int)p0.wavefront < per) per = (int)p0.wavefront;
@@ -1712,7 +1717,8 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
             // the graph bakes in sizes, launch shapes and buffer addresses
             std::vector<uint64_t> key = {n, total, max_rounds, block, stack, (uint64_t)stats, wc.extend_grid,
                                          (uint64_t)wide, (uint64_t)binary_asked(&p0), (uint64_t)cheap, p0.tail_paths,
-                                         (uint64_t)(uintptr_t)c->wf_ray_o.p, (uint64_t)(uintptr_t)c->batch_slots.p,
+                                         (uint64_t)(uintptr_t)c->wf_ray_o.p, (uint64_t)(uintptr_t)c->wf_hit0.p,
+                                         (uint64_t)(uintptr_t)c->batch_slots.p,
                                          (uint64_t)(uintptr_t)c->b_rgba8.p, (uint64_t)(uintptr_t)c->b_rgba32f.p,
                                          (uint64_t)(uintptr_t)c->b_hit.p, mask};
             if (key != c->graph_key || !c->graph_exec) {

@@ -604,20 +604,6 @@ __device__ __forceinline__ bool adj_replay_bounce(TR& tr, const TraceArgs& a, co
     return cont && p.depth < a.max_depth;
 }
 
-__device__ __forceinline__ uint4 hit_pack(const Hit& h)
-{
-    return make_uint4(__float_as_uint(h.t), h.prim, h.slot, (uint32_t)h.kind);
-}
-__device__ __forceinline__ Hit hit_unpack(uint4 v)
-{
-    Hit h;
-    h.t = __uint_as_float(v.x);
-    h.prim = v.y;
-    h.slot = v.z;
-    h.kind = (int)v.w;
-    return h;
-}
-
 // One bounce of whichever pass the path is in, given the closest hit h of
 // its ray, then the bookkeeping: pass 1 ends -> pass 2 of the same sample
 // from the sample's first ray and RNG state; pass 2 ends -> the next sample
@@ -698,13 +684,7 @@ __global__ void __launch_bounds__(256) wf_adj_shade(TraceArgs a, WfState s, AdjW
             const uint32_t x = pid % a.width, y = pid / a.width;
             AdjPath p;
             adj_load(s, a, pid, x, y, p);
-            const uint4 hr = s.hit[pid];
-            Hit h;
-            h.t = __uint_as_float(hr.x);
-            h.prim = hr.y;
-            h.slot = hr.z;
-            h.kind = (int)hr.w;
-            again = adj_advance(tr, a, w, pid, x, y, h, p, w.pix + pid, s.prim0 + pid);
+            again = adj_advance(tr, a, w, pid, x, y, hit_unpack(s.hit[pid]), p, w.pix + pid, s.prim0 + pid);
             if (again) adj_store(s, pid, p);
         }
         warp_append(again, pid, next, &s.count[qsel ^ 1]);

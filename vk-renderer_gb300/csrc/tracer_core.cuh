@@ -221,6 +221,15 @@ struct Tracer {
     }
 };
 
+__device__ __forceinline__ uint4 hit_pack(const Hit& h)
+{
+    return make_uint4(__float_as_uint(h.t), h.prim, h.slot, (uint32_t)h.kind);
+}
+__device__ __forceinline__ Hit hit_unpack(uint4 v)
+{
+    return Hit{__uint_as_float(v.x), v.y, (int)v.w, v.z};
+}
+
 // Surface data of a hit (Tracer.comp:384-392, :404-408, :420-424).
 __device__ __forceinline__ void surface(const DevScene& sc, const Ray& ray, const Hit& h, V3& P, V3& N, Material& m)
 {

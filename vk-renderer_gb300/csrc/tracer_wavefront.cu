@@ -649,6 +649,15 @@ __device__ __forceinline__ bool advance_path(TR& tr, const TraceArgs& A, bool on
     return on && next_ray(A, x, y, cont, p);
 }
 
+// The next sample of pixel pid starts with its primary ray, whose hit sample 0
+// kept (s.hit0): h = that hit, and no ray to trace.  False with p elsewhere.
+__device__ __forceinline__ bool known_hit(const WfState& s, uint32_t pid, const PathRegs& p, Hit& h)
+{
+    if (!s.hit0 || p.depth > 0 || p.sample == 0) return false;
+    h = hit_unpack(s.hit0[pid]);
+    return true;
+}
+
 // ------------------------------------------------------------------- shade --
 template <int TIE, bool BVH, bool STATS, bool MULTI, bool NEE>
 __global__ void __launch_bounds__(256) wf_shade(TraceArgs a, WfState s, int qsel, const TraceArgs* slots)
@@ -665,7 +674,7 @@ __global__ void __launch_bounds__(256) wf_shade(TraceArgs a, WfState s, int qsel
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         const uint32_t qi = base + threadIdx.x;
-        const bool on = qi < n;
+        bool on = qi < n;
         const uint32_t pid = on ? queue[qi] : 0;
         const TraceArgs& A = SCENE_ARGS(MULTI, a, slots, MULTI && on ? s.scene_of[pid] : 0);
         PathTracer<TIE, BVH, STATS> tr(A.sc, stk, cnt, a.status, A.trav_limit);
@@ -675,13 +684,15 @@ __global__ void __launch_bounds__(256) wf_shade(TraceArgs a, WfState s, int qsel
         Hit h;
         if (on) {
             load_path(s, A, pid, x, y, ps);
-            const uint4 hr = s.hit[pid];
-            h.t = __uint_as_float(hr.x);
-            h.prim = hr.y;
-            h.slot = hr.z;
-            h.kind = (int)hr.w;
+            h = hit_unpack(s.hit[pid]);
+            if (s.hit0 && ps.sample == 0 && ps.depth == 0) s.hit0[pid] = hit_pack(h);
         }
-        const bool again = advance_path<NEE>(tr, A, on, x, y, h, ps);
+        bool again = false;
+        while (NEE ? __any_sync(0xFFFFFFFFu, on) : on) {
+            const bool more = advance_path<NEE>(tr, A, on, x, y, h, ps);
+            again = on ? more : again;
+            on = on && more && known_hit(s, pid, ps, h);
+        }
         if (again) store_path(s, pid, ps);
         warp_append(again, pid, next, &s.count[qsel ^ 1]);
     }
@@ -737,16 +748,23 @@ __global__ void __launch_bounds__(128) wf_finish(TraceArgs a, WfState s, int qse
         PathTracer<TIE, BVH, STATS, W8> tr(A.sc, stk, cnt, a.status, A.trav_limit);
         Hit h;
         h.t = on ? depth_tmax(ps.depth) : 0.0f;
-        bool again;
+        bool again = false;
+        const auto first_hit = [&](bool found, const Hit& first) {
+            note_primary(ps, found, first);
+            if (s.hit0 && ps.sample == 0 && ps.depth == 0) s.hit0[pid] = hit_pack(first);
+        };
         if (NEE) {
+            const bool given = on && known_hit(s, pid, ps, h);
             if (on) ps.acc = vclamp01(ps.acc);
-            const bool cont = trace_bounce(tr, A, on, false, false, h, ps.depth, ps.ray, ps.acc, ps.mask, ps.g,
-                                           [&](bool found, const Hit& first) { note_primary(ps, found, first); });
+            const bool cont = trace_bounce(tr, A, on, given, given && h.kind != 0, h, ps.depth, ps.ray, ps.acc, ps.mask,
+                                           ps.g, first_hit);
             again = on && next_ray(A, x, y, cont, ps);
         } else {
-            if (on) tr.trace(ps.ray, h, false);
+            if (on) first_hit(tr.trace(ps.ray, h, false), h);
             __syncwarp();
-            again = advance_path<false>(tr, A, on, x, y, h, ps);
+            for (bool go = on; go; go = again && known_hit(s, pid, ps, h))
+                again = advance_path<false>(tr, A, true, x, y, h, ps);
+            __syncwarp();
         }
         if (on && !again) {
             qi = n > threads ? threads + atomicAdd(&s.count[2], 1u) : n;

@@ -24,6 +24,8 @@ struct WfState {
     uint32_t* prim0;     // primary-hit primitive id
     uint32_t* queue[2];
     uint32_t* count;     // [0], [1]: queue lengths; [2]: extend's fetch cursor
+    uint4* hit0;         // as hit: the pixel's primary hit, which its later samples start from;
+                         // nullptr (with statistics): they trace the ray again
     uint32_t* scene_of;  // batched: scene index of each slot (written by generate)
 };
 
