@@ -39,21 +39,19 @@ UNIT = "Mrays/s"
 L2_FLUSH_BYTES = 256 << 20
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per ray of the
-# 8-wide extend kernel, from one ncu capture of every extend launch of two
-# whole c1 frames (1920x1080, 16 spp, finishing kernel off so that every ray
-# goes through it: 3.816 GB read + 0.26 GB written per frame of 67.6 M rays;
+# 8-wide extend kernel, from one ncu capture of every launch of a whole c1
+# frame (1920x1080, 16 spp: 2.311 GB read + 0.137 GB written for 36.5 M rays;
 # profiles/wf_extend_cw8_c1_dram.md); the frame's traffic is this times its
 # rays.
-NCU_EXTEND_DRAM_BYTES_PER_RAY = 60.3
+NCU_EXTEND_DRAM_BYTES_PER_RAY = 67.0
 
-# DRAM bytes of one replay of the c2 batch's graph (the bench's tuned shape:
-# 8-wide, 256 threads, hand-over at 1M paths), from one ncu capture of every
-# kernel of four replays (profiles/batch_c2_graph_launches.md): the extend
-# kernel's (21.4 GB read + 2.45 GB written) and all kernels' (42.0 + 14.5 GB;
-# wf_shade 20.4 + 9.8 GB).  The 2.1M triangles' 64-byte records and nodes
+# DRAM bytes of one c2 batch (8-wide, rounds launched one by one), from one ncu
+# capture of every kernel (profiles/batch_c2_graph_launches.md): the extend
+# kernel's (8.39 GB read + 0.97 GB written) and all kernels' (20.97 + 6.93 GB;
+# wf_shade 12.56 + 3.73 GB).  The 2.1M triangles' 64-byte records and nodes
 # exceed L2, unlike c1's.
-NCU_BATCH_EXTEND_DRAM_BYTES = 23.85e9
-NCU_BATCH_ALL_DRAM_BYTES = 56.45e9
+NCU_BATCH_EXTEND_DRAM_BYTES = 9.35e9
+NCU_BATCH_ALL_DRAM_BYTES = 27.90e9
 
 
 def peaks():
@@ -231,12 +229,22 @@ def tail_summary(rounds, tail_paths: int) -> dict | None:
     return out
 
 
+def traced_stats(st: dict, first: dict, spp: int) -> dict:
+    """What the forward kernels trace of a frame: st, the canonical counts of
+    the reference's rays, without the primary rays of every sample but the
+    first.  A pixel's samples all start with the same ray (no jitter,
+    Tracer.comp:568-574) and share its hit.  first: the counts of the frame
+    at one sample of depth 1 (no lights: its rays are the primary ones)."""
+    return {k: v - (spp - 1) * first[k] for k, v in st.items()}
+
+
 def batched_section(local: int, steps: int, warmup: int) -> dict:
     """c2: 64 scenes (triangles log-uniform in [1k, 200k], c1 geometry,
     resolutions from {128^2 .. 1024^2}, 4 spp, depth 6) traced (a) by the plain
     kernel launched once per scene and (b) as one wavefront over all scenes
     replayed as one CUDA graph, with the launch shape picked by the autotuner.
-    Mrays/s from canonical ray counts; L2 flushed before every timed step."""
+    Mrays/s from the rays that both trace (traced_stats); L2 flushed before
+    every timed step."""
     import numpy as np
     import torch
     from vktrace import abi, configs, tune
@@ -245,15 +253,19 @@ def batched_section(local: int, steps: int, warmup: int) -> dict:
     tr.upload_scenes([w.scene for w in wls])
     frames = [w.frame for w in wls]
 
-    def prm(kernel, stats=False, aovs=(abi.AOV_RGBA8,)):
-        return [abi.Tracer.params(w.width, w.height, spp=w.spp, max_depth=w.max_depth, rr_start=w.rr_start,
-                                  sky=w.sky, kernel=kernel, aovs=aovs, stats=stats) for w in wls]
+    def prm(kernel, stats=False, aovs=(abi.AOV_RGBA8,), first=False):
+        return [abi.Tracer.params(w.width, w.height, spp=1 if first else w.spp, max_depth=1 if first else w.max_depth,
+                                  rr_start=w.rr_start, sky=w.sky, kernel=kernel, aovs=aovs, stats=stats) for w in wls]
 
     stream = torch.cuda.current_stream()
     sptr = stream.cuda_stream
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device="cuda")
-    tr.trace_batched(frames, prm(abi.KERNEL_PLAIN, stats=True), use_graph=False, stream=sptr)
-    st = {k: int(v) for k, v in zip(abi.STATS_FIELDS, tr.readback_scene(0, abi.AOV_STATS))}
+    counts = []
+    for first in (False, True):
+        tr.trace_batched(frames, prm(abi.KERNEL_PLAIN, stats=True, first=first), use_graph=False, stream=sptr)
+        counts.append({k: int(v) for k, v in zip(abi.STATS_FIELDS, tr.readback_scene(0, abi.AOV_STATS))})
+    reference_rays = counts[0]["closest_rays"] + counts[0]["shadow_rays"]
+    st = traced_stats(*counts, wls[0].spp)
     rays = st["closest_rays"] + st["shadow_rays"]
 
     def timed(params, use_graph):
@@ -300,13 +312,14 @@ def batched_section(local: int, steps: int, warmup: int) -> dict:
             "plain_per_scene": {"value": rays / (ms_plain / 1e3) / 1e6, "ms_per_step": ms_plain,
                                 "kernel": "k_plain, one launch per scene"},
             "speedup_vs_plain_per_scene": ms_plain / ms_wf,
-            "max_image_rmse_vs_plain": rmse, "rays_per_step": rays, "scenes": len(wls), "pixels": pixels,
+            "max_image_rmse_vs_plain": rmse, "rays_per_step": rays, "reference_rays_per_step": reference_rays,
+            "scenes": len(wls), "pixels": pixels,
             "triangles": int(sum(len(w.scene.triangles) for w in wls)),
             "autotuned": best, "autotune_candidates": len(table),
             "decomposition": decomp,
             # canonical algorithmic bytes (the plain kernel's counts) over the
             # whole replay, against measured HBM; DRAM traffic from ncu
-            "roofline": {"bound": "issue / L2 latency (extend kernel, 88.6 % of a replay); the scenes exceed L2",
+            "roofline": {"bound": "L1 data pipe, ALU and issue (extend kernel, 77 % of a replay); the scenes exceed L2",
                          "achieved": k_bytes / (ms_wf / 1e3) / 1e9, "peak": hbm, "unit": "GB/s",
                          "frac": k_bytes / (ms_wf / 1e3) / 1e9 / hbm, "peak_source": hbm_src,
                          "algorithmic_bytes_per_step": k_bytes, "traffic": NCU_BATCH_EXTEND_DRAM_BYTES,
@@ -478,7 +491,10 @@ def adjoint_section(local: int, steps: int) -> dict:
     campos = campos_check(tr, wl, p_run)
     campos1 = campos_check(tr, wl, p_run, depth=1)
     tr.close()
-    fwd = fwd_rays / (ms_fwd / 1e3) / 1e6
+    # (the timed forward frames trace each pixel's primary ray once, the counted
+    # one and the adjoint every sample's)
+    fwd_traced = fwd_rays - (wl.spp - 1) * wl.pixels
+    fwd = fwd_traced / (ms_fwd / 1e3) / 1e6
     # headline: the forward frame's rays per second of adjoint time, i.e.
     # adjoint speed against forward speed on the same frame, by pure path
     # replay (the default); beside it the rays the adjoint traced (both
@@ -487,7 +503,8 @@ def adjoint_section(local: int, steps: int) -> dict:
     replay = adj_rays / (ms_adj / 1e3) / 1e6
     return {"metric": "adjoint Mrays/s (c3, path replay; forward rays per adjoint second)", "value": adjv,
             "unit": UNIT, "ms_per_step": ms_adj,
-            "forward": {"value": fwd, "ms_per_step": ms_fwd, "rays_per_step": fwd_rays},
+            "forward": {"value": fwd, "ms_per_step": ms_fwd, "rays_per_step": fwd_traced,
+                        "reference_rays_per_step": fwd_rays},
             "ratio_adjoint_to_forward": ms_fwd / ms_adj,
             "traced_rays": {"rays_per_step": adj_rays, "mrays_per_s": replay,
                             "ratio_to_forward_mrays_per_s": replay / fwd},
@@ -676,7 +693,7 @@ def small_configs_section(local: int, steps: int, cpu: bool) -> dict:
             if rays is None:  # canonical counts from the plain kernel
                 tr.trace(wl.frame, p, sptr)
                 st = tr.stats()
-                rays = st["closest_rays"] + st["shadow_rays"]
+                rays = st["closest_rays"] + st["shadow_rays"] - (wl.spp - 1) * wl.pixels  # traced_stats
                 p.stats = 0
             for _ in range(3):
                 tr.trace(wl.frame, p, sptr)
@@ -957,14 +974,19 @@ def run_ours(args):
     p_run = abi.Tracer.params(wl.width, wl.height, aovs=(abi.AOV_RGBA8,), stats=False, **common)
     # counting pass (untimed) with the plain kernel, whose node-visiting order
     # is the oracle's: the canonical ray / node / primitive counts of the frame.
-    # Every kernel traces exactly these rays (the wavefront's speculative
-    # traversal fetches ~1.5 % more nodes than this canonical count).
+    # Without statistics every kernel traces these less the repeated primary
+    # rays (traced_stats), and those are the rays of `value` (the wavefront's
+    # speculative traversal fetches ~1.5 % more nodes than the canonical count).
     p_count = abi.Tracer.params(wl.width, wl.height, aovs=(abi.AOV_RGBA8, abi.AOV_RGBA32F), stats=True,
                                 **dict(common, kernel=abi.KERNEL_PLAIN, block=0))
     tr.trace(wl.frame, p_count, sptr)
     st = tr.stats()
-    rays = st["closest_rays"] + st["shadow_rays"]
     plain_img = tr.readback(abi.AOV_RGBA32F)
+    p_first = abi.Tracer.params(wl.width, wl.height, aovs=(abi.AOV_RGBA8,), stats=True,
+                                **dict(common, kernel=abi.KERNEL_PLAIN, block=0, spp=1, max_depth=1))
+    tr.trace(wl.frame, p_first, sptr)
+    st_traced = traced_stats(st, tr.stats(), wl.spp)
+    rays = st_traced["closest_rays"] + st_traced["shadow_rays"]
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device="cuda")
 
     for _ in range(args.warmup):
@@ -1036,7 +1058,7 @@ def run_ours(args):
     if rank == 0:
         peak, peak_kind = peaks()
         l2_gbs = tr.measure_l2_read(32 << 20, 64)
-        ab = algorithmic_bytes(st, wl.pixels, 4)
+        ab = algorithmic_bytes(st_traced, wl.pixels, 4)
         # dominant kernel: the traversal (extend) kernel of the wavefront, one
         # launch per round; its algorithmic bytes are the traversal bytes of
         # the frame, its time the sum of its launches (CUDA events)
@@ -1056,18 +1078,19 @@ def run_ours(args):
             "impl_config": {"kernel": args.kernel, "block": args.block, "bvh_depth": bvh_depth,
                             "traversal": TRAVERSAL_LABEL[args.bvh_width], "tail_paths": args.tail_paths},
             "rays_per_step": rays,
+            "reference_rays_per_step": st["closest_rays"] + st["shadow_rays"],
             "max_image_rmse_vs_plain": rmse_vs_plain,
             "stats": st,
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": 96,
                     "d2h_bytes_per_step": wl.pixels * 4},
-            # the traversal's working set (4.8 MB of triangles, 2.1 MB of nodes)
-            # stays in L2: what bounds it is instruction issue (the integer
-            # pipe of the slab tests), the warps' SIMD efficiency and the
-            # latency of dependent L1/L2 node fetches, not HBM bandwidth.
+            # the traversal's working set (8-wide nodes and triangle records)
+            # stays in L2: what bounds it is the L1 data pipe (a wavefront per
+            # lane and load), the integer pipe of the slab tests and issue,
+            # not HBM bandwidth.
             # peak/frac: against the measured HBM copy bandwidth (the common
             # denominator); l2.frac: against L2 read bandwidth
-            "roofline": {"bound": "instruction issue (integer ALU, 68 % issue active in ncu) with L1/L2 latency "
-                                  "behind it; scene L2-resident", "achieved": achieved, "peak": peak,
+            "roofline": {"bound": "L1 data pipe (68 %), integer ALU (62 %) and issue (60 % active in ncu) "
+                                  "together; scene L2-resident", "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak,
                          "traffic": (NCU_EXTEND_DRAM_BYTES_PER_RAY * rays
                                      if kern == abi.KERNEL_WAVEFRONT else None),

@@ -312,7 +312,7 @@ int tracer_set_edge_sampling(tracer_ctx* ctx, uint32_t samples_per_edge);
  * (width x height x max_depth x 16 bytes; allocated on first use and kept
  * for later adjoints of the context): pass 2 then replays them without
  * tracing, which halves the adjoint's traced rays with the same gradients
- * (c3: 0.48 against 0.79 ms).  A trace whose hits would exceed the limit
+ * (c3: 0.32 against 0.54 ms).  A trace whose hits would exceed the limit
  * traces pass 2 instead.  0 = never keep them, the default: pure path replay,
  * no stored path vertices (frees the buffer).  No counterpart in the
  * reference. */

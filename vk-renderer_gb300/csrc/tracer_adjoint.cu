@@ -212,12 +212,11 @@ __device__ __forceinline__ V3 pixel_delta(float4 dl, V3 lin, uint32_t spp)
 
 // One thread per pixel; the warp's lanes go through the same jobs together,
 // bounce by bounce: with no linear image given, every sample's radiance first
-// (job 0 .. spp - 1), then pass 1 and pass 2 of every sample.  One loop body
-// holds the kernel's only closest-hit traversal and the two passes' shadow
-// rays, which the lanes trace together: with a traversal inlined at every use
-// and lanes going their own ways, two thirds of the issue slots were lost to
-// instruction fetches (160^2 x 4 spp, one light: 8.87 ms, no-instruction
-// stalls 9.7 of 17 cycles per issue).
+// (job 0 .. spp - 1), then pass 1 and pass 2 of every sample.  All its rays go
+// through one copy of the traversal (trace_rays): with five and lanes going
+// their own ways, two thirds of the issue slots were lost to instruction
+// fetches (160^2 x 4 spp, one light, with outlines: 11.1 ms; 1.59 with three
+// copies and the lanes together, 1.26 with one; 1.35 at 168 registers).
 template <int TIE, bool BVH, bool CAM>
 __global__ void __launch_bounds__(128) k_adjoint(TraceArgs a, AdjArgs ga)
 {
