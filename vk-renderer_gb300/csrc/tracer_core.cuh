@@ -262,10 +262,11 @@ static __device__ __noinline__ V3 jitter(V3 d, float phi, float sina, float cosa
     return (u * c + v * s) * sina + w * cosa;
 }
 
-// powf, rand01's cosine and jitter are out of line: the kernels that shade hold
-// several copies of each otherwise, and lose a third of their issue slots to
-// instruction fetches (the reference's frame, k_plain: 1506 us inlined, 1379
-// out of line with the primitive loops not unrolled either, 1611 at first).
+// powf and jitter are out of line: the kernels that shade hold several copies
+// of each otherwise, and lose issue slots to instruction fetches (the
+// reference's frame, k_plain: 1506 us inlined with rand01, 1379 out of line
+// with the primitive loops not unrolled either, 1611 at first; alone, jitter
+// inlined costs 1.5 to 5 % there, powf 1 to 2 %).
 static __device__ __noinline__ float pow_call(float x, float y) { return powf(x, y); }
 
 // Tracer.comp:265-272
@@ -304,7 +305,8 @@ __device__ __forceinline__ float geometry_smith(V3 N, V3 V, V3 L, float roughnes
 // hit, in two parts around its shadow ray.  nee_ray: the direction to a
 // random point of the light's cone, and the distance to the light; consumes
 // two random numbers whether or not the light is visible.
-__device__ __forceinline__ V3 nee_ray(const DevScene& sc, uint32_t si, V3 P, Rng& g, float& t)
+template <class G>
+__device__ __forceinline__ V3 nee_ray(const DevScene& sc, uint32_t si, V3 P, G& g, float& t)
 {
     const float4 geo = __ldg(sc.sph_rec + 4 * (size_t)si + 3);
     const V3 sP = v3(geo);
@@ -362,8 +364,9 @@ struct Bounce {
 // The closest hit's part, for a lane that is `on`: sky on a miss (surv: the
 // share of it that counts; 1 but in the adjoint replay), else the surface and
 // the diffuse lobe's random numbers.
+template <class G>
 __device__ __forceinline__ void bounce_begin(const TraceArgs& a, bool on, bool found, const Hit& h, const Ray& ray,
-                                             V3 surv, V3& acc, const V3& mask, Rng& g, Bounce& b)
+                                             V3 surv, V3& acc, const V3& mask, G& g, Bounce& b)
 {
     b.hit = on && found;
     b.diffuse = false;
@@ -384,8 +387,9 @@ __device__ __forceinline__ void bounce_begin(const TraceArgs& a, bool on, bool f
 
 // After the next-event estimates: material scatter, Russian roulette.  Updates
 // acc, mask and ray; returns false when the path ends or the lane has no hit.
+template <class G>
 __device__ __forceinline__ bool bounce_end(const TraceArgs& a, const Bounce& b, uint32_t depth, Ray& ray, V3& acc,
-                                           V3& mask, Rng& g)
+                                           V3& mask, G& g)
 {
     if (!b.hit) return false;
     const Material& mat = b.mat;
@@ -422,9 +426,9 @@ __device__ __forceinline__ bool bounce_end(const TraceArgs& a, const Bounce& b, 
 // the shadow rays of some run while the others wait, or trace something else
 // of the same warp: 3.5 of 32 lanes active in the finishing kernel of a
 // 640x360 frame with two lights.
-template <bool NEE = true, bool SYNC = false, class TR>
+template <bool NEE = true, bool SYNC = false, class TR, class G>
 __device__ __forceinline__ bool shade_bounce(TR& tr, const TraceArgs& a, bool on, uint32_t depth, bool found,
-                                             const Hit& h, Ray& ray, V3& acc, V3& mask, Rng& g)
+                                             const Hit& h, Ray& ray, V3& acc, V3& mask, G& g)
 {
     Bounce b;
     bounce_begin(a, on, found, h, ray, splat(1.0f), acc, mask, g, b);
@@ -458,16 +462,16 @@ __device__ __forceinline__ bool shade_bounce(TR& tr, const TraceArgs& a, bool on
 //   first(found, h)            sees the closest hit; fills P, N, mat, diffuse of b
 //   light(si, L, t, g0)        an emitter that the surface sees; g0: the random
 //                              numbers of its direction L are the next two
-template <class TR, class First, class Light>
+template <class TR, class G, class First, class Light>
 __device__ __forceinline__ void trace_rays(TR& tr, const TraceArgs& a, bool on, bool given, bool found, Hit h,
-                                           const Ray& ray, Rng& g, Bounce& b, const First& first, const Light& light)
+                                           const Ray& ray, G& g, Bounce& b, const First& first, const Light& light)
 {
     bool go = on;
     V3 L;
     float t = 0.0f;
     uint32_t si = 0;
     Ray r = ray;
-    Rng g0 = g;
+    G g0 = g;
 #pragma unroll 1
     for (uint32_t k = 0;; ++k) {
         bool hit = found;
@@ -490,9 +494,9 @@ __device__ __forceinline__ void trace_rays(TR& tr, const TraceArgs& a, bool on, 
 }
 
 // A whole depth iteration by a whole warp, its rays in trace_rays.
-template <class TR, class F>
+template <class TR, class G, class F>
 __device__ __forceinline__ bool trace_bounce(TR& tr, const TraceArgs& a, bool on, bool given, bool found0, const Hit& h0,
-                                             uint32_t depth, Ray& ray, V3& acc, V3& mask, Rng& g, const F& first_hit)
+                                             uint32_t depth, Ray& ray, V3& acc, V3& mask, G& g, const F& first_hit)
 {
     Bounce b;
     trace_rays(
@@ -501,7 +505,7 @@ __device__ __forceinline__ bool trace_bounce(TR& tr, const TraceArgs& a, bool on
             if (on) first_hit(found, h);
             bounce_begin(a, on, found, h, ray, splat(1.0f), acc, mask, g, b);
         },
-        [&](uint32_t si, V3 L, float t, const Rng&) { b.e = b.e + nee_value(a, si, b.P, b.N, b.mat, L, t); });
+        [&](uint32_t si, V3 L, float t, const G&) { b.e = b.e + nee_value(a, si, b.P, b.N, b.mat, L, t); });
     return bounce_end(a, b, depth, ray, acc, mask, g);
 }
 
@@ -532,7 +536,8 @@ __device__ __forceinline__ Ray primary_ray(const TraceArgs& a, uint32_t x, uint3
 }
 
 // Tracer.comp:585-592: average, Reinhard, gamma 1/2.2, dither, store.
-__device__ __forceinline__ void resolve_pixel(const TraceArgs& a, uint32_t x, uint32_t y, V3 accum, Rng& g,
+template <class G>
+__device__ __forceinline__ void resolve_pixel(const TraceArgs& a, uint32_t x, uint32_t y, V3 accum, G& g,
                                               uint32_t prim0, float t0)
 {
     accum = accum / (float)a.spp;

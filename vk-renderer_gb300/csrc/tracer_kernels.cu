@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(256, BLOCKS) k_plain(TraceArgs a)
     const uint32_t x = blockIdx.x * 16 + (tid & 15);
     const uint32_t y = blockIdx.y * (nthreads >> 4) + (tid >> 4);
     bool alive = x < a.width && y < a.height;
-    Rng g;
+    std::conditional_t<!BVH && NEE && BLOCKS >= 4, RngCall, Rng> g;
     seed_rng(a, x, y, g);
     const Ray pr = primary_ray(a, x, y);
     Ray ray = pr;
