@@ -383,20 +383,18 @@ int tracer_last_rounds(tracer_ctx* ctx, tracer_round_info* out, uint32_t cap, ui
  * has already allocated.  Such a caller creates the context and uploads the
  * scene once at start-up, then calls this entry point per frame.
  *
- * It runs the wavefront kernels on the scene uploaded to ctx, 128 threads per
- * block (the rounds with the binary traversal, the finishing launch with the
- * 8-wide one unless bvh_width is 2; widths other than 0 and 2 are refused; the
- * block field is not read), with no queue length read back: when the image
- * has fewer pixels than tail_paths -- always with the automatic threshold,
- * which is the extend kernel's resident threads as in tracer_trace -- the
- * generate kernel and one finishing launch; otherwise (tail_paths = 1, or a
- * tail_paths at most the pixel count) every one of the spp * max_depth + 1
- * rounds is launched (2 kernels each, a round with no live path returning at
- * once).  It writes the
- * image straight into caller-owned device buffers: rgba8_out (w*h*4 bytes)
+ * It traces the scene uploaded to ctx with 128 threads per block (the block
+ * field is not read) and no queue length read back: when the image has fewer
+ * pixels than tail_paths -- always with the automatic threshold, which is the
+ * extend kernel's resident threads as in tracer_trace -- one launch of the
+ * plain kernel, triangles over the 8-wide BVH unless bvh_width is 2 (widths
+ * other than 0 and 2 are refused); otherwise (tail_paths = 1, or a tail_paths
+ * at most the pixel count) the wavefront over the binary BVH with every one of
+ * the spp * max_depth + 1 rounds launched (2 kernels each, a round with no
+ * live path returning at once).  It writes the image straight into caller-owned device buffers: rgba8_out (w*h*4 bytes)
  * and/or rgba32f_out (w*h*16 bytes); either may be NULL, not both.  The
  * wavefront's path state, queues and counters live in one fixed array of
- * device memory inside the library (about 1.8 MB, reserved on every GPU that
+ * device memory inside the library (about 2.3 MB, reserved on every GPU that
  * loads the library until the process exits), so images are limited to
  * TRACER_NOALLOC_MAX_PIXELS pixels and spp * max_depth to
  * TRACER_NOALLOC_MAX_ROUNDS; larger requests return

@@ -296,8 +296,8 @@ cudaEvent_t prof_event(tracer_ctx* c, size_t i)
 }
 
 // Triangle-only scenes without lights whose rays visit at most this many 8-wide
-// nodes (build_cw8's estimate) run no rounds: the finishing kernel alone was
-// faster by (frame 640x360 x 4 spp / 1280x720 x 4 / 1920x1080 x 8) 1.95 / 1.90 /
+// nodes (build_cw8's estimate) run no rounds: the finishing kernel alone (every
+// sample's primary ray still traced) was faster by (frame 640x360 x 4 spp / 1280x720 x 4 / 1920x1080 x 8) 1.95 / 1.90 /
 // 1.84 on a soup of 500 triangles (estimate 5.1), 1.66 / 1.58 / 1.51 on 2k (9.0),
 // 1.31 / 1.22 / 1.15 on 10k (16.8); 1.35 / 1.54 / 1.25 on a height field of 2k
 // (7.2), 1.37 / 1.33 / 1.04 on 20k (10.4), 1.21 / 1.15 / 0.91 on 200k (13.8);
@@ -313,7 +313,10 @@ bool cheap_rays(double cost) { return cost > 0.0 && cost <= kCheapRays; }
 // was drawn, 1280x720 x 4 spp x depth 6, ms: height field of 20k triangles
 // 0.86 / 1.07, of 200k 1.67 / 1.81, soup of 10k 1.13 / 1.12; 20k triangles and
 // 30 spheres 3.48 / 5.13, 12k and 200 with 2 lights 14.2 / 21.3, 60k and 200
-// with 2 lights 33.4 / 44.1; 40 spheres 0.26 / 0.60, 2000 3.02 / 3.28.
+// with 2 lights 33.4 / 44.1; 40 spheres 0.26 / 0.60, 2000 3.02 / 3.28.  Since
+// both trace a pixel's primary ray once: the height fields 0.68 / 0.84 and 1.31 /
+// 1.43, soup of 10k 0.63 / 0.60, of 30k 1.82 / 1.31, 20k and 30 spheres 2.59 /
+// 3.18.
 bool plain_suits(const SceneBuffers& s)
 {
     if (s.cw8) return cheap_rays(s.cw8_cost);
