@@ -376,15 +376,28 @@ bool pack_w8(const std::vector<Cw8Node>& in, std::vector<W8Node>& out)
 void split_leaves(const tracer_bvh_node* nodes, uint32_t num_nodes, const double (*tri)[6],
                   std::vector<tracer_bvh_node>& out, std::vector<uint32_t>& slot_out)
 {
+    // Only what the root reaches is split: a caller's array may hold other
+    // entries, whose ranges nobody has checked.
+    std::vector<uint8_t> reached(num_nodes, 0);
+    std::vector<uint32_t> todo(1, 0u);
     uint32_t n_prims = 0;
-    for (uint32_t i = 0; i < num_nodes; ++i) n_prims += nodes[i].count > 0 ? (uint32_t)nodes[i].count : 0u;
+    while (!todo.empty()) {
+        const uint32_t i = todo.back();
+        todo.pop_back();
+        reached[i] = 1;
+        if (nodes[i].count > 0) {
+            n_prims += (uint32_t)nodes[i].count;
+        } else {
+            todo.push_back((uint32_t)nodes[i].left_or_first);
+            todo.push_back((uint32_t)nodes[i].left_or_first + 1);
+        }
+    }
     out.assign(nodes, nodes + num_nodes);
     out.reserve(2 * (size_t)n_prims + num_nodes);
     slot_out.resize(n_prims);
     for (uint32_t k = 0; k < n_prims; ++k) slot_out[k] = k;
-    std::vector<uint32_t> todo;
     for (uint32_t i = 0; i < num_nodes; ++i) {
-        if (nodes[i].count <= 1) continue;
+        if (!reached[i] || nodes[i].count <= 1) continue;
         const tracer_bvh_node leaf = nodes[i];  // every part's box stays inside it
         todo.assign(1, i);
         while (!todo.empty()) {

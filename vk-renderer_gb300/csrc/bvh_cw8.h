@@ -89,8 +89,9 @@ static_assert(sizeof(W8Node) == 96, "device node is 96 bytes");
 // primitives each; false otherwise.
 bool pack_w8(const std::vector<Cw8Node>& in, std::vector<W8Node>& out);
 
-// Splits every leaf of a binary BVH over triangles down to single triangles
-// (kCw8MaxLeafPrims at most per leaf), keeping the nodes above.  tri[k]: low
+// Splits every leaf that the root of a valid binary BVH over triangles reaches
+// down to single triangles (kCw8MaxLeafPrims at most per leaf), keeping the
+// nodes above and whatever else the array holds.  tri[k]: low
 // and high corner of the box of leaf-ordered triangle k.  out: the deeper
 // tree, its leaves ranges of a new order whose entry j is leaf-ordered slot
 // slot_out[j].  A part's box is that of its triangles, padded as the binary
