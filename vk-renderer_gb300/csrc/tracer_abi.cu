@@ -112,6 +112,7 @@ struct tracer_ctx {
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
     bool pending = false;
+    bool abandoned = false;  // what is pending belongs to a call that failed: nobody's result
     uint32_t timeout_ms = 60000;
     std::string err;
     SceneBuffers scene;
@@ -243,6 +244,10 @@ int finish(tracer_ctx* c)
     int r = wait_event(c, c->done, kSpinResult);
     if (r != TRACER_OK) return r;
     c->pending = false;
+    if (c->abandoned) {
+        c->abandoned = false;
+        return TRACER_OK;
+    }
     const int st = *static_cast<volatile int*>(c->status);
     if (st == ST_TRAVERSAL_LIMIT)
         return fail(c, TRACER_ERR_TRAVERSAL_LIMIT, "a ray exceeded the BVH traversal step limit");
@@ -250,6 +255,22 @@ int finish(tracer_ctx* c)
         return fail(c, TRACER_ERR_STACK_OVERFLOW, "traversal stack depth too small for the BVH");
     return TRACER_OK;
 }
+
+// A call's launches until it has recorded their end itself (kept): a call that
+// fails between (a queue length that came too late, a refused launch) leaves
+// kernels behind, and the next one waits for them before it clears the status
+// word and uses the buffers; their status is not the next call's.
+struct Launched {
+    tracer_ctx* c;
+    cudaStream_t st;
+    bool kept = false;
+    ~Launched()
+    {
+        if (kept || cudaEventRecord(c->done, st) != cudaSuccess) return;
+        c->pending = true;
+        c->abandoned = true;
+    }
+};
 
 constexpr int kCountSlots = 8;  // ring of lagged queue-length copies
 constexpr int kCountLag = 3;    // rounds the launch loop runs ahead of the GPU
@@ -956,6 +977,7 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
     c->last_finish = false;
     c->last_launches = 0;
     if (c->profiling) cudaEventRecord(c->prof_begin, st);
+    Launched launched{c, st};
 
     if (kernel == TRACER_KERNEL_PLAIN) {
         LaunchConfig lc{block, stats, p->tie_mode, s.bvh ? 1 : 0, s.cw8 ? 1 : 0, (uint32_t)c->sm_count};
@@ -989,7 +1011,7 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
     if (c->profiling) cudaEventRecord(c->prof_end, st);
     if (e == cudaSuccess) e = cudaEventRecord(c->done, st);
     if (e != cudaSuccess) return cuda_fail(c, e, "trace launch");
-    c->pending = true;
+    c->pending = launched.kept = true;
     return TRACER_OK;
 }
 
@@ -1675,6 +1697,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
     c->last_finish = false;
     c->last_launches = 0;
     if (c->profiling) cudaEventRecord(c->prof_begin, st);
+    Launched launched{c, st};
 
     if (kernel == TRACER_KERNEL_PLAIN) {
         LaunchConfig lc{block, stats, TRACER_TIES_STRICT, 1, 0, (uint32_t)c->sm_count};
@@ -1777,7 +1800,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
     if (c->profiling) cudaEventRecord(c->prof_end, st);
     if (e == cudaSuccess) e = cudaEventRecord(c->done, st);
     if (e != cudaSuccess) return cuda_fail(c, e, "batched trace launch");
-    c->pending = true;
+    c->pending = launched.kept = true;
     return TRACER_OK;
 }
 
@@ -1932,6 +1955,7 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
     c->last_mask = 1u << TRACER_AOV_STATS;
     c->width = p->width;
     c->height = p->height;
+    Launched launched{c, st};
     if (use_wf) {
         e = ensure_wavefront(c, npx);
         if (e == cudaSuccess) e = dalloc(ab.pix, npx);
@@ -1983,7 +2007,7 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
     if (e == cudaSuccess) e = launch_grad_to_float(ab.grad.p, ab.gradf.p, (uint32_t)ng, st);
     if (e == cudaSuccess) e = cudaEventRecord(c->done, st);
     if (e != cudaSuccess) return cuda_fail(c, e, "adjoint launch");
-    c->pending = true;
+    c->pending = launched.kept = true;
     // outputs: device pointers get asynchronous copies, host pointers wait
     float* outs[3] = {d_albedo, d_emission, d_campos};
     const size_t offs[3] = {0, 3 * (size_t)s.nm, 6 * (size_t)s.nm};
