@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(BLOCK, 896 / BLOCK)
                 }
                 uint2 P;
                 w8_visit(MULTI ? my_nodes : a.sc.tri_cw8, idx, cr, tbest, G, P);
-                if (STATS) cnt.c[C_NODES] += 4;
+                if (STATS) cnt.c[C_NODES] += 3;
                 held[nh * BLOCK] = P;
                 nh += w8_any(P) ? 1 : 0;
             }
