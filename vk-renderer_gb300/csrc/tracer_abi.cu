@@ -344,6 +344,19 @@ bool plain_suits(const SceneBuffers& s)
     return s.nt == 0 || s.tri_cw8.p;
 }
 
+// A pixel's primary hit is kept for its later samples (WfState::hit0) where there
+// are any and nothing counts rays.
+bool keeps_hits(int stats, uint32_t spp) { return !stats && spp > 1; }
+
+// Whether shade starts the next sample from it at once (the finishing kernel
+// always does): everywhere but on lit scenes without triangles, whose primary
+// ray costs less in a round of all paths than the shadow rays of the few lanes
+// of a warp that are at a sample's end cost in shade.  Lit spheres, 640x360 and
+// 1280x720 x 4 spp, 1920x1080 x 8, depth 6, at once / in a round, ms: 64 1.63 / 1.33,
+// 4.81 / 3.94, 20.9 / 16.2; 5000 5.53 / 4.65, 17.6 / 14.6, 76.9 / 60.5; with
+// triangles (2000, 20 spheres, one light) 1.14 / 1.26, 3.24 / 3.99, 12.7 / 16.2.
+bool shade_keeps_on(bool keeps, bool lit, uint32_t triangles) { return keeps && !(lit && triangles == 0); }
+
 // Launches the wavefront: generate, then rounds of extend + shade until the
 // path queue is empty (read back a few rounds behind the launches) or
 // max_rounds is reached (no path needs more than spp * max_depth rounds).
@@ -361,14 +374,15 @@ bool plain_suits(const SceneBuffers& s)
 // cheap: the scene's rays are short, so that a round's launches and path state
 // cost more than its traversals gain from the extend kernel: with the
 // automatic tail no round runs either (kCheapRays).
+// kept: keeps_hits.
 // With adj, the adjoint's generate, shade and finishing stages run instead of
 // the forward's (a.linear = the forward image).
 int run_wavefront(tracer_ctx* c, const TraceArgs& a, WfConfig& wc, size_t nslots, uint64_t max_rounds,
-                  uint32_t stack, uint32_t wavefront, uint32_t tail, bool cheap, cudaStream_t st,
+                  uint32_t stack, uint32_t wavefront, uint32_t tail, bool cheap, bool kept, cudaStream_t st,
                   const AdjWf* adj = nullptr)
 {
     WfState ws{c->wf_ray_o.p, c->wf_ray_d.p, c->wf_hit.p, c->wf_acc.p, c->wf_mask.p, c->wf_accum.p,
-               c->wf_prim0.p, {c->wf_q0.p, c->wf_q1.p}, c->wf_count.p, wc.stats ? nullptr : c->wf_hit0.p, c->wf_scene.p};
+               c->wf_prim0.p, {c->wf_q0.p, c->wf_q1.p}, c->wf_count.p, kept ? c->wf_hit0.p : nullptr, c->wf_scene.p};
     int per = wf_extend_blocks_per_sm(wc, stack);
     if (per <= 0) return fail(c, TRACER_ERR_INVALID_ARG, "extend kernel cannot be resident (stack %u)", stack);
     if (wavefront && (int)wavefront < per) per = (int)wavefront;
@@ -995,6 +1009,8 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
         wc.bvh = s.bvh ? 1 : 0;
         wc.stats = stats;
         wc.has_emitters = s.ne > 0;
+        const bool kept = keeps_hits(stats, p->spp);
+        wc.shade_samples = shade_keeps_on(kept, s.ne > 0, s.nt);
         wc.block = p->block ? p->block : 128;
         uint32_t wstack = stack;
         r = pick_width(c, p, wstack, wc.wide);
@@ -1005,7 +1021,7 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
         wc.finish_w8 = s.cw8 && !binary_asked(p);
         a.stack_depth = wstack;
         r = run_wavefront(c, a, wc, npx, (uint64_t)p->spp * p->max_depth + 1, wstack, p->wavefront, p->tail_paths,
-                          wc.wide == WF_WIDTH_8 && cheap_rays(s.cw8_cost), st);
+                          wc.wide == WF_WIDTH_8 && cheap_rays(s.cw8_cost), kept, st);
         if (r != TRACER_OK) return r;
     }
     if (c->profiling) cudaEventRecord(c->prof_end, st);
@@ -1284,19 +1300,21 @@ extern "C" int tracer_trace_noalloc(tracer_ctx* c, const tracer_frame* f, const 
     a.pixel_base = 0;
     a.num_slots = p->width * p->height;
 
+    const bool kept = keeps_hits(0, p->spp);
     WfState ws{reinterpret_cast<float4*>(base + kNaOffRayO), reinterpret_cast<float4*>(base + kNaOffRayD),
                reinterpret_cast<uint4*>(base + kNaOffHit), reinterpret_cast<float4*>(base + kNaOffAcc),
                reinterpret_cast<float4*>(base + kNaOffMask), reinterpret_cast<float4*>(base + kNaOffAccum),
                reinterpret_cast<uint32_t*>(base + kNaOffPrim0),
                {reinterpret_cast<uint32_t*>(base + kNaOffQ0), reinterpret_cast<uint32_t*>(base + kNaOffQ1)},
-               reinterpret_cast<uint32_t*>(base + kNaOffCount), reinterpret_cast<uint4*>(base + kNaOffHit0),
-               nullptr};
+               reinterpret_cast<uint32_t*>(base + kNaOffCount),
+               kept ? reinterpret_cast<uint4*>(base + kNaOffHit0) : nullptr, nullptr};
     WfConfig wc;
     std::memset(&wc, 0, sizeof wc);
     wc.tie = p->tie_mode;
     wc.bvh = s.bvh ? 1 : 0;
     wc.stats = 0;
     wc.has_emitters = s.ne > 0;
+    wc.shade_samples = shade_keeps_on(kept, s.ne > 0, s.nt);
     wc.finish_w8 = s.cw8 && !binary_asked(p);
     wc.block = 128;
     int per = wf_extend_blocks_per_sm(wc, stack);
@@ -1613,6 +1631,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
     std::vector<size_t> base(n);
     size_t total = 0;
     uint64_t max_rounds = 0;
+    uint32_t max_spp = 1;
     for (uint32_t k = 0; k < n; ++k) {
         const tracer_trace_params& p = params[k];
         if (p.width == 0 || p.height == 0 || p.width > 32768 || p.height > 32768)
@@ -1623,6 +1642,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
         base[k] = total;
         total += (size_t)p.width * p.height;
         max_rounds = std::max<uint64_t>(max_rounds, (uint64_t)p.spp * p.max_depth + 1);
+        max_spp = std::max(max_spp, p.spp);
     }
     if (total >= 0xFFFFFFFFull) return fail(c, TRACER_ERR_NO_SUITABLE_SURFACE, "batch has too many pixels");
     int r = finish(c);
@@ -1717,6 +1737,8 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
         wc.stats = stats;
         wc.multi = 1;
         wc.has_emitters = c->batch_emitters;
+        const bool kept = keeps_hits(stats, max_spp);
+        wc.shade_samples = shade_keeps_on(kept, c->batch_emitters, c->batch.nt);
         wc.finish_w8 = c->batch.cw8 && !binary_asked(&p0);
         wc.block = block;
         wc.wide = wide;
@@ -1728,11 +1750,11 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
         for (uint32_t k = 0; k < n; ++k) cost += c->batch_cost[k] * params[k].width * params[k].height / (double)total;
         const bool cheap = wide == WF_WIDTH_8 && cheap_rays(cost);
         if (!use_graph) {
-            r = run_wavefront(c, a, wc, total, max_rounds, stack, p0.wavefront, p0.tail_paths, cheap, st);
+            r = run_wavefront(c, a, wc, total, max_rounds, stack, p0.wavefront, p0.tail_paths, cheap, kept, st);
             if (r != TRACER_OK) return r;
         } else {
             WfState ws{c->wf_ray_o.p, c->wf_ray_d.p, c->wf_hit.p, c->wf_acc.p, c->wf_mask.p, c->wf_accum.p,
-                       c->wf_prim0.p, {c->wf_q0.p, c->wf_q1.p}, c->wf_count.p, wc.stats ? nullptr : c->wf_hit0.p,
+                       c->wf_prim0.p, {c->wf_q0.p, c->wf_q1.p}, c->wf_count.p, kept ? c->wf_hit0.p : nullptr,
                        c->wf_scene.p};
             int per = wf_extend_blocks_per_sm(wc, stack);
             if (per <= 0) return fail(c, TRACER_ERR_INVALID_ARG, "extend kernel cannot be resident");
@@ -1742,7 +1764,8 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
             wc.shade_grid = (uint32_t)(sg < (size_t)c->sm_count * 8 ? sg : (size_t)c->sm_count * 8);
             // the graph bakes in sizes, launch shapes and buffer addresses
             std::vector<uint64_t> key = {n, total, max_rounds, block, stack, (uint64_t)stats, wc.extend_grid,
-                                         (uint64_t)wide, (uint64_t)binary_asked(&p0), (uint64_t)cheap, p0.tail_paths,
+                                         (uint64_t)wide, (uint64_t)binary_asked(&p0), (uint64_t)cheap, (uint64_t)kept,
+                                         (uint64_t)wc.shade_samples, p0.tail_paths,
                                          (uint64_t)(uintptr_t)c->wf_ray_o.p, (uint64_t)(uintptr_t)c->wf_hit0.p,
                                          (uint64_t)(uintptr_t)c->batch_slots.p,
                                          (uint64_t)(uintptr_t)c->b_rgba8.p, (uint64_t)(uintptr_t)c->b_rgba32f.p,
@@ -1758,7 +1781,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
                 // run of this batch reaches (launched here, with read-backs).
                 // Any frame is still traced completely: the finishing kernel
                 // runs whatever paths are queued after that round.
-                r = run_wavefront(c, a, wc, total, max_rounds, stack, p0.wavefront, p0.tail_paths, cheap, st);
+                r = run_wavefront(c, a, wc, total, max_rounds, stack, p0.wavefront, p0.tail_paths, cheap, kept, st);
                 if (r != TRACER_OK) return r;
                 const int fin_per = c->last_finish ? wf_finish_blocks_per_sm(wc, stack) : 0;
                 const uint64_t rounds = fin_per > 0 ? c->last_handover : max_rounds;
@@ -1986,7 +2009,7 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
         if (c->profiling) cudaEventRecord(c->prof_begin, st);
         // a sample takes at most max_depth rounds in each pass
         r = run_wavefront(c, a, wc, npx, 2 * (uint64_t)p->spp * p->max_depth + 1, wstack, p->wavefront, p->tail_paths,
-                          wc.wide == WF_WIDTH_8 && cheap_rays(s.cw8_cost), st, &aw);
+                          wc.wide == WF_WIDTH_8 && cheap_rays(s.cw8_cost), false, st, &aw);
         if (r != TRACER_OK) return r;
     } else {
         c->last_kernel = 3;

@@ -659,7 +659,10 @@ __device__ __forceinline__ bool known_hit(const WfState& s, uint32_t pid, const 
 }
 
 // ------------------------------------------------------------------- shade --
-template <int TIE, bool BVH, bool STATS, bool MULTI, bool NEE>
+// KEEP: a pixel's next sample goes on from its kept primary hit here, without a
+// round.  A form of its own, as the loop costs the others 8 % (2000 spheres,
+// 1920x1080 x 1 spp, all shade launches: 0.40 ms, 0.37 without).
+template <int TIE, bool BVH, bool STATS, bool MULTI, bool NEE, bool KEEP>
 __global__ void __launch_bounds__(256) wf_shade(TraceArgs a, WfState s, int qsel, const TraceArgs* slots)
 {
     extern __shared__ int smem[];
@@ -691,6 +694,7 @@ __global__ void __launch_bounds__(256) wf_shade(TraceArgs a, WfState s, int qsel
         while (NEE ? __any_sync(0xFFFFFFFFu, on) : on) {
             const bool more = advance_path<NEE>(tr, A, on, x, y, h, ps);
             again = on ? more : again;
+            if (!KEEP) break;
             on = on && more && known_hit(s, pid, ps, h);
         }
         if (again) store_path(s, pid, ps);
@@ -824,7 +828,10 @@ static cudaError_t extend_t(const TraceArgs& a, const WfState& s, const WfConfig
 template <int TIE, bool BVH, bool STATS, bool MULTI>
 static cudaError_t shade_t(const TraceArgs& a, const WfState& s, const WfConfig& c, int qsel, cudaStream_t st)
 {
-    auto k = c.has_emitters ? wf_shade<TIE, BVH, STATS, MULTI, true> : wf_shade<TIE, BVH, STATS, MULTI, false>;
+    auto k = c.has_emitters ? wf_shade<TIE, BVH, STATS, MULTI, true, false> : wf_shade<TIE, BVH, STATS, MULTI, false, false>;
+    if constexpr (!STATS)
+        if (c.shade_samples)
+            k = c.has_emitters ? wf_shade<TIE, BVH, STATS, MULTI, true, true> : wf_shade<TIE, BVH, STATS, MULTI, false, true>;
     const size_t smem = (BVH && c.has_emitters) ? (size_t)a.stack_depth * 256 * 8 : 0;  // shadow rays' stack
     smem_attr(k, smem);
     k<<<c.shade_grid, 256, smem, st>>>(a, s, qsel, c.slots);

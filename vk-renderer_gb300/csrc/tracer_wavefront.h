@@ -25,7 +25,7 @@ struct WfState {
     uint32_t* queue[2];
     uint32_t* count;     // [0], [1]: queue lengths; [2]: extend's fetch cursor
     uint4* hit0;         // as hit: the pixel's primary hit, which its later samples start from;
-                         // nullptr (with statistics): they trace the ray again
+                         // nullptr (with statistics, or no later sample): they trace the ray again
     uint32_t* scene_of;  // batched: scene index of each slot (written by generate)
 };
 
@@ -33,6 +33,7 @@ struct WfConfig {
     int tie, bvh, stats;
     int multi;                // batched: per-slot scene table
     int has_emitters;         // some scene has emissive spheres (shade needs a traversal stack)
+    int shade_samples;        // WfState::hit0 is there and shade starts a pixel's next sample from it at once
     int wide;                 // extend's BVH: WF_WIDTH_2 (binary), WF_WIDTH_4 or WF_WIDTH_8 (every scene has it)
     uint32_t cw8_stack;       // WF_WIDTH_8: the extend kernel's stack entries (the 8-wide depth; 0 = the
                               // launch's stack_depth, which the shade and finishing kernels use)
