@@ -176,8 +176,9 @@ typedef struct tracer_scene_desc {
 #define TRACER_KERNEL_AUTO 0      /* WAVEFRONT for BVH scenes with >= 2^16 pixel x spp x depth when the
                                      scene has an 8-wide BVH (and bvh_width is 0 or 8), >= 2^22 otherwise;
                                      else PLAIN (tracer_trace_adjoint: WAVEFRONT wherever it applies).
-                                     PLAIN too at any size on scenes that it traces faster (with spheres,
-                                     or triangle-only ones of short rays), unless the call sets bvh_width,
+                                     PLAIN too at any size on scenes with spheres (but for more than 512
+                                     unlit ones and no triangle) and on triangle-only ones of short rays,
+                                     where it mostly is the faster one, unless the call sets bvh_width,
                                      tail_paths, wavefront, block or stack_depth, collects statistics or is
                                      profiled; the images are the same */
 #define TRACER_KERNEL_PLAIN 1     /* one thread per pixel, nested sample/bounce loops */

@@ -327,21 +327,28 @@ cudaEvent_t prof_event(tracer_ctx* c, size_t i)
 constexpr double kCheapRays = 20.0;
 bool cheap_rays(double cost) { return cost > 0.0 && cost <= kCheapRays; }
 
-// BVH scenes whose frames the plain kernel traces faster than the wavefront at
-// every size (its stages and path state cost more than they gain): scenes with
-// spheres, and triangle-only ones of short rays (kCheapRays; above, rounds win
-// on large frames: soup of 30k 2.74 / 2.39 ms).  Plain / wavefront as this line
-// was drawn, 1280x720 x 4 spp x depth 6, ms: height field of 20k triangles
-// 0.86 / 1.07, of 200k 1.67 / 1.81, soup of 10k 1.13 / 1.12; 20k triangles and
-// 30 spheres 3.48 / 5.13, 12k and 200 with 2 lights 14.2 / 21.3, 60k and 200
-// with 2 lights 33.4 / 44.1; 40 spheres 0.26 / 0.60, 2000 3.02 / 3.28.  Since
-// both trace a pixel's primary ray once: the height fields 0.68 / 0.84 and 1.31 /
-// 1.43, soup of 10k 0.63 / 0.60, of 30k 1.82 / 1.31, 20k and 30 spheres 2.59 /
-// 3.18.
+// BVH scenes that the automatic choice gives to the plain kernel at any size.
+// Plain / wavefront, ms, 640x360 and 1280x720 x 4 spp, 1920x1080 x 8, depth 6:
+//   triangles alone, short rays (kCheapRays): height field of 20k 0.49 / 0.63,
+//     0.90 / 1.20, 2.9 / 4.1, of 1M 0.92 / 1.08, 1.74 / 1.77, 5.8 / 6.1; soup of 3k 0.12
+//     / 0.14, 0.27 / 0.27, 0.68 / 0.67, of 10k 0.31 / 0.31, 0.66 / 0.60, 1.83 / 1.60;
+//     longer ones, soup of 30k: 0.75 / 0.65, 1.9 / 1.3, 6.5 / 3.7
+//   spheres, no lights: 64 0.38 / 0.53, 0.90 / 1.23, 3.2 / 4.3; 512 0.75 / 0.80, 2.0 / 2.0,
+//     7.7 / 7.2; 1000 0.98 / 0.99, 2.7 / 2.4, 10.5 / 8.7; 20k 1.87 / 1.64, 5.2 / 3.9, 20.3 /
+//     14.0: up to kPlainSpheres
+//   spheres with lights: 64 1.06 / 1.33, 2.7 / 3.9, 10.0 / 16.2; 20k 5.2 / 5.7, 14.2 / 17.4,
+//     56.8 / 70.9
+//   triangles and spheres: 5k and 1 0.19 / 0.42, 0.40 / 0.66, 1.04 / 1.25; 1M and 1 5.9 /
+//     6.3, 18.5 / 21.1, 74.8 / 74.7; between them the wavefront is the faster one on
+//     large frames, 60k and 1 1.67 / 1.67, 4.8 / 4.4, 17.1 / 14.2, 200k and 30 4.7 / 4.2,
+//     14.4 / 13.1, 57.7 / 47.7, which no rule here tells apart; with lights 12k and 200
+//     5.8 / 6.5, 14.9 / 22.6, 58 / 93, 60k and 200 14.0 / 15.7, 41 / 58, 165 / 246
+constexpr uint32_t kPlainSpheres = 512;
 bool plain_suits(const SceneBuffers& s)
 {
     if (s.cw8) return cheap_rays(s.cw8_cost);
-    return s.nt == 0 || s.tri_cw8.p;
+    if (s.nt == 0) return s.ne > 0 || s.ns <= kPlainSpheres;
+    return s.tri_cw8.p;
 }
 
 // A pixel's primary hit is kept for its later samples (WfState::hit0) where there
