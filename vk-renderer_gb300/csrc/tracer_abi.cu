@@ -290,7 +290,12 @@ void release_wavefront(tracer_ctx* c)
     c->wf_scene.release();
 }
 
-cudaError_t ensure_wavefront(tracer_ctx* c, size_t npx)
+// A pixel's primary hit is kept for its later samples (WfState::hit0) where there
+// are any and nothing counts rays.
+bool keeps_hits(int stats, uint32_t spp) { return !stats && spp > 1; }
+
+// kept: with room for the primary hits (keeps_hits).
+cudaError_t ensure_wavefront(tracer_ctx* c, size_t npx, bool kept)
 {
     cudaError_t e = dalloc(c->wf_ray_o, npx);
     if (e == cudaSuccess) e = dalloc(c->wf_ray_d, npx);
@@ -298,7 +303,7 @@ cudaError_t ensure_wavefront(tracer_ctx* c, size_t npx)
     if (e == cudaSuccess) e = dalloc(c->wf_mask, npx);
     if (e == cudaSuccess) e = dalloc(c->wf_accum, npx);
     if (e == cudaSuccess) e = dalloc(c->wf_hit, npx);
-    if (e == cudaSuccess) e = dalloc(c->wf_hit0, npx);
+    if (e == cudaSuccess && kept) e = dalloc(c->wf_hit0, npx);
     if (e == cudaSuccess) e = dalloc(c->wf_prim0, npx);
     if (e == cudaSuccess) e = dalloc(c->wf_q0, npx);
     if (e == cudaSuccess) e = dalloc(c->wf_q1, npx);
@@ -351,17 +356,14 @@ bool plain_suits(const SceneBuffers& s)
     return s.tri_cw8.p;
 }
 
-// A pixel's primary hit is kept for its later samples (WfState::hit0) where there
-// are any and nothing counts rays.
-bool keeps_hits(int stats, uint32_t spp) { return !stats && spp > 1; }
-
-// Whether shade starts the next sample from it at once (the finishing kernel
-// always does): everywhere but on lit scenes without triangles, whose primary
-// ray costs less in a round of all paths than the shadow rays of the few lanes
-// of a warp that are at a sample's end cost in shade.  Lit spheres, 640x360 and
-// 1280x720 x 4 spp, 1920x1080 x 8, depth 6, at once / in a round, ms: 64 1.63 / 1.33,
-// 4.81 / 3.94, 20.9 / 16.2; 5000 5.53 / 4.65, 17.6 / 14.6, 76.9 / 60.5; with
-// triangles (2000, 20 spheres, one light) 1.14 / 1.26, 3.24 / 3.99, 12.7 / 16.2.
+// Whether shade starts a pixel's next sample from its kept primary hit at once
+// (the finishing kernel always does): everywhere but on lit scenes without
+// triangles, whose primary ray costs less in a round of all paths than the
+// shadow rays of the few lanes of a warp that are at a sample's end cost in
+// shade.  Lit spheres, 640x360 and 1280x720 x 4 spp, 1920x1080 x 8, depth 6, at
+// once / in a round, ms: 64 1.63 / 1.33, 4.81 / 3.94, 20.9 / 16.2; 5000 5.53 / 4.65,
+// 17.6 / 14.6, 76.9 / 60.5; with triangles (2000, 20 spheres, one light) 1.14 / 1.26,
+// 3.24 / 3.99, 12.7 / 16.2.
 bool shade_keeps_on(bool keeps, bool lit, uint32_t triangles) { return keeps && !(lit && triangles == 0); }
 
 // Launches the wavefront: generate, then rounds of extend + shade until the
@@ -1006,7 +1008,8 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
         e = launch_plain(a, lc, st);
         c->last_launches = 1;
     } else {
-        e = ensure_wavefront(c, npx);
+        const bool kept = keeps_hits(stats, p->spp);
+        e = ensure_wavefront(c, npx, kept);
         if (e != cudaSuccess) return cuda_fail(c, e, "wavefront state allocation");
         a.pixel_base = 0;
         a.num_slots = (uint32_t)npx;
@@ -1016,7 +1019,6 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
         wc.bvh = s.bvh ? 1 : 0;
         wc.stats = stats;
         wc.has_emitters = s.ne > 0;
-        const bool kept = keeps_hits(stats, p->spp);
         wc.shade_samples = shade_keeps_on(kept, s.ne > 0, s.nt);
         wc.block = p->block ? p->block : 128;
         uint32_t wstack = stack;
@@ -1652,6 +1654,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
         max_spp = std::max(max_spp, p.spp);
     }
     if (total >= 0xFFFFFFFFull) return fail(c, TRACER_ERR_NO_SUITABLE_SURFACE, "batch has too many pixels");
+    const bool kept = keeps_hits(stats, max_spp);
     int r = finish(c);
     if (r != TRACER_OK) return r;
     cudaSetDevice(c->device);
@@ -1668,7 +1671,7 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
         if (e == cudaSuccess) c->pinned_slots_n = n;
     }
     if (e == cudaSuccess && kernel == TRACER_KERNEL_WAVEFRONT) {
-        e = ensure_wavefront(c, total);
+        e = ensure_wavefront(c, total, kept);
         if (e == cudaSuccess) e = dalloc(c->wf_scene, total);
     }
     if (e != cudaSuccess) return cuda_fail(c, e, "batch allocation");
@@ -1744,7 +1747,6 @@ extern "C" int tracer_trace_batched(tracer_ctx* c, const tracer_frame* frames, c
         wc.stats = stats;
         wc.multi = 1;
         wc.has_emitters = c->batch_emitters;
-        const bool kept = keeps_hits(stats, max_spp);
         wc.shade_samples = shade_keeps_on(kept, c->batch_emitters, c->batch.nt);
         wc.finish_w8 = c->batch.cw8 && !binary_asked(&p0);
         wc.block = block;
@@ -1987,7 +1989,7 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
     c->height = p->height;
     Launched launched{c, st};
     if (use_wf) {
-        e = ensure_wavefront(c, npx);
+        e = ensure_wavefront(c, npx, false);
         if (e == cudaSuccess) e = dalloc(ab.pix, npx);
         // pass 1's hits for pass 2 to replay without tracing, when they fit the limit
         const size_t log_n = npx * (size_t)p->max_depth;
