@@ -536,6 +536,15 @@ uint32_t trav_limit(const tracer_ctx* c, uint32_t nodes)
     return c->trav_cap ? c->trav_cap : 2 * nodes + 16;
 }
 
+// Time between two events, false if they were not both recorded (by an
+// unprofiled trace, say); that error is not left for the next launch to report.
+bool elapsed(float& ms, cudaEvent_t from, cudaEvent_t to)
+{
+    if (cudaEventElapsedTime(&ms, from, to) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
 // Inverse of the matrix with columns dir, right, up (row-major), for the
 // image projection of the camera's boundary term; false if singular.
 bool camera_inverse(const tracer_camera& cam, float out[9])
@@ -1092,17 +1101,17 @@ int tracer_last_timings(tracer_ctx* c, tracer_timings* out)
     out->launches = c->last_launches;
     if (!c->profiling) return fail(c, TRACER_ERR_INVALID_ARG, "profiling is off (tracer_set_profiling)");
     float ms = 0.0f;
-    if (cudaEventElapsedTime(&ms, c->prof_begin, c->prof_end) == cudaSuccess) out->total_ms = ms;
+    if (elapsed(ms, c->prof_begin, c->prof_end)) out->total_ms = ms;
     if (c->last_kernel == TRACER_KERNEL_WAVEFRONT) {
         for (uint32_t i = 0; i < c->last_prof_rounds && 3 * (size_t)i + 2 < c->prof_events.size(); ++i) {
-            if (cudaEventElapsedTime(&ms, c->prof_events[3 * i], c->prof_events[3 * i + 1]) == cudaSuccess)
+            if (elapsed(ms, c->prof_events[3 * i], c->prof_events[3 * i + 1]))
                 out->extend_ms += ms;
-            if (cudaEventElapsedTime(&ms, c->prof_events[3 * i + 1], c->prof_events[3 * i + 2]) == cudaSuccess)
+            if (elapsed(ms, c->prof_events[3 * i + 1], c->prof_events[3 * i + 2]))
                 out->shade_ms += ms;
         }
         const size_t f = c->last_prof_rounds;
         if (c->last_finish && 3 * f + 1 < c->prof_events.size() &&
-            cudaEventElapsedTime(&ms, c->prof_events[3 * f], c->prof_events[3 * f + 1]) == cudaSuccess)
+            elapsed(ms, c->prof_events[3 * f], c->prof_events[3 * f + 1]))
             out->finish_ms = ms;
     }
     return TRACER_OK;
@@ -1132,10 +1141,10 @@ int tracer_last_rounds(tracer_ctx* c, tracer_round_info* out, uint32_t cap, uint
         o.shade_ms = 0.0f;
         float ms = 0.0f;
         if (3 * (size_t)i + 1 < c->prof_events.size() &&
-            cudaEventElapsedTime(&ms, c->prof_events[3 * i], c->prof_events[3 * i + 1]) == cudaSuccess)
+            elapsed(ms, c->prof_events[3 * i], c->prof_events[3 * i + 1]))
             o.extend_ms = ms;
         if (!o.finish && 3 * (size_t)i + 2 < c->prof_events.size() &&
-            cudaEventElapsedTime(&ms, c->prof_events[3 * i + 1], c->prof_events[3 * i + 2]) == cudaSuccess)
+            elapsed(ms, c->prof_events[3 * i + 1], c->prof_events[3 * i + 2]))
             o.shade_ms = ms;
     }
     return TRACER_OK;
