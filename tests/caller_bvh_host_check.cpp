@@ -141,6 +141,21 @@ int main(int argc, char** argv)
     if (!vkt::build_cw8(split.data(), (uint32_t)split.size(), coded, order, &depth) || !vkt::pack_w8(coded, w))
         fail("8-wide build");
 
+    // the same on any number of host threads
+    for (uint32_t threads : {2u, 8u}) {
+        std::vector<tracer_bvh_node> split2;
+        std::vector<uint32_t> slot2, order2;
+        std::vector<vkt::Cw8Node> coded2;
+        double cost = 0.0;
+        vkt::split_leaves(nodes.data(), (uint32_t)nodes.size(), reinterpret_cast<const double(*)[6]>(box.data()), split2,
+                          slot2, threads);
+        if (!vkt::build_cw8(split2.data(), (uint32_t)split2.size(), coded2, order2, &depth, &cost, threads) ||
+            slot2 != slot_of || order2 != order || coded2.size() != coded.size() ||
+            std::memcmp(split2.data(), split.data(), split.size() * sizeof split[0]) ||
+            std::memcmp(coded2.data(), coded.data(), coded.size() * sizeof coded[0]))
+            fail("another tree on threads", threads);
+    }
+
     // the device's slab test over every node whose parent it enters
     long hits = 0;
     std::vector<uint32_t> stack;

@@ -5,7 +5,9 @@
 // a hit mask on the traversal stack; the layout below is this project's).
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
+#include <thread>
 #include <vector>
 
 #include "tracer_abi.h"
@@ -50,6 +52,23 @@ static_assert(sizeof(Cw8Node) == 96, "8-wide node is 96 bytes");
 constexpr uint32_t kCw8MaxLeafPrims = 6;
 constexpr uint32_t kCw8MaxNodePrims = 24;
 
+// fn(from, to) over parts of [0, n), `least` or more each, on up to `threads` host
+// threads, this one among them.  fn allocates nothing and throws nothing; a part whose thread
+// cannot be started runs here.
+template <class F> void over_chunks(size_t n, uint32_t threads, const F& fn, size_t least = 2048)
+{
+    const size_t parts = std::max<size_t>(1, std::min<size_t>(threads, n / least));
+    std::vector<std::thread> pool;
+    pool.reserve(parts - 1);
+    try {
+        for (size_t p = 1; p < parts; ++p) pool.emplace_back([&fn, n, p, parts] { fn(n * p / parts, n * (p + 1) / parts); });
+    } catch (...) {
+    }
+    fn(0, n / parts);
+    for (size_t p = pool.size() + 1; p < parts; ++p) fn(n * p / parts, n * (p + 1) / parts);
+    for (std::thread& t : pool) t.join();
+}
+
 // Collapses a binary BVH (tracer_bvh_node, root 0, children side by side,
 // leaves = ranges of the leaf-ordered primitive array) into 8-wide nodes:
 // the cut of the binary tree with the least expected cost (the dynamic
@@ -63,8 +82,10 @@ constexpr uint32_t kCw8MaxNodePrims = 24;
 // (the quantised slab test's range).  *cost_out = the plan's cost over the
 // root's surface area: what a random ray through the root box is expected to
 // visit, in nodes.
+// threads: host threads to use; the tree is the same on any number.
 bool build_cw8(const tracer_bvh_node* nodes, uint32_t num_nodes, std::vector<Cw8Node>& out,
-               std::vector<uint32_t>& order_out, uint32_t* depth_out, double* cost_out = nullptr);
+               std::vector<uint32_t>& order_out, uint32_t* depth_out, double* cost_out = nullptr,
+               uint32_t threads = 1);
 
 // The node the kernels read, 96 bytes (three 256-bit loads), as 24
 // little-endian words: a Cw8Node's boxes with the grid written out as floats
@@ -95,8 +116,8 @@ bool pack_w8(const std::vector<Cw8Node>& in, std::vector<W8Node>& out);
 // and high corner of the box of leaf-ordered triangle k.  out: the deeper
 // tree, its leaves ranges of a new order whose entry j is leaf-ordered slot
 // slot_out[j].  A part's box is that of its triangles, padded as the binary
-// builder's, and inside the leaf's.
+// builder's, and inside the leaf's.  threads: as build_cw8.
 void split_leaves(const tracer_bvh_node* nodes, uint32_t num_nodes, const double (*tri)[6],
-                  std::vector<tracer_bvh_node>& out, std::vector<uint32_t>& slot_out);
+                  std::vector<tracer_bvh_node>& out, std::vector<uint32_t>& slot_out, uint32_t threads = 1);
 
 }  // namespace vkt

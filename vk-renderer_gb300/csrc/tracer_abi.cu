@@ -576,44 +576,55 @@ int pick_width(tracer_ctx* c, const tracer_trace_params* p, uint32_t& stack, int
     return pick_width_for(c, p, s.bvh && s.wide, s.wide_depth, s.bvh && s.cw8, s.cw8_depth, stack, wide);
 }
 
+// Threads of one scene's 8-wide build.
+uint32_t host_threads() { return std::min(8u, std::max(1u, std::thread::hardware_concurrency())); }
+
 // The 8-wide BVH of a triangle BVH and the triangles in its order: 64-byte
 // records (v0, original id) (v1 - v0, leaf-ordered slot) (v2 - v0, 0) (0),
 // from the leaf-ordered triangle records `tri` (3 float4 each, as uploaded).
 // The binary leaves are split to single triangles first.  Returns false when
-// the scene gets none (bvh_cw8.h).
-bool make_cw8(const std::vector<tracer_bvh_node>& tnodes, const std::vector<float4>& tri, std::vector<W8Node>& nodes,
-              std::vector<float4>& prims, uint32_t& depth, double& cost)
+// the scene gets none (bvh_cw8.h).  On up to `threads` host threads: a whole
+// upload on 16 Arm cores, ms, with binary leaves as leaf children / leaves split,
+// one thread / now: soup of 10k 12.4 / 15.3 / 13.7, 100k 141 / 169 / 139, 1M 1670 /
+// 1960 / 1650, height field of 1M 1050 / 1210 / 970; 60k triangles and a sphere (first
+// without an 8-wide BVH) 72 / 98 / 81; 16 scenes of 1k to 100k at once 157 / 187 / 157.
+bool make_cw8(const std::vector<tracer_bvh_node>& tnodes, const std::vector<float4>& tri, uint32_t threads,
+              std::vector<W8Node>& nodes, std::vector<float4>& prims, uint32_t& depth, double& cost)
 {
     if (tnodes.empty()) return false;
     for (const tracer_bvh_node& n : tnodes)
         if ((uint32_t)n.count > kCw8MaxLeafPrims) return false;
     const size_t nt = tri.size() / 3;
     std::vector<double> box(6 * nt);  // of (v0, v0 + e1, v0 + e2), the triangle the kernels test
-    for (size_t k = 0; k < nt; ++k) {
-        const float4 a = tri[3 * k], b = tri[3 * k + 1], e = tri[3 * k + 2];
-        const double v[3] = {a.x, a.y, a.z}, e1[3] = {b.x, b.y, b.z}, e2[3] = {e.x, e.y, e.z};
-        for (int q = 0; q < 3; ++q) {
-            box[6 * k + q] = v[q] + std::min(0.0, std::min(e1[q], e2[q]));
-            box[6 * k + 3 + q] = v[q] + std::max(0.0, std::max(e1[q], e2[q]));
+    over_chunks(nt, threads, [&](size_t from, size_t to) {
+        for (size_t k = from; k < to; ++k) {
+            const float4 a = tri[3 * k], b = tri[3 * k + 1], e = tri[3 * k + 2];
+            const double v[3] = {a.x, a.y, a.z}, e1[3] = {b.x, b.y, b.z}, e2[3] = {e.x, e.y, e.z};
+            for (int q = 0; q < 3; ++q) {
+                box[6 * k + q] = v[q] + std::min(0.0, std::min(e1[q], e2[q]));
+                box[6 * k + 3 + q] = v[q] + std::max(0.0, std::max(e1[q], e2[q]));
+            }
         }
-    }
+    });
     std::vector<tracer_bvh_node> split;
     std::vector<uint32_t> order, slot_of;
     split_leaves(tnodes.data(), (uint32_t)tnodes.size(), reinterpret_cast<const double(*)[6]>(box.data()), split,
-                 slot_of);
+                 slot_of, threads);
     std::vector<Cw8Node> coded;
-    if (!build_cw8(split.data(), (uint32_t)split.size(), coded, order, &depth, &cost) || !pack_w8(coded, nodes)) return false;
-    for (uint32_t& s : order) s = slot_of[s];
+    if (!build_cw8(split.data(), (uint32_t)split.size(), coded, order, &depth, &cost, threads) || !pack_w8(coded, nodes))
+        return false;
     prims.assign(4 * order.size(), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-    for (size_t k = 0; k < order.size(); ++k) {
-        const uint32_t slot = order[k];
-        const float4 a = tri[3 * (size_t)slot], b = tri[3 * (size_t)slot + 1], e = tri[3 * (size_t)slot + 2];
-        float fslot;
-        std::memcpy(&fslot, &slot, 4);
-        prims[4 * k + 0] = make_float4(a.x, a.y, a.z, b.w);  // v0, original id
-        prims[4 * k + 1] = make_float4(b.x, b.y, b.z, fslot);
-        prims[4 * k + 2] = make_float4(e.x, e.y, e.z, 0.0f);
-    }
+    over_chunks(order.size(), threads, [&](size_t from, size_t to) {
+        for (size_t k = from; k < to; ++k) {
+            const uint32_t slot = slot_of[order[k]];
+            const float4 a = tri[3 * (size_t)slot], b = tri[3 * (size_t)slot + 1], e = tri[3 * (size_t)slot + 2];
+            float fslot;
+            std::memcpy(&fslot, &slot, 4);
+            prims[4 * k + 0] = make_float4(a.x, a.y, a.z, b.w);  // v0, original id
+            prims[4 * k + 1] = make_float4(b.x, b.y, b.z, fslot);
+            prims[4 * k + 2] = make_float4(e.x, e.y, e.z, 0.0f);
+        }
+    });
     return true;
 }
 
@@ -858,7 +869,7 @@ int tracer_upload_scene(tracer_ctx* c, const tracer_scene_desc* d)
     std::vector<float4> cw8_prims;
     uint32_t cw8_depth = 0;
     double cw8_cost = 0.0;
-    const bool cw8_ok = s.bvh && s.nt > 0 && make_cw8(tnodes, tri, cw8, cw8_prims, cw8_depth, cw8_cost);
+    const bool cw8_ok = s.bvh && s.nt > 0 && make_cw8(tnodes, tri, host_threads(), cw8, cw8_prims, cw8_depth, cw8_cost);
 
     cudaError_t e = upload(s.tri, tri.data(), tri.size());
     if (e == cudaSuccess) e = upload(s.mats, reinterpret_cast<const float4*>(d->materials), 3 * (size_t)s.nm);
@@ -1459,7 +1470,9 @@ void pack_scene(const tracer_scene_desc& d, PackedScene& out)
         const float* em = d.spheres[i].mat.emissive;
         if (!(em[0] == 0.0f && em[1] == 0.0f && em[2] == 0.0f)) out.emit.push_back(i);
     }
-    out.cw8_ok = d.num_triangles > 0 && make_cw8(out.tnodes, out.tri, out.cw8, out.cw8_prims, out.cw8_depth, out.cw8_cost);
+    // (the largest scenes finish last, with the other scenes' cores idle)
+    out.cw8_ok = d.num_triangles > 0 &&
+                 make_cw8(out.tnodes, out.tri, host_threads(), out.cw8, out.cw8_prims, out.cw8_depth, out.cw8_cost);
     if (!out.cw8_ok) out.cw8_depth = 0;
 }
 
