@@ -28,7 +28,7 @@
 // common, the conversion unit (an eighth of the FMA pipe's rate) is avoided,
 // and the four neighbour taps are only evaluated where the variance test
 // needs them.  1024^2 -> 1920x1080, RGBA8, half of the picture above the
-// threshold: 44 us with scalar arithmetic, PRESENT_US packed.
+// threshold: 44 us with scalar arithmetic, 32 packed.
 
 #include <cuda_runtime.h>
 
@@ -85,14 +85,6 @@ __device__ __forceinline__ void fetch4(const uchar4* im, const size_t (&at)[4], 
     for (int k = 0; k < 4; ++k) w[k] = in[k] ? __ldg(reinterpret_cast<const uint32_t*>(im) + at[k]) : 0u;
     decode4(w, t);
 }
-__device__ __forceinline__ void fetch4(const float4* im, const size_t (&at)[4], const bool (&in)[4], Texel (&t)[4])
-{
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float4 v = in[k] ? __ldg(im + at[k]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        t[k] = Texel{make_float2(v.x, v.y), v.z};
-    }
-}
 
 // floor(x) and (int)x of an integer-valued x, for |x| < 2^22, on the FMA and
 // integer pipes (adding 1.5 x 2^23 rounds x to an integer in the low mantissa
@@ -116,8 +108,32 @@ __device__ __forceinline__ Axis axis(float s, float size)
     return Axis{int_of_small(fi), u - fi};
 }
 
-template <class T>
-__device__ __forceinline__ V3 bilinear(const T* im, uint32_t w, uint32_t h, Axis x, Axis y)
+// Float texels, four loads from one base but at the border and scalar products:
+// nothing is decoded, and the packed form below takes longer (1920x1080 to
+// 3840x2160, pictures alike: 82 us, scalar 72).
+__device__ __forceinline__ V3 bilinear(const float4* im, uint32_t w, uint32_t h, Axis x, Axis y)
+{
+    const float w00 = (1.0f - x.f) * (1.0f - y.f), w10 = x.f * (1.0f - y.f);
+    const float w01 = (1.0f - x.f) * y.f, w11 = x.f * y.f;
+    V3 t[4];
+    if (x.i >= 0 && y.i >= 0 && x.i + 1 < (int)w && y.i + 1 < (int)h) {
+        const float4* p = im + ((size_t)y.i * w + x.i);
+        t[0] = v3(__ldg(p));
+        t[1] = v3(__ldg(p + 1));
+        t[2] = v3(__ldg(p + w));
+        t[3] = v3(__ldg(p + w + 1));
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = x.i + (k & 1), j = y.i + (k >> 1);
+            const bool in = i >= 0 && j >= 0 && i < (int)w && j < (int)h;
+            t[k] = in ? v3(__ldg(im + ((size_t)j * w + i))) : splat(0.0f);  // border: black
+        }
+    }
+    return ((t[0] * w00 + t[1] * w10) + t[2] * w01) + t[3] * w11;
+}
+
+__device__ __forceinline__ V3 bilinear(const uchar4* im, uint32_t w, uint32_t h, Axis x, Axis y)
 {
     const float2 cx = make_float2(1.0f - x.f, x.f);
     const float2 w0 = mul2(cx, both(1.0f - y.f)), w1 = mul2(cx, both(y.f));  // (w00, w10), (w01, w11)
