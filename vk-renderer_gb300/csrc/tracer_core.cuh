@@ -44,7 +44,11 @@ struct Stack {
     int cap;
 };
 
-template <int TIE, bool BVH, bool STATS>
+// SHORT: the scans' loops are not unrolled, for k_plain with lights, which waits
+// for instructions (the reference's scene, 800x600 x 4: 0.93 ms, 1.09 unrolled).
+// The other kernels have room for unrolled ones (100 spheres, 320x180 x 4: plain
+// 0.26 ms, 0.33 not unrolled, adjoint 0.61, 0.85).
+template <int TIE, bool BVH, bool STATS, bool SHORT = false>
 struct Tracer {
     const DevScene& sc;
     Stack stk;
@@ -172,6 +176,23 @@ struct Tracer {
         }
     }
 
+    __device__ __forceinline__ bool test_plane(const Ray& ray, uint32_t i, Hit& h, float tmax, bool any)
+    {
+        count(C_PLANES);
+        const float4* p = sc.planes + 4 * (size_t)i;
+        const float4 q = __ldg(p + 3);
+        const float tt = plane_intersect(ray, v3(q), q.w);
+        const uint32_t id = sc.nt + sc.ns + i;
+        if (accept<TIE>(tt, id, h, tmax, true)) {
+            h.t = tt;
+            h.prim = id;
+            h.kind = 3;
+            h.slot = i;
+            return any;
+        }
+        return false;
+    }
+
     // Tracer.comp:374-431.  h.t holds tmax on entry; on return h describes
     // the winning primitive (kind 0 = none).
     __device__ __forceinline__ bool trace(const Ray& ray, Hit& h, bool shadow)
@@ -184,36 +205,29 @@ struct Tracer {
         if (isnan3(ray.d)) return false;  // no intersection routine accepts a NaN direction
         const bool any = shadow;
         bool done = false;
-        if (BVH && sc.n_tri_nodes && sc.nt) {
-            BoxRay br = make_boxray(ray);
-            done = traverse<0>(sc.tri_nodes, sc.n_tri_nodes, ray, br, h, tmax, any);
-        } else {
-#pragma unroll 1
+        if constexpr (!BVH && !SHORT) {
             for (uint32_t i = 0; i < sc.nt && !done; ++i) done = test_tri(ray, i, h, tmax, any);
-        }
-        if (!done) {
-            if (BVH && sc.n_sph_nodes && sc.ns) {
+            for (uint32_t i = 0; i < sc.ns && !done; ++i) done = test_sphere(ray, i, h, tmax, any);
+            for (uint32_t i = 0; i < sc.np && !done; ++i) done = test_plane(ray, i, h, tmax, any);
+        } else {
+            if (BVH && sc.n_tri_nodes && sc.nt) {
                 BoxRay br = make_boxray(ray);
-                done = traverse<1>(sc.sph_nodes, sc.n_sph_nodes, ray, br, h, tmax, any);
+                done = traverse<0>(sc.tri_nodes, sc.n_tri_nodes, ray, br, h, tmax, any);
             } else {
 #pragma unroll 1
-                for (uint32_t i = 0; i < sc.ns && !done; ++i) done = test_sphere(ray, i, h, tmax, any);
+                for (uint32_t i = 0; i < sc.nt && !done; ++i) done = test_tri(ray, i, h, tmax, any);
             }
-        }
+            if (!done) {
+                if (BVH && sc.n_sph_nodes && sc.ns) {
+                    BoxRay br = make_boxray(ray);
+                    done = traverse<1>(sc.sph_nodes, sc.n_sph_nodes, ray, br, h, tmax, any);
+                } else {
 #pragma unroll 1
-        for (uint32_t i = 0; i < sc.np && !done; ++i) {
-            count(C_PLANES);
-            const float4* p = sc.planes + 4 * (size_t)i;
-            const float4 q = __ldg(p + 3);
-            const float tt = plane_intersect(ray, v3(q), q.w);
-            const uint32_t id = sc.nt + sc.ns + i;
-            if (accept<TIE>(tt, id, h, tmax, true)) {
-                h.t = tt;
-                h.prim = id;
-                h.kind = 3;
-                h.slot = i;
-                done = any;
+                    for (uint32_t i = 0; i < sc.ns && !done; ++i) done = test_sphere(ray, i, h, tmax, any);
+                }
             }
+#pragma unroll 1
+            for (uint32_t i = 0; i < sc.np && !done; ++i) done = test_plane(ray, i, h, tmax, any);
         }
         if (h.kind == 0) return false;
         if (!shadow) count(C_HITS);  // closest-hit rays that hit (each reads a material record)
@@ -458,11 +472,12 @@ __device__ __forceinline__ bool shade_bounce(TR& tr, const TraceArgs& a, bool on
 // waited 7 of 11 cycles per issue for instructions: a 640x360 frame with two
 // lights took 3.74 ms, with one 2.80.  (k_plain keeps two: it is smaller, at
 // its register limit, and 6 % slower this way.)
+//   NEE      false: the scene has no lights, the closest hits alone
 //   given    the lane has its closest hit in h already (found)
 //   first(found, h)            sees the closest hit; fills P, N, mat, diffuse of b
 //   light(si, L, t, g0)        an emitter that the surface sees; g0: the random
 //                              numbers of its direction L are the next two
-template <class TR, class G, class First, class Light>
+template <bool NEE, class TR, class G, class First, class Light>
 __device__ __forceinline__ void trace_rays(TR& tr, const TraceArgs& a, bool on, bool given, bool found, Hit h,
                                            const Ray& ray, G& g, Bounce& b, const First& first, const Light& light)
 {
@@ -475,12 +490,13 @@ __device__ __forceinline__ void trace_rays(TR& tr, const TraceArgs& a, bool on, 
 #pragma unroll 1
     for (uint32_t k = 0;; ++k) {
         bool hit = found;
-        if (go && !(given && k == 0)) hit = tr.trace(r, h, k > 0);
+        if (go && !(given && k == 0)) hit = tr.trace(r, h, NEE && k > 0);
         __syncwarp();
         if (k == 0)
             first(hit, h);
         else if (go && !hit)
             light(si, L, t, g0);
+        if (!NEE) break;
         go = b.diffuse && k < a.sc.ne;
         if (!__any_sync(0xFFFFFFFFu, go)) break;
         if (go) {
@@ -499,7 +515,7 @@ __device__ __forceinline__ bool trace_bounce(TR& tr, const TraceArgs& a, bool on
                                              uint32_t depth, Ray& ray, V3& acc, V3& mask, G& g, const F& first_hit)
 {
     Bounce b;
-    trace_rays(
+    trace_rays<true>(
         tr, a, on, given, found0, h0, ray, g, b,
         [&](bool found, const Hit& h) {
             if (on) first_hit(found, h);

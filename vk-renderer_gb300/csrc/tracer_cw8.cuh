@@ -250,19 +250,19 @@ __device__ __forceinline__ bool trace_bvh(const DevScene& sc, const Ray& ray, Hi
 
 // The per-thread trace_ray of the path kernels: trace_bvh on scenes with
 // BVHs, else the linear scan.
-template <int TIE, bool BVH, bool STATS, bool W8 = false>
-struct PathTracer : Tracer<TIE, false, STATS> {
+template <int TIE, bool BVH, bool STATS, bool W8 = false, bool SHORT = false>
+struct PathTracer : Tracer<TIE, false, STATS, SHORT> {
     PairStack pstk;
     __device__ __forceinline__ PathTracer(const DevScene& sc, const PairStack& p, Counters& cnt, int* status,
                                           uint32_t trav_limit)
-        : Tracer<TIE, false, STATS>{sc, Stack{nullptr, nullptr, 0, 0}, cnt, status, trav_limit}, pstk(p)
+        : Tracer<TIE, false, STATS, SHORT>{sc, Stack{nullptr, nullptr, 0, 0}, cnt, status, trav_limit}, pstk(p)
     {
     }
     __device__ __forceinline__ bool trace(const Ray& ray, Hit& h, bool shadow)
     {
         if (BVH)
             return trace_bvh<STATS, W8>(this->sc, ray, h, shadow, pstk, this->status, this->trav_limit, this->cnt);
-        return Tracer<TIE, false, STATS>::trace(ray, h, shadow);
+        return Tracer<TIE, false, STATS, SHORT>::trace(ray, h, shadow);
     }
 };
 

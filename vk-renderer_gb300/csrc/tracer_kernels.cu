@@ -16,19 +16,19 @@ namespace vkt {
 
 // With statistics, the canonical traversal (its node visiting order is the
 // oracle's); without, the path kernels' faster one, which finds the same hits.
-template <int TIE, bool BVH, bool STATS, bool W8>
-using PlainTracer = std::conditional_t<STATS, Tracer<TIE, BVH, STATS>, PathTracer<TIE, BVH, STATS, W8>>;
+template <int TIE, bool BVH, bool STATS, bool W8, bool SHORT>
+using PlainTracer = std::conditional_t<STATS, Tracer<TIE, BVH, STATS, SHORT>, PathTracer<TIE, BVH, STATS, W8, SHORT>>;
 
-template <int TIE, bool BVH, bool STATS, bool W8>
-__device__ __forceinline__ PlainTracer<TIE, BVH, STATS, W8> plain_tracer(const TraceArgs& a, int* smem, Counters& cnt)
+template <int TIE, bool BVH, bool STATS, bool W8, bool SHORT>
+__device__ __forceinline__ PlainTracer<TIE, BVH, STATS, W8, SHORT> plain_tracer(const TraceArgs& a, int* smem, Counters& cnt)
 {
     if constexpr (STATS) {
         const int n = blockDim.x, tid = threadIdx.x;
-        return Tracer<TIE, BVH, STATS>{
+        return Tracer<TIE, BVH, STATS, SHORT>{
             a.sc, Stack{smem + tid, reinterpret_cast<float*>(smem + (size_t)a.stack_depth * n) + tid, n, (int)a.stack_depth},
             cnt, a.status, a.trav_limit};
     } else {
-        return PathTracer<TIE, BVH, STATS, W8>(a.sc, thread_stack(smem, a.stack_depth), cnt, a.status, a.trav_limit);
+        return PathTracer<TIE, BVH, STATS, W8, SHORT>(a.sc, thread_stack(smem, a.stack_depth), cnt, a.status, a.trav_limit);
     }
 }
 
@@ -58,7 +58,8 @@ __global__ void __launch_bounds__(256, BLOCKS) k_plain(TraceArgs a)
     Counters cnt;
 #pragma unroll
     for (int k = 0; k < C_COUNT; ++k) cnt.c[k] = 0;
-    PlainTracer<TIE, BVH, STATS, W8> tr = plain_tracer<TIE, BVH, STATS, W8>(a, smem, cnt);
+    constexpr bool kShort = !BVH && NEE;
+    PlainTracer<TIE, BVH, STATS, W8, kShort> tr = plain_tracer<TIE, BVH, STATS, W8, kShort>(a, smem, cnt);
     const uint32_t x = blockIdx.x * 16 + (tid & 15);
     const uint32_t y = blockIdx.y * (nthreads >> 4) + (tid >> 4);
     bool alive = x < a.width && y < a.height;
@@ -124,28 +125,28 @@ static cudaError_t launch_k(const TraceArgs& a, const LaunchConfig& lc, cudaStre
 // soup of 10k triangles at 320x180 x 4 spp took 225 us (232 at three blocks,
 // 247 at four), a lit scene of 12.7k primitives 2.79 ms (3.09, 3.16); linear
 // scans with lights too, the reference's scene at that size 206 us (229 at four).
-// Larger ones: four, three on triangle-only scenes (1280x720 x 4 spp, three /
+// (Counted traversals of BVHs, 100k triangles: 3.3 ms without a bound, 3.5 at
+// three.)  Larger ones: four, three on triangle-only scenes (1280x720 x 4 spp, three /
 // four: height field of 20k triangles 0.86 / 0.90 ms; 64 spheres 1.23 / 1.11,
 // the lit scene 15.3 / 14.2).
-template <int TIE, bool BVH, bool NEE, bool W8>
+template <int TIE, bool BVH, bool STATS, bool NEE, bool W8>
 static cudaError_t launch_sized(const TraceArgs& a, const LaunchConfig& lc, cudaStream_t s)
 {
-    constexpr int kSmall = BVH || NEE ? 2 : 4, kLarge = W8 ? 3 : 4;
-    if ((uint64_t)a.width * a.height <= 512ull * lc.sms) return launch_k<TIE, BVH, false, NEE, W8, kSmall>(a, lc, s);
-    return launch_k<TIE, BVH, false, NEE, W8, kLarge>(a, lc, s);
+    constexpr int kSmall = STATS && BVH ? 1 : BVH || NEE ? 2 : 4, kLarge = W8 || (STATS && BVH) ? 3 : 4;
+    if ((uint64_t)a.width * a.height <= 512ull * lc.sms) return launch_k<TIE, BVH, STATS, NEE, W8, kSmall>(a, lc, s);
+    return launch_k<TIE, BVH, STATS, NEE, W8, kLarge>(a, lc, s);
 }
 
 template <int TIE, bool BVH>
 static cudaError_t launch_s(const TraceArgs& a, const LaunchConfig& lc, cudaStream_t s)
 {
-    constexpr int kStats = BVH ? 3 : 4;
     if (lc.stats)
-        return a.sc.ne ? launch_k<TIE, BVH, true, true, false, kStats>(a, lc, s)
-                       : launch_k<TIE, BVH, true, false, false, kStats>(a, lc, s);
-    if (a.sc.ne) return launch_sized<TIE, BVH, true, false>(a, lc, s);
+        return a.sc.ne ? launch_sized<TIE, BVH, true, true, false>(a, lc, s)
+                       : launch_sized<TIE, BVH, true, false, false>(a, lc, s);
+    if (a.sc.ne) return launch_sized<TIE, BVH, false, true, false>(a, lc, s);
     if constexpr (BVH)
-        if (lc.w8) return launch_sized<TIE, BVH, false, true>(a, lc, s);
-    return launch_sized<TIE, BVH, false, false>(a, lc, s);
+        if (lc.w8) return launch_sized<TIE, BVH, false, false, true>(a, lc, s);
+    return launch_sized<TIE, BVH, false, false, false>(a, lc, s);
 }
 
 // Reads n 16-byte words `passes` times with loads that are cached in L2 only

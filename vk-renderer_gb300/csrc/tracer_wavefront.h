@@ -12,6 +12,8 @@ struct TraceArgs;
 // its compressed 8-wide collapse (bvh_wide.h, bvh_cw8.h).
 enum : int { WF_WIDTH_2 = 0, WF_WIDTH_4 = 1, WF_WIDTH_8 = 2 };
 
+constexpr uint32_t kShortScan = 32;  // most primitives of a short linear scan
+
 // One slot per pixel (index = scene's pixel_base + y * width + x), structure
 // of arrays.
 struct WfState {
