@@ -202,7 +202,8 @@ typedef struct tracer_trace_params {
     int32_t tie_mode;       /* TRACER_TIES_* */
     int32_t kernel;         /* TRACER_KERNEL_* */
     uint32_t block;         /* threads per block (multiple of 32, <= 1024); 0 = default */
-    uint32_t stack_depth;   /* traversal stack entries per thread; 0 = BVH depth */
+    uint32_t stack_depth;   /* binary traversal stack entries per thread; 0 = BVH depth (the 8-wide
+                               traversal's stack is always as deep as its tree) */
     uint32_t wavefront;     /* wavefront extend kernel: resident CTAs per SM; 0 = occupancy maximum */
     uint32_t aov_mask;      /* bit (1 << TRACER_AOV_*) per image written; 0 = RGBA8 only */
     uint32_t stats;         /* nonzero: count rays, node fetches and primitive tests */
@@ -236,7 +237,11 @@ int tracer_create(tracer_ctx** out, int cuda_device);
 void tracer_destroy(tracer_ctx* ctx);
 const char* tracer_last_error(const tracer_ctx* ctx);
 const char* tracer_status_string(int status);
-/* Bound for every wait on the GPU (default 60000 ms). */
+/* Bound for every wait on the GPU (default 60000 ms).  A wait polls: for its
+ * first 2 ms (0.1 ms inside a wavefront trace) without sleeping, a CPU core at
+ * full load, as a sleep takes longer than many traces.  A trace whose own wait
+ * runs out leaves its kernels running; the context's next call waits for them,
+ * within the same bound. */
 int tracer_set_timeout(tracer_ctx* ctx, uint32_t timeout_ms);
 /* Cap on the BVH traversal steps of one ray (no counterpart in the
  * reference, whose linear scan has no such loop).  0 = automatic: twice the

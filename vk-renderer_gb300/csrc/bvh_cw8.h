@@ -30,20 +30,22 @@ namespace vkt {
 //            lo x (w8, w9), lo y (w10, w11), lo z (w12, w13),
 //            hi x (w14, w15), hi y (w16, w17), hi z (w18, w19);
 //            box = [p + lo * 2^(e - 127), p + hi * 2^(e - 127)] per axis,
-//            which contains the binary child's (padded) box with a margin of
-//            1/64 grid step on each side (the kernel's slab distances, with
-//            2^15 steps added and taken off, round by up to 3/512 step);
+//            which contains the binary child's box with a margin of 1/64
+//            grid step on each side: the kernel's slab distances, with 2^15
+//            steps added and taken off, round by some 1/512 step and by 2^-23
+//            of the distance from the ray's origin to p.  The second part, for
+//            origins more than 2^16 steps away the larger one, is covered by
+//            the acceptance's 2^-20, as in the binary test;
 //            p - 2^15 * 2^(e - 127) is a float too
 //   w20, w21 hit-mask bits of slot k: a leaf of c primitives (1..6) ->
 //            (1 << c) - 1; an interior child -> 1; an empty slot -> 0
 //   w22, w23 bit position of slot k: a leaf -> o, its first primitive being
 //            prim_base + o (o + c <= 24); an interior child -> 24 + slot
-// A child hit by a ray of octant s (bit a set for a negative direction
-// component on axis a) adds its bits at position (position ^ (mask & s ^ 7)):
-// the primitives to test in bits 0..23, the interior children in bits 24..31,
-// slot k at bit 24 + (k ^ s ^ 7).  Slot order: slot s holds the child met
-// first by rays of octant s; the traversal visits the hit interior children
-// highest bit first, i.e. in descending order of slot ^ s ^ 7.
+// The kernels read it as a W8Node (below), without w6, w7 and w20..w23's
+// positions; those are for a traversal that keeps one mask of a node's hits: a
+// child hit by a ray of octant s (bit a set for a negative direction
+// component on axis a) adds its bits at position (position ^ (mask & s ^ 7)).
+// Slot order: slot s holds the child met first by rays of octant s.
 struct alignas(32) Cw8Node {
     uint32_t w[24];
 };
@@ -52,9 +54,9 @@ static_assert(sizeof(Cw8Node) == 96, "8-wide node is 96 bytes");
 constexpr uint32_t kCw8MaxLeafPrims = 6;
 constexpr uint32_t kCw8MaxNodePrims = 24;
 
-// fn(from, to) over parts of [0, n), `least` or more each, on up to `threads` host
-// threads, this one among them.  fn allocates nothing and throws nothing; a part whose thread
-// cannot be started runs here.
+// fn(from, to) over parts of [0, n), `least` or more each, on up to `threads`
+// host threads, this one among them.  fn allocates nothing and throws nothing; a
+// part whose thread cannot be started runs here.
 template <class F> void over_chunks(size_t n, uint32_t threads, const F& fn, size_t least = 2048)
 {
     const size_t parts = std::max<size_t>(1, std::min<size_t>(threads, n / least));

@@ -322,13 +322,12 @@ cudaEvent_t prof_event(tracer_ctx* c, size_t i)
 }
 
 // Triangle-only scenes without lights whose rays visit at most this many 8-wide
-// nodes (build_cw8's estimate) run no rounds: the finishing kernel alone (every
-// sample's primary ray still traced) was faster by (frame 640x360 x 4 spp / 1280x720 x 4 / 1920x1080 x 8) 1.95 / 1.90 /
-// 1.84 on a soup of 500 triangles (estimate 5.1), 1.66 / 1.58 / 1.51 on 2k (9.0),
-// 1.31 / 1.22 / 1.15 on 10k (16.8); 1.35 / 1.54 / 1.25 on a height field of 2k
-// (7.2), 1.37 / 1.33 / 1.04 on 20k (10.4), 1.21 / 1.15 / 0.91 on 200k (13.8);
-// slower from 1.05 / 0.96 / 0.86 on a soup of 30k (27) to 0.91 / 0.63 / 0.54 on
-// 200k (66).
+// nodes (build_cw8's estimate) run no rounds in the wavefront (frames that fit
+// the resident threads run none anyway).  Finishing kernel alone against rounds,
+// 1280x720 x 4 spp / 1920x1080 x 8: 1.79 / 1.42 times as fast on a soup of 500
+// triangles (estimate 5.1), 1.37 / 1.12 on 2k (9.0), 1.07 / 0.89 on 10k (16.8), 0.89 /
+// 0.80 on 30k (27), 0.62 / 0.53 on 200k (66); 1.38 / 1.17 on a height field of 2k
+// (7.2), 1.09 / 0.92 on 20k (10.4), 1.17 / 0.90 on 200k (13.8).
 constexpr double kCheapRays = 20.0;
 bool cheap_rays(double cost) { return cost > 0.0 && cost <= kCheapRays; }
 
@@ -380,12 +379,9 @@ bool shade_keeps_on(bool keeps, bool bvh, bool lit, uint32_t triangles, uint32_t
 // grow from round to round, so the lagged count bounds the current one).
 // tail: 0 = twice the extend kernel's resident threads (below about one path
 // per lane a round costs the latency of its slowest ray, whatever its size;
-// measured on c1 with the finishing kernel as built: 1x 89.1 ms, 1.5x 88.6,
-// 2x 88.5), 1 = never.  With fewer path slots than that from the start (for
+// drawn on c1 when a frame took 88.5 ms: 1x 89.1, 1.5x 88.6), 1 = never.  With fewer path slots than that from the start (for
 // auto: fewer than the resident threads themselves), no round runs: the
-// finishing kernel traces every pixel after generate (c3's 256^2 adjoint:
-// 1.33 ms with four rounds first; a 640x360 frame of c1's scene, 230k
-// pixels: 5.0 ms without rounds against 4.5 with them).
+// finishing kernel traces every pixel after generate.
 // cheap: the scene's rays are short, so that a round's launches and path state
 // cost more than its traversals gain from the extend kernel: with the
 // automatic tail no round runs either (kCheapRays).
@@ -936,11 +932,12 @@ int tracer_trace(tracer_ctx* c, const tracer_frame* f, const tracer_trace_params
         return fail(c, TRACER_ERR_INVALID_ARG, "unknown tie mode %d", p->tie_mode);
     if (p->tie_mode == TRACER_TIES_REFERENCE && c->scene.bvh)
         return fail(c, TRACER_ERR_INVALID_ARG, "reference ties depend on scan order and need a linear-scan scene");
-    // AUTO: the plain kernel on linear-scan scenes, small frames and scenes that
-    // it traces faster (plain_suits); else the wavefront, from 2^16 path bounces
-    // where the scene has an 8-wide BVH, from 2^22 otherwise (c1 scene, plain /
-    // wavefront ms: 256^2 x 4 spp x depth 8 2.95 / 1.83, 640x360 x 4 x 8 8.06 /
-    // 3.08, 1920x1080 x 16 x 8 222 / 58).  A call that asks for something of the
+    // AUTO: the plain kernel on linear-scan scenes, small frames and where
+    // plain_suits; else the wavefront, from 2^16 path bounces where the scene has
+    // an 8-wide BVH, from 2^22 otherwise (c1 scene, plain / wavefront ms: 2^16
+    // bounces 0.43 / 0.45, 2^17 0.27 / 0.31, 2^19 0.83 / 0.82, 2^21 1.08 / 1.05, 640x360 x
+    // 4 spp x depth 8 2.57 / 1.76, 1920x1080 x 16 x 8 58.6 / 24.4: the line could lie
+    // at 2^19).  A call that asks for something of the
     // wavefront, for statistics or, with profiling on, for its stages' times
     // keeps the rule on bounces.
     const uint64_t bounces = (uint64_t)p->width * p->height * p->spp * p->max_depth;
@@ -1287,7 +1284,7 @@ extern "C" int tracer_trace_noalloc(tracer_ctx* c, const tracer_frame* f, const 
     if (p->tie_mode == TRACER_TIES_REFERENCE && c->scene.bvh)
         return fail(c, TRACER_ERR_INVALID_ARG, "reference ties depend on scan order and need a linear-scan scene");
     if (p->bvh_width != 0 && p->bvh_width != 2)
-        return fail(c, TRACER_ERR_INVALID_ARG, "bvh_width %u: the no-alloc trace runs the binary traversal only (0 or 2)",
+        return fail(c, TRACER_ERR_INVALID_ARG, "bvh_width %u: the no-alloc trace takes 0 or 2",
                     p->bvh_width);
     const SceneBuffers& s = c->scene;
     const uint32_t need = s.bvh ? (s.depth > 1 ? s.depth : 1) : 0;
@@ -1932,10 +1929,9 @@ extern "C" int tracer_trace_adjoint(tracer_ctx* c, const tracer_frame* f, const 
         return fail(c, TRACER_ERR_STACK_OVERFLOW, "stack depth %u below the BVH depth %u", stack, need);
     if ((size_t)stack * 128 * 8 > 100 * 1024)
         return fail(c, TRACER_ERR_INVALID_ARG, "stack depth %u exceeds shared memory", stack);
-    // AUTO: the wavefront wherever it applies (below).  With its finishing
-    // kernel it is the faster form at every size measured on the c3 scene
-    // (per-pixel / wavefront ms): 64^2 x 4 spp 1.29 / 1.25, 128^2 1.30 / 1.13,
-    // 256^2 1.72 / 1.36, 512^2 4.65 / 2.48; 1024^2 x 64 spp: 5.8x.
+    // AUTO: the wavefront wherever it applies (below), the faster form but on the
+    // smallest frames (c3 scene, per-pixel / wavefront ms: 64^2 x 4 spp 0.38 / 0.41,
+    // 128^2 0.38 / 0.37, 256^2 0.59 / 0.51, 512^2 1.36 / 1.01, 1024^2 x 16 14.7 / 11.1).
     const int kernel = p->kernel == TRACER_KERNEL_AUTO ? TRACER_KERNEL_WAVEFRONT : p->kernel;
     if (kernel != TRACER_KERNEL_PLAIN && kernel != TRACER_KERNEL_WAVEFRONT)
         return fail(c, TRACER_ERR_INVALID_ARG, "unknown kernel %d", p->kernel);

@@ -470,8 +470,9 @@ __device__ __forceinline__ bool shade_bounce(TR& tr, const TraceArgs& a, bool on
 // closest hit, then each emitter's shadow ray, so that the kernel holds one
 // copy of the traversal.  With two, on scenes with lights, the finishing kernel
 // waited 7 of 11 cycles per issue for instructions: a 640x360 frame with two
-// lights took 3.74 ms, with one 2.80.  (k_plain keeps two: it is smaller, at
-// its register limit, and 6 % slower this way.)
+// lights took 3.74 ms, with one 2.80.  (k_plain's lit
+// linear scans keep two: they are smaller, at their register limit, and 6 % slower
+// this way.)
 //   NEE      false: the scene has no lights, the closest hits alone
 //   given    the lane has its closest hit in h already (found)
 //   first(found, h)            sees the closest hit; fills P, N, mat, diffuse of b

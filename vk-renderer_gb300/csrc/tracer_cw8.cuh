@@ -49,8 +49,10 @@ __device__ __forceinline__ bool w8_any(uint2 G) { return (G.y & 0xFFu) != 0u; }
 // distances are fma(2^15 + q, step * ix, fma(p - 2^15 * step, ix, -o * ix)); a
 // child is hit iff max(near distances, 0) <= min(far distances, tbest), the
 // right side times (1 + 2^-20): the binary test's acceptance, on a box that
-// contains the binary box with a margin above these distances' rounding, so
-// every box the binary traversal enters is entered here too.
+// contains the binary box with a margin (Cw8Node).  A box that a ray passes
+// through is entered; of boxes that it only touches within rounding, a caller's
+// unpadded ones far from the origin among them, the two tests may enter
+// different ones.
 __device__ __forceinline__ void w8_visit(const float4* nodes, uint32_t idx, const W8Ray& r, float tbest, uint2& G,
                                          uint2& P)
 {
